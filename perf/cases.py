@@ -99,11 +99,47 @@ def _lengths(case):
 
 
 def _rows(gen, shape, dtype, k):
-    """K or V rows: normal values; K with the few large channels that keys have, the same in every sequence."""
+    """K or V rows: normal values; K with the few large channels that keys have, V about a mean of every channel that its
+    tokens share (so that the average over a long context does not vanish), the same in every sequence."""
     x = torch.randn(shape, generator=gen, device="cuda", dtype=dtype)
     if k:
         x[..., 5::31] *= 4
+    else:
+        x += torch.linspace(-1, 1, D, device="cuda", dtype=dtype)
     return x
+
+
+def _cached_rows(gen, case):
+    """Where the cache's blocks go (page table or None, and the rows of every sequence or page), then its unquantized rows
+    in the order they are packed, as (first, last, k, v)."""
+    b, s, page, block = case["b"], case["s"], case["page"], B.pack_block_tokens(case["bits"])
+    table, n, rows = None, b, max(block, (s + block - 1) // block * block)
+    if page:
+        per = (s + page - 1) // page
+        n, rows = b * per, page
+        table = torch.randperm(n, generator=gen, device="cuda").to(torch.int32).view(b, per)
+    yield table, n, rows
+    step = max(1, (1 << 20) // rows)
+    for i in range(0, n, step):
+        j = min(n, i + step)
+        k, v = (_rows(gen, (j - i, rows, case["h_k"], D), DTYPES[case["dtype"]], x) for x in (True, False))
+        yield i, j, k, v
+
+
+def _query_and_tail(gen, case):
+    b, dtype, tail = case["b"], DTYPES[case["dtype"]], case["tail"]
+    q = torch.randn(b, 1, case["h"], D, generator=gen, device="cuda", dtype=dtype)
+    return q, [_rows(gen, (b, tail, case["h_k"], D), dtype, x) for x in (True, False)] if tail else None
+
+
+def _exchange(gen, case):
+    """A generation's prompts, its tokens' queries and rows, and the rotary tables."""
+    b, s, n, h_k, dtype = case["b"], case["s"], case["tokens"], case["h_k"], DTYPES[case["dtype"]]
+    k, v = (_rows(gen, (b, s, h_k, D), dtype, x) for x in (True, False))
+    q = torch.randn(n, b, 1, case["h"], D, generator=gen, device="cuda", dtype=dtype)
+    kn, vn = (_rows(gen, (n, b, 1, h_k, D), dtype, x) for x in (True, False))
+    angle = torch.arange(s + n, device="cuda")[:, None] * 10000.0 ** (-torch.arange(D // 2, device="cuda") / (D // 2))
+    return dict(k=k, v=v, q=q, kn=kn, vn=vn, cos=angle.cos().to(dtype), sin=angle.sin().to(dtype))
 
 
 def prepare(case, seed):
@@ -117,36 +153,19 @@ def prepare(case, seed):
         k, v = (_rows(gen, (b, s, h_k, D), dtype, x) for x in (True, False))
         return dict(kind=kind, k=k, v=v, s=s, fmt=fmt, bufs=B.alloc_packed_cache(b, s, h_k, D, bits, group))
     if kind == "generate":
-        n = case["tokens"]
-        k, v = (_rows(gen, (b, s, h_k, D), dtype, x) for x in (True, False))
-        q = torch.randn(n, b, 1, h, D, generator=gen, device="cuda", dtype=dtype)
-        kn, vn = (_rows(gen, (n, b, 1, h_k, D), dtype, x) for x in (True, False))
-        angle = torch.arange(s + n, device="cuda")[:, None] * 10000.0 ** (-torch.arange(D // 2, device="cuda") / (D // 2))
-        cache = PackedKVCache(b, s + n + block, h_k, D, bits, group, dtype)
-        return dict(kind=kind, cache=cache, k=k, v=v, q=q, kn=kn, vn=vn, scale=scale, lens=_lengths(case)[0],
-                    cos=angle.cos().to(dtype), sin=angle.sin().to(dtype))
+        cache = PackedKVCache(b, s + case["tokens"] + block, h_k, D, bits, group, dtype)
+        return dict(kind=kind, cache=cache, scale=scale, lens=_lengths(case)[0], **_exchange(gen, case))
     # a packed cache, filled sequence by sequence (page by page where it is paged)
     lens, tails = _lengths(case)
-    page = case["page"]
-    table = None
-    if page:
-        per = (s + page - 1) // page
-        pages = b * per
-        order = torch.randperm(pages, generator=gen, device="cuda").to(torch.int32)
-        table = order.view(b, per)
-        rows = [page] * pages
-    else:
-        rows = [max(block, (s + block - 1) // block * block)] * b
-    bufs = B.alloc_packed_cache(len(rows), rows[0], h_k, D, bits, group)
-    step = max(1, (1 << 20) // rows[0])
-    for i in range(0, len(rows), step):
-        j = min(len(rows), i + step)
-        k, v = (_rows(gen, (j - i, rows[0], h_k, D), dtype, x) for x in (True, False))
-        B.kvcache_pack_int(k, bufs[0][i:j], bufs[1][i:j], v, bufs[2][i:j], bufs[3][i:j], None, None, rows[0], *fmt)
-    q = torch.randn(b, 1, h, D, generator=gen, device="cuda", dtype=dtype)
+    rows = _cached_rows(gen, case)
+    table, n, per = next(rows)
+    bufs = B.alloc_packed_cache(n, per, h_k, D, bits, group)
+    for i, j, k, v in rows:
+        B.kvcache_pack_int(k, bufs[0][i:j], bufs[1][i:j], v, bufs[2][i:j], bufs[3][i:j], None, None, per, *fmt)
+    q, tail = _query_and_tail(gen, case)
     kw = {}
-    if case["tail"]:
-        kw["k_res"], kw["v_res"] = (_rows(gen, (b, case["tail"], h_k, D), dtype, x) for x in (True, False))
+    if tail:
+        kw["k_res"], kw["v_res"] = tail
     if case["ragged"]:
         kw["cache_seqlens"] = torch.tensor(lens, dtype=torch.int32, device="cuda")
         if case["tail"]:
@@ -214,3 +233,69 @@ def tolerance(case):
     # the length as the average over V shrinks (probabilities and their products with the scales are rounded to
     # fp16); bf16, whose output is rounded to 8 bits, at most 2.4e-3 and 1.2e-2.
     return {"rel": 8e-3, "max": 6e-2} if case["dtype"] == "fp16" else {"rel": 1.2e-2, "max": 8e-2}
+
+
+def _dequantized(x, dim, case):
+    """(tokens, KV heads, D) rows as the cache's codes, scales and zeros hold them (groups along `dim`), in 64 bits."""
+    bits, group = case["bits"], case["group"]
+    x = x.float().unflatten(dim, (-1, group))
+    dim = dim % 3 + 1
+    lo, hi = x.amin(dim, keepdim=True), x.amax(dim, keepdim=True)
+    top = torch.full_like(lo, 2 ** bits - 1)
+    inv = torch.where(hi > lo, torch.div(top, hi - lo), 0 * top)
+    scale = torch.where(inv == 0, 0 * top, torch.div(torch.ones_like(top), inv))
+    codes = ((x - lo) * inv).add(0.5).floor().clamp(0, 2 ** bits - 1).double()
+    return (codes * scale.half().double() + lo.half().double()).flatten(dim - 1, dim)
+
+
+def _attend(q, k, v, scale):
+    """(h, D) over (tokens, h_k, D): the output and the log-sum-exp of the scaled scores."""
+    h_k = k.shape[1]
+    scores = torch.einsum("hgd,thd->hgt", q.double().view(h_k, -1, D), k.double()) * scale
+    lse = scores.logsumexp(-1)
+    return torch.einsum("hgt,thd->hgd", (scores - lse[..., None]).exp(), v.double()).reshape(-1, D), lse.reshape(-1)
+
+
+def _rotated(x, cos, sin):
+    """(heads, D) at one position, pairs (2i, 2i + 1), in 64 bits."""
+    a, b, cos, sin = x[..., ::2].double(), x[..., 1::2].double(), cos.double(), sin.double()
+    return torch.stack([a * cos - b * sin, a * sin + b * cos], -1).flatten(-2)
+
+
+def exact(case, seed):
+    if case["kind"] == "pack":
+        return None                                    # bytes, not computed numbers
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    scale, block, dtype = 1.0 / math.sqrt(D), B.pack_block_tokens(case["bits"]), DTYPES[case["dtype"]]
+    lens, tails = _lengths(case)
+    if case["kind"] == "generate":
+        x = _exchange(gen, case)
+        outs = [torch.empty(case["b"], 1, case["h"], D, dtype=torch.float64, device="cuda") for _ in range(case["tokens"])]
+        for i, n in enumerate(lens):
+            full = n // block * block
+            old = [_dequantized(x["k"][i, :full], 0, case), _dequantized(x["v"][i, :full], -1, case)] if full else \
+                [torch.empty(0, case["h_k"], D, dtype=torch.float64, device="cuda")] * 2
+            new = [x["k"][i, full:n], x["v"][i, full:n]]
+            for t, out in enumerate(outs):
+                cos, sin = x["cos"][n + t], x["sin"][n + t]
+                new = [torch.cat([new[0], _rotated(x["kn"][t, i], cos, sin).to(dtype)]), torch.cat([new[1], x["vn"][t, i]])]
+                out[i, 0] = _attend(_rotated(x["q"][t, i, 0], cos, sin), torch.cat([old[0], new[0].double()]),
+                                    torch.cat([old[1], new[1].double()]), scale)[0]
+                if len(new[0]) == block:
+                    old = [torch.cat([o, _dequantized(y, dim, case)]) for o, y, dim in zip(old, new, (0, -1))]
+                    new = [y[:0] for y in new]
+        return outs, [None] * 4, None, None, None, None
+    rows = _cached_rows(gen, case)
+    table, n, per = next(rows)
+    k, v = (torch.cat(x) for x in zip(*(r[2:] for r in rows)))
+    q, tail = _query_and_tail(gen, case)
+    out = torch.empty(q.shape, dtype=torch.float64, device="cuda")
+    lse = torch.empty(q.shape[0], q.shape[2], dtype=torch.float64, device="cuda")
+    for i, (n, r) in enumerate(zip(lens, tails)):
+        whole = (n + block - 1) // block * block
+        ki, vi = (x[table[i].long()].flatten(0, 1) if case["page"] else x[i] for x in (k, v))
+        ki, vi = _dequantized(ki[:whole], 0, case)[:n], _dequantized(vi[:whole], -1, case)[:n]
+        if r:
+            ki, vi = torch.cat([ki, tail[0][i, :r].double()]), torch.cat([vi, tail[1][i, :r].double()])
+        out[i, 0], lse[i] = _attend(q[i, 0], ki, vi, scale)
+    return (out, lse) if case["lse"] else out
