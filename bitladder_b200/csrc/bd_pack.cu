@@ -10,10 +10,9 @@
 // writes when it is built without --use_fast_math (4-bit, group 128 and 32).  PackParams::approx_div
 // selects the division of the reference as shipped instead (see scale_from_minmax).
 //
-// One CTA handles one pack block (NB = 32 * 16/bits tokens) of one KV head.
-// The work is pure streaming (read 2*NB*d*2 bytes, write a quarter or an eighth
-// of that): every thread keeps 64 packed pairs in flight for K, rows are read
-// and written in 128-byte warp segments, and nothing is re-read.
+// The work is pure streaming (read 2*NB*d*2 bytes of a pack block, NB = 32 * 16/bits tokens of one KV head,
+// write a quarter or an eighth of that): every thread keeps 32 words of input in flight, rows are read and
+// written in segments of at least 64 bytes per row, and nothing is re-read.
 #include <type_traits>
 #include "bd_common.cuh"
 #include "bd_kernels.h"
@@ -93,7 +92,7 @@ __device__ __forceinline__ void scale_from_minmax(float mn, float mx, float maxv
         scale = (scale_inv == 0.0f) ? 0.0f : __fdividef(1.0f, scale_inv);
     } else {
         scale_inv = (range > 0.0f) ? __fdiv_rn(maxv, range) : 0.0f;
-        scale = (scale_inv == 0.0f) ? 0.0f : __fdiv_rn(1.0f, scale_inv);
+        scale = (scale_inv == 0.0f) ? 0.0f : __frcp_rn(scale_inv);
     }
 }
 
@@ -112,18 +111,25 @@ __device__ __forceinline__ void param_slot(int g, int c, int &row, int &col) {
     }
 }
 
-// Four token subsets of 64 threads per CTA; resident threads per SM (and with them the
-// registers a thread may hold) chosen by measurement: 768 at 4 bits, 512 at 2 bits, where a
-// thread keeps twice as many fields.
-constexpr int kPackSubsets = 4;
-constexpr int kPackThreads = 64 * kPackSubsets;
+// A block of a head is the work of 2 * kPackSplit CTAs of 128 threads: kPackSplit share its K by channels, as many its
+// V by tokens.  A CTA is three phases (load, reduce, quantize and store) that cannot overlap inside it, so what keeps
+// HBM busy is eight small CTAs per SM in different phases (1024 threads of 64 registers), each thread with 32 words
+// of input in flight.  Measured, 4 bits / 2 bits, 8 x 32768 x 8 heads and 2 x 16384 x 32 heads (group 64, bf16),
+// graph replay: one CTA of 256 threads for K and then V (768 / 512 threads per SM) 212.5 / 135.7 us; split 2 ways
+// 197.6 / 110.0, 4 ways 203.7 / 102.9; with fewer resident threads (768) 216.4 / 105.2.
+template <int BITS> constexpr int kPackSplit = BITS == 4 ? 2 : 4;
+template <int BITS> constexpr int kPackSubsets = BITS == 4 ? 4 : 8;         // token subsets of the K half
+template <int BITS> constexpr int kPackThreads = (64 / kPackSplit<BITS>) * kPackSubsets<BITS>;
+constexpr int kPackResident = 1024;                                         // threads per SM
 template <int BITS, int GROUP, bool BF16>
-__global__ void __launch_bounds__(kPackThreads, (BITS == 4 ? 768 : 512) / kPackThreads)
+__global__ void __launch_bounds__(kPackThreads<BITS>, kPackResident / kPackThreads<BITS>)
 bd_pack_kernel(const PackParams p) {
     constexpr int P = 16 / BITS;            // codes per 16-bit word
     constexpr int NB = 32 * P;              // tokens per pack block
-    constexpr int NT = kPackSubsets;        // token subsets (threads = 64 * NT)
-    constexpr int NTHREADS = 64 * NT;
+    constexpr int SPLIT = kPackSplit<BITS>;  // CTAs that share a block's K (by channels), and as many its V (by tokens)
+    constexpr int KP = 64 / SPLIT;          // channel pairs of a CTA (K)
+    constexpr int NT = kPackSubsets<BITS>;  // token subsets (K)
+    constexpr int NTHREADS = KP * NT;
     constexpr int PPT = 32 / NT;            // pack rows per thread (K)
     constexpr int NGK = NB / GROUP;         // K token groups per block
     constexpr int FPG = GROUP / 32;         // K fields per group
@@ -134,12 +140,17 @@ bd_pack_kernel(const PackParams p) {
     const float maxv = static_cast<float>((1 << BITS) - 1);
     const bool approx_div = p.approx_div != 0;
 
-    __shared__ float red[NT][NGK][2][D];
-    __shared__ __half vprm[NGD][2][NB];
+    __shared__ union {
+        struct {
+            uint32_t red[NT][NGK][2][KP];   // K: minima and maxima of the token subsets, two channels each, in the input format
+            float4 coef[NGK][KP];           //    and what the groups are quantized with: zeros and scaled inverses of two channels
+        } k;
+        __half vprm[NGD][2][NB / SPLIT];    // V: scales and zeros of the CTA's tokens
+    } sh;
 
     const int tid = threadIdx.x;
     // heads vary fastest: CTAs that run together read neighbouring 256-byte pieces of the same token rows
-    const int ih = blockIdx.x, blk = blockIdx.y, ib = blockIdx.z;
+    const int blk = blockIdx.y, ib = blockIdx.z;
     int dst_off = p.dst_token_offset;
     if (p.roll_res_lens != nullptr) {          // roll-over: only sequences whose tail this step's token filled
         // The roll-over is staged early behind the decode kernel that files the token, and the kernel that moves
@@ -156,8 +167,9 @@ bd_pack_kernel(const PackParams p) {
     const uint16_t *vin = static_cast<const uint16_t *>(p.v);
 
     // ------------------------------------------------------------------ K
-    {
-        const int cp = tid & 63, T = tid >> 6;
+    if (blockIdx.x < SPLIT * p.h_k) {
+        const int ih = blockIdx.x / SPLIT;
+        const int cl = tid % KP, T = tid / KP, cp = (blockIdx.x % SPLIT) * KP + cl;
         const uint16_t *kbase = kin + ib * p.k_stride_b + static_cast<int64_t>(blk) * NB * p.k_stride_s +
                                 ih * p.k_stride_h + 2 * cp;
         uint32_t raw[PPT][P];
@@ -168,7 +180,6 @@ bd_pack_kernel(const PackParams p) {
                 const int t = T * PPT + pi + 32 * j;
                 raw[pi][j] = __ldg(reinterpret_cast<const unsigned int *>(kbase + t * p.k_stride_s));
             }
-        float mn[NGK][2], mx[NGK][2];
         {
             uint32_t pmn[NGK], pmx[NGK];        // both channels at once, in the input format
 #pragma unroll
@@ -183,45 +194,38 @@ bd_pack_kernel(const PackParams p) {
                 }
 #pragma unroll
             for (int gk = 0; gk < NGK; ++gk) {
-                const float2 a = pair_to_float2<BF16>(pmn[gk]), b2 = pair_to_float2<BF16>(pmx[gk]);
-                mn[gk][0] = a.x; mn[gk][1] = a.y; mx[gk][0] = b2.x; mx[gk][1] = b2.y;
+                sh.k.red[T][gk][0][cl] = pmn[gk];
+                sh.k.red[T][gk][1][cl] = pmx[gk];
             }
-        }
-#pragma unroll
-        for (int gk = 0; gk < NGK; ++gk) {
-            red[T][gk][0][2 * cp] = mn[gk][0]; red[T][gk][0][2 * cp + 1] = mn[gk][1];
-            red[T][gk][1][2 * cp] = mx[gk][0]; red[T][gk][1][2 * cp + 1] = mx[gk][1];
         }
         __syncthreads();
-        float sinv[NGK][2];
+        // One thread per (group, channel pair) works out the scales (two IEEE divisions a channel cost as much as
+        // twenty of its codes) and stores the parameters; the others take them from shared memory.
+        for (int i = tid; i < NGK * KP; i += NTHREADS) {
+            const int gk = i / KP, c = i % KP;
+            uint32_t a = sh.k.red[0][gk][0][c], b = sh.k.red[0][gk][1][c];
 #pragma unroll
-        for (int gk = 0; gk < NGK; ++gk)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                float a = red[0][gk][0][2 * cp + e], b = red[0][gk][1][2 * cp + e];
-#pragma unroll
-                for (int t2 = 1; t2 < NT; ++t2) {
-                    a = fminf(a, red[t2][gk][0][2 * cp + e]);
-                    b = fmaxf(b, red[t2][gk][1][2 * cp + e]);
-                }
-                mn[gk][e] = a;
-                float sc;
-                scale_from_minmax(a, b, maxv, approx_div, sinv[gk][e], sc);
-                sinv[gk][e] *= 1.0f / float(1 << BITS);      // exact; see put_field
-                mx[gk][e] = sc;   // reuse as the stored scale
+            for (int t2 = 1; t2 < NT; ++t2) {
+                a = pair_min<BF16>(a, sh.k.red[t2][gk][0][c]);
+                b = pair_max<BF16>(b, sh.k.red[t2][gk][1][c]);
             }
-        if (T == 0) {
-#pragma unroll
-            for (int gk = 0; gk < NGK; ++gk) {
-                int prow, pcol;
-                param_slot<BITS, GROUP>(gk, 2 * cp, prow, pcol);
-                const int64_t grow = static_cast<int64_t>(dst_blk) * NGK + prow;
-                __half *prm = reinterpret_cast<__half *>(p.k_params) +
-                              2 * (ib * p.k_params_stride_b + (grow * p.h_k + ih) * D);
-                *reinterpret_cast<__half2 *>(prm + pcol) = __floats2half2_rn(mx[gk][0], mx[gk][1]);
-                *reinterpret_cast<__half2 *>(prm + D + pcol) = __floats2half2_rn(mn[gk][0], mn[gk][1]);
-            }
+            const float2 lo = pair_to_float2<BF16>(a), hi = pair_to_float2<BF16>(b);
+            float si0, si1, sc0, sc1;
+            scale_from_minmax(lo.x, hi.x, maxv, approx_div, si0, sc0);
+            scale_from_minmax(lo.y, hi.y, maxv, approx_div, si1, sc1);
+            constexpr float kDiv = 1.0f / float(1 << BITS);      // exact; see put_field
+            sh.k.coef[gk][c] = make_float4(lo.x, lo.y, si0 * kDiv, si1 * kDiv);
+            int prow, pcol;
+            param_slot<BITS, GROUP>(gk, 2 * (cp - cl + c), prow, pcol);
+            const int64_t grow = static_cast<int64_t>(dst_blk) * NGK + prow;
+            __half *prm = reinterpret_cast<__half *>(p.k_params) + 2 * (ib * p.k_params_stride_b + (grow * p.h_k + ih) * D);
+            *reinterpret_cast<__half2 *>(prm + pcol) = __floats2half2_rn(sc0, sc1);
+            *reinterpret_cast<__half2 *>(prm + D + pcol) = __floats2half2_rn(lo.x, lo.y);
         }
+        __syncthreads();
+        float4 coef[NGK];
+#pragma unroll
+        for (int gk = 0; gk < NGK; ++gk) coef[gk] = sh.k.coef[gk][cl];
         uint16_t *kp = static_cast<uint16_t *>(p.k_pack) + ib * p.k_pack_stride_b +
                        ((static_cast<int64_t>(dst_blk) * 32 + T * PPT) * p.h_k + ih) * D + 2 * cp;
 #pragma unroll
@@ -231,8 +235,8 @@ bd_pack_kernel(const PackParams p) {
                 constexpr int J = decltype(jc)::value;
                 const float2 x = pair_to_float2<BF16>(raw[pi][J]);
                 constexpr int gk = J / FPG;
-                lo = put_field<BITS, J>(lo, x.x, mn[gk][0], sinv[gk][0]);
-                hi = put_field<BITS, J>(hi, x.y, mn[gk][1], sinv[gk][1]);
+                lo = put_field<BITS, J>(lo, x.x, coef[gk].x, coef[gk].z);
+                hi = put_field<BITS, J>(hi, x.y, coef[gk].y, coef[gk].w);
             };
             put(std::integral_constant<int, 0>{}); put(std::integral_constant<int, 1>{});
             put(std::integral_constant<int, 2>{}); put(std::integral_constant<int, 3>{});
@@ -242,17 +246,17 @@ bd_pack_kernel(const PackParams p) {
             }
             *reinterpret_cast<uint32_t *>(kp + static_cast<int64_t>(pi) * p.h_k * D) = lo | (hi << 16);
         }
-    }
-
+    } else {
     // ------------------------------------------------------------------ V
-    {
         // A thread owns 8 consecutive output words of one token (one 16-byte store) and so needs,
         // for every field j, the 8 dims  p0 + DP*j .. +7: P loads of 16 bytes.  DP/8 threads per token
         // (4 at 4 bits, 2 at 2 bits): the min/max over a token's group takes one or two shuffles.
         constexpr int TPT = DP / 8;              // threads per token
         constexpr int TPI = NTHREADS / TPT;      // tokens per iteration
-        constexpr int VITER = NB / TPI;
-        static_assert(VITER * TPI == NB, "token tiling");
+        constexpr int VITER = NB / SPLIT / TPI;
+        static_assert(VITER * TPI * SPLIT == NB, "token tiling");
+        const int xv = blockIdx.x - SPLIT * p.h_k;
+        const int ih = xv % p.h_k, tok0 = (xv / p.h_k) * (NB / SPLIT);      // the CTA's tokens start here
         const int q8 = tid % TPT, tsub = tid / TPT;
         const uint16_t *vbase = vin + ib * p.v_stride_b + static_cast<int64_t>(blk) * NB * p.v_stride_s +
                                 ih * p.v_stride_h + 8 * q8;
@@ -261,52 +265,59 @@ bd_pack_kernel(const PackParams p) {
         uint4 raw[VITER][P];
 #pragma unroll
         for (int u = 0; u < VITER; ++u) {
-            const int t = u * TPI + tsub;
+            const int t = tok0 + u * TPI + tsub;
 #pragma unroll
             for (int j = 0; j < P; ++j)
                 raw[u][j] = __ldg(reinterpret_cast<const uint4 *>(vbase + t * p.v_stride_s + DP * j));
         }
+        // Minima and maxima of all the thread's tokens first; then the lanes that share a token divide the (token, dim
+        // group) pairs among themselves: one lane works out a pair's scales and hands the inverse to the others.
+        float mn[VITER][NGD], mx[VITER][NGD], sinv[VITER][NGD];
 #pragma unroll
-        for (int u = 0; u < VITER; ++u) {
-            const int t = u * TPI + tsub;
-            float mn[NGD], mx[NGD];
-            {
-                uint32_t pmn[NGD], pmx[NGD];
+        for (int u = 0; u < VITER; ++u)
 #pragma unroll
-                for (int gd = 0; gd < NGD; ++gd) { pmn[gd] = kPairPosInf<BF16>; pmx[gd] = kPairNegInf<BF16>; }
+            for (int gd = 0; gd < NGD; ++gd) {
+                uint32_t pmn = kPairPosInf<BF16>, pmx = kPairNegInf<BF16>;
 #pragma unroll
-                for (int j = 0; j < P; ++j) {
-                    const int gd = j / FPGV;
+                for (int j = gd * FPGV; j < (gd + 1) * FPGV; ++j) {
                     const uint32_t w4[4] = {raw[u][j].x, raw[u][j].y, raw[u][j].z, raw[u][j].w};
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
-                        pmn[gd] = pair_min<BF16>(pmn[gd], w4[r]);
-                        pmx[gd] = pair_max<BF16>(pmx[gd], w4[r]);
+                        pmn = pair_min<BF16>(pmn, w4[r]);
+                        pmx = pair_max<BF16>(pmx, w4[r]);
                     }
                 }
 #pragma unroll
-                for (int gd = 0; gd < NGD; ++gd) {
-                    const float2 a = pair_to_float2<BF16>(pmn[gd]), b2 = pair_to_float2<BF16>(pmx[gd]);
-                    mn[gd] = fminf(a.x, a.y);
-                    mx[gd] = fmaxf(b2.x, b2.y);
-                }
-            }
-            float sinv[NGD];
-#pragma unroll
-            for (int gd = 0; gd < NGD; ++gd) {
-#pragma unroll
                 for (int off = 1; off < TPT; off <<= 1) {
-                    mn[gd] = fminf(mn[gd], __shfl_xor_sync(0xffffffffu, mn[gd], off));
-                    mx[gd] = fmaxf(mx[gd], __shfl_xor_sync(0xffffffffu, mx[gd], off));
+                    pmn = pair_min<BF16>(pmn, __shfl_xor_sync(0xffffffffu, pmn, off));
+                    pmx = pair_max<BF16>(pmx, __shfl_xor_sync(0xffffffffu, pmx, off));
                 }
-                float sc;
-                scale_from_minmax(mn[gd], mx[gd], maxv, approx_div, sinv[gd], sc);
-                sinv[gd] *= 1.0f / float(1 << BITS);         // exact; see put_field
-                if (q8 == 0) {
-                    vprm[gd][0][t] = __float2half_rn(sc);
-                    vprm[gd][1][t] = __float2half_rn(mn[gd]);
-                }
+                const float2 a = pair_to_float2<BF16>(pmn), b2 = pair_to_float2<BF16>(pmx);
+                mn[u][gd] = fminf(a.x, a.y);
+                mx[u][gd] = fmaxf(b2.x, b2.y);
             }
+        constexpr int ITEMS = VITER * NGD;
+#pragma unroll
+        for (int i0 = 0; i0 < ITEMS; i0 += TPT) {
+            float lo = mn[i0 / NGD][i0 % NGD], hi = mx[i0 / NGD][i0 % NGD];
+#pragma unroll
+            for (int i = 1; i < TPT; ++i)
+                if (i0 + i < ITEMS && q8 == i) { lo = mn[(i0 + i) / NGD][(i0 + i) % NGD]; hi = mx[(i0 + i) / NGD][(i0 + i) % NGD]; }
+            float si, sc;
+            scale_from_minmax(lo, hi, maxv, approx_div, si, sc);
+            si *= 1.0f / float(1 << BITS);                   // exact; see put_field
+            if (i0 + q8 < ITEMS) {
+                const int u = (i0 + q8) / NGD, gd = (i0 + q8) % NGD;
+                sh.vprm[gd][0][u * TPI + tsub] = __float2half_rn(sc);
+                sh.vprm[gd][1][u * TPI + tsub] = __float2half_rn(lo);
+            }
+#pragma unroll
+            for (int i = 0; i < TPT; ++i)
+                if (i0 + i < ITEMS) sinv[(i0 + i) / NGD][(i0 + i) % NGD] = __shfl_sync(0xffffffffu, si, i, TPT);
+        }
+#pragma unroll
+        for (int u = 0; u < VITER; ++u) {
+            const int t = u * TPI + tsub;
             uint32_t outw[4];
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
@@ -316,8 +327,8 @@ bd_pack_kernel(const PackParams p) {
                     const uint32_t w = r == 0 ? raw[u][J].x : (r == 1 ? raw[u][J].y : (r == 2 ? raw[u][J].z : raw[u][J].w));
                     const float2 x = pair_to_float2<BF16>(w);
                     constexpr int gd = J / FPGV;
-                    lo = put_field<BITS, J>(lo, x.x, mn[gd], sinv[gd]);
-                    hi = put_field<BITS, J>(hi, x.y, mn[gd], sinv[gd]);
+                    lo = put_field<BITS, J>(lo, x.x, mn[u][gd], sinv[u][gd]);
+                    hi = put_field<BITS, J>(hi, x.y, mn[u][gd], sinv[u][gd]);
                 };
                 put(std::integral_constant<int, 0>{}); put(std::integral_constant<int, 1>{});
                 put(std::integral_constant<int, 2>{}); put(std::integral_constant<int, 3>{});
@@ -327,24 +338,21 @@ bd_pack_kernel(const PackParams p) {
                 }
                 outw[r] = lo | (hi << 16);
             }
-            *reinterpret_cast<uint4 *>(vp + static_cast<int64_t>(t) * p.h_k * DP) = make_uint4(outw[0], outw[1], outw[2], outw[3]);
+            *reinterpret_cast<uint4 *>(vp + static_cast<int64_t>(tok0 + t) * p.h_k * DP) = make_uint4(outw[0], outw[1], outw[2], outw[3]);
         }
         __syncthreads();
-        // scales / zeros of this block's tokens: per dim group, per run of 128 tokens,
-        // 128 scales then 128 zeros.
-        constexpr int RUNS = NB / 128;
+        // scales / zeros of these tokens: per dim group, per run of 128 tokens, 128 scales then 128 zeros.
+        constexpr int RUNS = NB / 128, W = NB / SPLIT / 2;      // W: token pairs of this CTA
         const int64_t run0 = static_cast<int64_t>(dst_blk) * RUNS;
-        for (int i = tid; i < NGD * RUNS * 2 * 64; i += NTHREADS) {
-            const int w = i & 63;                  // pair index inside 128 values
-            const int z = (i >> 6) & 1;            // 0 scales, 1 zeros
-            const int run = (i >> 7) % RUNS;
-            const int gd = (i >> 7) / RUNS;
+        for (int i = tid; i < NGD * 2 * W; i += NTHREADS) {
+            const int w = i % W, z = (i / W) & 1, gd = i / (2 * W);      // z: 0 scales, 1 zeros
+            const int t = tok0 + 2 * w;
             int plane, pcol;
-            param_slot<BITS, GROUP>(gd, 2 * w, plane, pcol);
+            param_slot<BITS, GROUP>(gd, t & 127, plane, pcol);
             __half *dst = reinterpret_cast<__half *>(p.v_params) +
                           2 * (ib * p.v_params_stride_b + plane * p.v_params_stride_g + ih * p.v_params_stride_h) +
-                          256 * (run0 + run) + 128 * z + pcol;
-            *reinterpret_cast<__half2 *>(dst) = *reinterpret_cast<const __half2 *>(&vprm[gd][z][128 * run + 2 * w]);
+                          256 * (run0 + (t >> 7)) + 128 * z + pcol;
+            *reinterpret_cast<__half2 *>(dst) = *reinterpret_cast<const __half2 *>(&sh.vprm[gd][z][2 * w]);
         }
     }
 }
@@ -352,8 +360,8 @@ bd_pack_kernel(const PackParams p) {
 template <int BITS, int GROUP, bool BF16>
 static cudaError_t launch_pack_t(const PackParams &p, cudaStream_t stream) {
     constexpr int NB = 32 * (16 / BITS);
-    constexpr int NTHREADS = kPackThreads;
-    dim3 grid(p.h_k, p.s / NB, p.b);
+    constexpr int NTHREADS = kPackThreads<BITS>;
+    dim3 grid(2 * kPackSplit<BITS> * p.h_k, p.s / NB, p.b);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(NTHREADS);

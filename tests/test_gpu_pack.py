@@ -18,6 +18,16 @@ def test_pack_bit_exact(bits, group, dtype):
     G.assert_pack_equal(G.pack_gpu(B, x["k"], x["v"], bits, group), H.oracle_pack(x["k"], x["v"], bits, group, dtype))
 
 
+@pytest.mark.parametrize("bits,group", [(4, 128), (2, 128), (4, 64), (2, 64), (4, 32), (2, 32)])
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+def test_pack_one_block_of_odd_heads(bits, group, dtype):
+    """A single block: every CTA's share of the channels (K) and of the tokens (V), for head counts that are no
+    power of two."""
+    import bitladder_b200 as B
+    x = H.gen_qkv(3, B.pack_block_tokens(bits), 15, 5, seed=19, dtype=dtype)
+    G.assert_pack_equal(G.pack_gpu(B, x["k"], x["v"], bits, group), H.oracle_pack(x["k"], x["v"], bits, group, dtype))
+
+
 @pytest.mark.parametrize("bits,group", [(4, 128), (2, 64), (4, 32), (2, 32)])
 def test_pack_edge_values(bits, group):
     """All-zero and constant groups (scale 0), fp16 max, huge and tiny magnitudes, outlier channels."""
