@@ -674,34 +674,37 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
             if (!mbar_wait_bounded(kbar, phase, p.spin_limit)) { aborted = true; break; }
             if (phase == 0 && blk == blk0) { BD_TRACE_MARK(22); }
 
-            // q . zero per token group (rows of the A operand all equal the zero vector)
+            // q . zero per token group (rows 0-7 and 8-15 of the A operand all equal a group's zero vector)
             float Zc[NGK][NQT][2];
             {
-                float Z[NGK][NQT][4];
+                constexpr int NZP = (NGK + 1) / 2;          // two groups at a time: rows 0-7 the one, rows 8-15 the other
+                float Z[NZP][NQT][4];
 #pragma unroll
-                for (int gk = 0; gk < NGK; ++gk)
+                for (int zp = 0; zp < NZP; ++zp)
 #pragma unroll
                     for (int nq = 0; nq < NQT; ++nq)
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) Z[gk][nq][e] = 0.f;
+                        for (int e = 0; e < 4; ++e) Z[zp][nq][e] = 0.f;
 #pragma unroll
-                for (int gk = 0; gk < NGK; ++gk)
+                for (int zp = 0; zp < NZP; ++zp)
 #pragma unroll
                     for (int a = 0; a < 4; ++a) {
-                        uint32_t z0, z1, z2, z3;
-                        lds128(kprm + kprm_off<BITS, GROUP>(gk, a, l) + 256, z0, z1, z2, z3);
+                        uint32_t z0, z1, z2, z3, y0, y1, y2, y3;
+                        lds128(kprm + kprm_off<BITS, GROUP>(2 * zp, a, l) + 256, z0, z1, z2, z3);
+                        y0 = z0; y1 = z1; y2 = z2; y3 = z3;
+                        if constexpr (NGK > 1) lds128(kprm + kprm_off<BITS, GROUP>(2 * zp + 1, a, l) + 256, y0, y1, y2, y3);
 #pragma unroll
                         for (int nq = 0; nq < NQT; ++nq) {
-                            mma_f16(Z[gk][nq], z0, z0, z1, z1, qr[nq][a][0], qr[nq][a][1]);
-                            mma_f16(Z[gk][nq], z2, z2, z3, z3, qr[nq][a][2], qr[nq][a][3]);
+                            mma_f16(Z[zp][nq], z0, y0, z1, y1, qr[nq][a][0], qr[nq][a][1]);
+                            mma_f16(Z[zp][nq], z2, y2, z3, y3, qr[nq][a][2], qr[nq][a][3]);
                         }
                     }
 #pragma unroll
                 for (int gk = 0; gk < NGK; ++gk)
 #pragma unroll
                     for (int nq = 0; nq < NQT; ++nq) {
-                        Zc[gk][nq][0] = Z[gk][nq][0] * p.scale_log2;
-                        Zc[gk][nq][1] = Z[gk][nq][1] * p.scale_log2;
+                        Zc[gk][nq][0] = Z[gk / 2][nq][2 * (gk & 1)] * p.scale_log2;
+                        Zc[gk][nq][1] = Z[gk / 2][nq][2 * (gk & 1) + 1] * p.scale_log2;
                     }
             }
 
@@ -820,38 +823,33 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                         const uint32_t base = kcode + (a >> 1) * 4096 + u * 2048 + k_row_off + k_chunk_off[a & 1];
                         lds128(base, wl[0], wl[1], wl[2], wl[3]);
                         lds128(base + 1024, wh[0], wh[1], wh[2], wh[3]);
-                        uint32_t wls[4], whs[4];
+                        // One k-slice after the other, the fields of a slice one by one: four masks and an MMA each,
+                        // no two MMAs in a row with the same accumulator.  The masks and the MMAs share the warp
+                        // scheduler's dispatch (2 cycles a mask, 4 an MMA), which is what bounds the 2-bit kernels.
 #pragma unroll
-                        for (int x = 0; x < 4; ++x) { wls[x] = aux_word<BITS>(wl[x]); whs[x] = aux_word<BITS>(wh[x]); }
-                        // all fields first, then the MMAs of the first k-slice, then of the second:
-                        // consecutive MMAs never share an accumulator
-                        uint32_t F[P][8];
-                        auto extract = [&](auto jc) {
-                            constexpr int J = decltype(jc)::value;
-#pragma unroll
-                            for (int x = 0; x < 4; ++x) {
-                                F[J][2 * x] = field<BITS, J, kFieldPairs<BITS, GROUP>>(wl[x], wls[x]);
-                                F[J][2 * x + 1] = field<BITS, J, kFieldPairs<BITS, GROUP>>(wh[x], whs[x]);
-                            }
-                        };
-                        extract(std::integral_constant<int, 0>{});
-                        extract(std::integral_constant<int, 1>{});
-                        extract(std::integral_constant<int, 2>{});
-                        extract(std::integral_constant<int, 3>{});
-                        if constexpr (P == 8) {
-                            extract(std::integral_constant<int, 4>{});
-                            extract(std::integral_constant<int, 5>{});
-                            extract(std::integral_constant<int, 6>{});
-                            extract(std::integral_constant<int, 7>{});
-                        }
-#pragma unroll
-                        for (int half = 0; half < 2; ++half)
-#pragma unroll
-                            for (int j = 0; j < P; ++j)
+                        for (int half = 0; half < 2; ++half) {
+                            const uint32_t w0 = wl[2 * half], w1 = wh[2 * half], w2 = wl[2 * half + 1], w3 = wh[2 * half + 1];
+                            const uint32_t s0 = aux_word<BITS>(w0), s1 = aux_word<BITS>(w1), s2 = aux_word<BITS>(w2), s3 = aux_word<BITS>(w3);
+                            auto do_kfield = [&](auto jc) {
+                                constexpr int J = decltype(jc)::value;
+                                constexpr bool PR = kFieldPairs<BITS, GROUP>;
+                                const uint32_t f0 = field<BITS, J, PR>(w0, s0), f1 = field<BITS, J, PR>(w1, s1);
+                                const uint32_t f2 = field<BITS, J, PR>(w2, s2), f3 = field<BITS, J, PR>(w3, s3);
 #pragma unroll
                                 for (int nq = 0; nq < NQT; ++nq)
-                                    mma_f16(S[uu][j][nq], F[j][4 * half], F[j][4 * half + 1], F[j][4 * half + 2],
-                                            F[j][4 * half + 3], qs[j / FPG][nq][2 * half], qs[j / FPG][nq][2 * half + 1]);
+                                    mma_f16(S[uu][J][nq], f0, f1, f2, f3, qs[J / FPG][nq][2 * half], qs[J / FPG][nq][2 * half + 1]);
+                            };
+                            do_kfield(std::integral_constant<int, 0>{});
+                            do_kfield(std::integral_constant<int, 1>{});
+                            do_kfield(std::integral_constant<int, 2>{});
+                            do_kfield(std::integral_constant<int, 3>{});
+                            if constexpr (P == 8) {
+                                do_kfield(std::integral_constant<int, 4>{});
+                                do_kfield(std::integral_constant<int, 5>{});
+                                do_kfield(std::integral_constant<int, 6>{});
+                                do_kfield(std::integral_constant<int, 7>{});
+                            }
+                        }
                     }
                 }
 
