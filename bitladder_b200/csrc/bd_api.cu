@@ -320,7 +320,7 @@ int bd_decode_plan(const bd_decode_args *a, int32_t out[4]) {
     out[0] = plan.rows;
     out[1] = bd::decode_ctas_per_sm(a->bits, a->group, gq, plan.two_ctas);
     out[2] = bd::decode_warps(a->bits, a->group, gq, plan.two_ctas);
-    out[3] = (plan.ragged ? 1 : 0) + (a->rotary_dim > 0 ? 1 : 0) + 1 + (plan.rows > 4 * a->b ? 1 : 0) + (a->advance ? 2 : 0);
+    out[3] = (plan.ragged && a->b > bd::kInlineSeqs ? 1 : 0) + (a->rotary_dim > 0 ? 1 : 0) + 1 + (plan.rows > 4 * a->b ? 1 : 0) + (a->advance ? 2 : 0);
     return BD_OK;
 }
 
@@ -425,7 +425,8 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     part.R = plan.rows;
 
     cudaError_t err;
-    if (plan.ragged) {
+    const bool inline_table = plan.ragged && a->b <= bd::kInlineSeqs && !x;      // (the exchange kernel reads the table)
+    if (plan.ragged && !inline_table) {
         bd::PrefixParams pp;
         pp.cache_seqlens = a->cache_seqlens;
         pp.res_lens = a->k_res ? a->res_lens : nullptr;
@@ -468,6 +469,8 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     p.dtype = a->dtype;
     p.scale_log2 = a->softmax_scale * 1.4426950408889634f;
     p.part = part;
+    p.inline_table = inline_table ? 1 : 0;
+    p.block_tokens = nb;
     // workspace: [status word, 16 B][arrival counters][sequence table][segment partials]
     p.counters = reinterpret_cast<int32_t *>(ws + plan.off_counters);
     p.warp_acc = reinterpret_cast<float *>(ws + plan.off_warp_acc);

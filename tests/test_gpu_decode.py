@@ -219,6 +219,23 @@ def test_many_short_ragged_sequences(bits, dtype):
     _check(x, ref, out, lse, bits, 128, dtype, cs, rl, res=True)
 
 
+@pytest.mark.parametrize("b,s,bits,splits", [(1, 4096, 4, 0), (2, 4096, 2, 0), (31, 512, 4, 0), (32, 512, 4, 0), (31, 512, 2, 3)])
+def test_ragged_batches_at_the_table_limit(b, s, bits, splits):
+    """Up to 31 sequences the kernels work the table of units out themselves (a lane per sequence and one for the
+    total), with the parts merged in the decode kernel or, for few sequences, by the kernel behind it."""
+    import bitladder_b200 as B
+    res = 17
+    x = H.gen_qkv(b, s, 16, 4, seed=91, res=res)
+    ref = H.oracle_pack(x["k"], x["v"], bits, 128, "fp16")
+    bufs = G.pack_gpu(B, x["k"], x["v"], bits, 128)
+    g = torch.Generator().manual_seed(12)
+    cs = torch.randint(0, s + 1, (b,), generator=g, dtype=torch.int32)
+    rl = torch.randint(0, res + 1, (b,), generator=g, dtype=torch.int32)
+    cs[-1], rl[-1] = s - 1, 0
+    out, lse = _run(B, x, bufs, bits, 128, "fp16", num_splits=splits, k_res=x["k_res"], v_res=x["v_res"], cache_seqlens=cs, res_lens=rl)
+    _check(x, ref, out, lse, bits, 128, "fp16", cs, rl, res=True)
+
+
 def test_plan_reports_what_the_step_launches():
     """DecodeStep.plan(): ranges per KV head, CTAs per SM and launches as the library plans them on this GPU."""
     import bitladder_b200 as B
