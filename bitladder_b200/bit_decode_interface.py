@@ -24,6 +24,7 @@ Differences from the reference, all of them additions or stricter checks:
 from __future__ import annotations
 
 import ctypes as C
+import warnings
 from typing import Optional
 
 import torch
@@ -34,6 +35,41 @@ __all__ = ["kvcache_pack_int", "fwd_kvcache_int", "combine_partials", "decode_wo
            "plan_splits", "pack_block_tokens", "alloc_packed_cache", "DecodeStep"]
 
 _WORKSPACES = {}
+
+
+class _InterpretedCalls:
+    """Stands in for the ``_torch_calls`` extension where it cannot be loaded: every call takes the Python code below."""
+
+    @staticmethod
+    def decode(*_):
+        return None
+
+    pack = decode
+
+    @staticmethod
+    def step(args: int, device: int) -> int:
+        with torch.cuda.device(device):
+            return _lib.load().bd_decode(C.cast(args, C.POINTER(_lib.DecodeArgs)), _stream(device))
+
+
+_CALLS = None
+
+
+def _calls():
+    """The extension that takes plainly valid calls to the library without interpreted code (``csrc/bd_torch.cpp``); it
+    answers ``None`` to any other call, which the Python code then checks, refuses or serves."""
+    global _CALLS
+    if _CALLS is None:
+        lib = _lib.load()
+        try:
+            from . import _torch_calls as calls
+            calls.bind(*(C.cast(f, C.c_void_p).value for f in (lib.bd_decode, lib.bd_pack, lib.bd_decode_workspace_bytes)))
+        except ImportError as exc:
+            warnings.warn(f"bitladder_b200._torch_calls cannot be loaded ({exc}): calls cost 20 to 30 us more; run "
+                          "`python -m bitladder_b200.build`")
+            calls = _InterpretedCalls
+        _CALLS = calls
+    return _CALLS
 
 
 def pack_block_tokens(num_bits: int) -> int:
@@ -142,6 +178,10 @@ def kvcache_pack_int(k_cache: torch.Tensor, k_pack: torch.Tensor, k_params: torc
     built without that flag and of a CPU evaluation of its formulas.  The two differ by one code
     step at exact rounding ties, a few codes in 10^5.  Asynchronous on the current stream.
     """
+    if opt_block_table is None and isinstance(k_cache, torch.Tensor) and k_cache.is_cuda and _calls().pack(
+            k_cache, k_pack, k_params, v_cache, v_pack, v_params, quant_mode, group_size, num_bits, dst_token_offset,
+            reference_fast_math):
+        return
     _check_config(quant_mode, group_size, num_bits)
     # A paged pool is packed page by page: quantization groups never cross a pack block, so the
     # pages are just `num_pages` independent sequences of `page_size` tokens and the table is not needed.
@@ -341,6 +381,12 @@ def fwd_kvcache_int(q: torch.Tensor,
     ``opt_block_table`` entry outside the page pool).  Without ``check`` such a step returns
     unusable values silently; a serving loop checks every n-th step.
     """
+    if out is None and workspace is None and not (check or spin_limit or _test_starve) and isinstance(q, torch.Tensor) and q.is_cuda:
+        result = _calls().decode(_WORKSPACES, q, k_pack, k_params, v_pack, v_params, opt_block_table, softmax_scale, quant_mode,
+                                 group_size, num_bits, k_res, v_res, res_lens, cache_seqlens, seqlen_k, return_lse, out_dtype,
+                                 num_splits, k_new, v_new, advance, rotary_cos, rotary_sin, rotary_interleaved)
+        if result is not None:
+            return result
     _check_config(quant_mode, group_size, num_bits)
     _check_cuda(q, k_pack, k_params, v_pack, v_params, k_res, v_res, res_lens, cache_seqlens, out, workspace,
                 opt_block_table, k_new, v_new)
@@ -421,19 +467,16 @@ class DecodeStep:
         self._args.workspace, self._args.workspace_bytes = self._workspace.data_ptr(), need
         self._keep = (q, k_pack, k_params, v_pack, v_params, opt_block_table, k_res, v_res, res_lens, cache_seqlens,
                       k_new, v_new, rotary_cos, rotary_sin)
-        self._fn = _lib.load().bd_decode
         self._ref = C.byref(self._args)
+        self._launch = _calls().step
+        self._where = (C.addressof(self._args), self._device.index)
 
     def step(self, check: bool = False):
         """Launch the step on the current stream of the tensors' device; returns ``out`` (or
         ``(out, lse)``), the same buffers every time.  ``check=True`` waits for the step and raises
         ``RuntimeError`` if the kernel reported an error (see ``fwd_kvcache_int``); it synchronises,
         so a loop uses it every n-th step, and never inside a stream capture."""
-        if torch.cuda.current_device() != self._device.index:
-            with torch.cuda.device(self._device):
-                rc = self._fn(self._ref, _stream(self._device))
-        else:
-            rc = self._fn(self._ref, _stream(self._device))
+        rc = self._launch(*self._where)
         if rc != 0:
             _lib.check(rc, "bd_decode")
         if check:

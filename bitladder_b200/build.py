@@ -3,6 +3,8 @@
 Run as ``python -m bitladder_b200.build`` or call :func:`build`.  nvcc
 cross-compiles without a GPU, so this works on a CPU-only host; the resulting
 shared object sits beside this file and is what :mod:`bitladder_b200._lib` loads.
+``_torch_calls.so`` beside it (g++, the headers of the installed torch) takes the operators' calls
+on torch tensors to that library.
 """
 from __future__ import annotations
 
@@ -10,12 +12,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(_HERE, "csrc")
 BUILD_DIR = os.path.join(_HERE, "build")
 LIB_PATH = os.path.join(_HERE, "libbitdecode.so")
+CALLS_PATH = os.path.join(_HERE, "_torch_calls.so")
+CALLS_SOURCE = os.path.join(CSRC, "bd_torch.cpp")
 SOURCES = ["bd_pack.cu", "bd_decode.cu", "bd_combine.cu", "bd_exchange.cu", "bd_rope.cu", "bd_api.cu"]
 HEADERS = ["bd_common.cuh", "bd_kernels.h", os.path.join("..", "..", "include", "bitdecode.h")]
 
@@ -48,6 +53,16 @@ def _stale(target: str, deps) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _calls_command():
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    return [os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *(f"-I{d}" for d in (os.path.join(root, "include"), os.path.join(cuda, "include"), sysconfig.get_paths()["include"])),
+            CALLS_SOURCE, "-o", CALLS_PATH, f"-L{os.path.join(root, 'lib')}", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+
+
 def build(force: bool = False, verbose: bool = False, extra_flags=()) -> str:
     """Compile every CUDA source and link the shared library; returns its path."""
     nvcc = _nvcc()
@@ -65,10 +80,13 @@ def build(force: bool = False, verbose: bool = False, extra_flags=()) -> str:
                 cmd.insert(1, "-Xptxas=-v")
             jobs.append(cmd)
 
+    if force or _stale(CALLS_PATH, [CALLS_SOURCE, os.path.abspath(__file__), hdrs[-1]]):
+        jobs.append(_calls_command())
+
     def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
-            raise RuntimeError("nvcc failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+            raise RuntimeError("build failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
         return r.stdout + r.stderr
 
     if jobs:
@@ -76,7 +94,7 @@ def build(force: bool = False, verbose: bool = False, extra_flags=()) -> str:
             for out in ex.map(run, jobs):
                 if verbose and out:
                     print(out)
-    if force or jobs or _stale(LIB_PATH, objs):
+    if force or _stale(LIB_PATH, objs):
         run([nvcc, "-shared", "-o", LIB_PATH, *objs, "-lcudart"])
     return LIB_PATH
 

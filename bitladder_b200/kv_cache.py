@@ -18,6 +18,7 @@ device keeps them itself, roll-over included, and the mirror is plain arithmetic
 """
 from __future__ import annotations
 
+from operator import add
 from typing import List, Optional, Sequence
 
 import torch
@@ -100,9 +101,9 @@ class PackedKVCache:
         """Pack every tail that is full as its sequence's next block (one ``kvcache_pack_int`` call per
         sequence that rolls over, one for the whole batch when all do at the same length)."""
         nb = self.block
-        full = [ib for ib in range(self.batch) if self._tail[ib] == nb]
-        if not full:
+        if nb not in self._tail:
             return
+        full = [ib for ib in range(self.batch) if self._tail[ib] == nb]
         if any(self._packed[ib] + nb > self.capacity for ib in full):
             raise RuntimeError("cache capacity exceeded")
         same = len(full) == self.batch and len({self._packed[ib] for ib in full}) == 1
@@ -150,11 +151,12 @@ class PackedKVCache:
 
     def _advance_mirror(self) -> None:
         """What the device did to the lengths in a step with ``advance``: pure host arithmetic."""
-        for ib in range(self.batch):
-            self._tail[ib] += 1
-            if self._tail[ib] == self.block and self._packed[ib] + self.block <= self.capacity:
-                self._packed[ib] += self.block
-                self._tail[ib] = 0
+        self._tail = [t + 1 for t in self._tail]
+        if self.block in self._tail:
+            for ib in range(self.batch):
+                if self._tail[ib] == self.block and self._packed[ib] + self.block <= self.capacity:
+                    self._packed[ib] += self.block
+                    self._tail[ib] = 0
 
     def append_and_decode(self, q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, softmax_scale: float,
                           **kw) -> torch.Tensor:
@@ -165,7 +167,7 @@ class PackedKVCache:
         if k_new.shape != (self.batch, 1, self.nheads_k, self.head_dim) or v_new.shape != k_new.shape:
             raise RuntimeError("append_and_decode expects k_new/v_new of shape (batch, 1, nheads_k, head_dim)")
         self._roll_full_tails()                        # only after plain append() calls left a tail full
-        if any(p + t + 1 > self.capacity for p, t in zip(self._packed, self._tail)):
+        if max(map(add, self._packed, self._tail), default=-1) >= self.capacity:
             raise RuntimeError("cache capacity exceeded")
         seq_hi = max(self._packed) if self._packed else 0
         out = fwd_kvcache_int(q, self.k_pack, self.k_params, self.v_pack, self.v_params, None, softmax_scale,
