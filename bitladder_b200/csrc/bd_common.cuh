@@ -67,6 +67,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *tmap, uint
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1)
         : "memory");
 }
+// A 16-byte load that is issued where it is written.
+__device__ __forceinline__ void ldg128_pinned(const void *p, uint32_t (&r)[4]) {
+    asm volatile("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "l"(p) : "memory");
+}
 // Untiled bulk copy: both addresses 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile(

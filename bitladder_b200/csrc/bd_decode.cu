@@ -516,25 +516,16 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
             *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(p.v_res_out) + dst) = vw;
         }
 
-        // Query rows as B fragments: thread (g, l) holds q[row g][32a + 8l .. +7], a = 0..3.
+        // Query rows as B fragments: thread (g, l) holds q[row g][32a + 8l .. +7], a = 0..3.  Requested here, first looked
+        // at (bf16: converted) behind the bookkeeping below, which their latency covers.
         uint32_t qr[NQT][4][4];
 #pragma unroll
         for (int nq = 0; nq < NQT; ++nq) {
             const int qrow = nq * 8 + g;
+            const uint16_t *qp = static_cast<const uint16_t *>(p.q) + ib * p.q_stride_b +
+                                 (int64_t(ih) * p.gq + (qrow < p.gq ? qrow : 0)) * p.q_stride_h + 8 * l;
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                uint4 v = make_uint4(0, 0, 0, 0);
-                if (qrow < p.gq) {
-                    const uint16_t *qp = static_cast<const uint16_t *>(p.q) + ib * p.q_stride_b +
-                                         (int64_t(ih) * p.gq + qrow) * p.q_stride_h + 32 * a + 8 * l;
-                    v = *reinterpret_cast<const uint4 *>(qp);
-                    if (bf16) {
-                        v.x = bf16x2_to_f16x2(v.x); v.y = bf16x2_to_f16x2(v.y);
-                        v.z = bf16x2_to_f16x2(v.z); v.w = bf16x2_to_f16x2(v.w);
-                    }
-                }
-                qr[nq][a][0] = v.x; qr[nq][a][1] = v.y; qr[nq][a][2] = v.z; qr[nq][a][3] = v.w;
-            }
+            for (int a = 0; a < 4; ++a) ldg128_pinned(qp + 32 * a, qr[nq][a]);
         }
 
         // Which warps of this CTA share the sequence, which of them goes on with another sequence
@@ -571,6 +562,15 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                 *note = make_int4(int(share_mask), (goes_on + 1) | ((pr.c1 - pr.c0 + 1) << 8), pr.c0, (nparts << 1) | (pr.dense ? 1 : 0));
             __syncwarp();
         }
+#pragma unroll
+        for (int nq = 0; nq < NQT; ++nq)
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    if (bf16) qr[nq][a][x] = bf16x2_to_f16x2(qr[nq][a][x]);
+                    if (nq * 8 + g >= p.gq) qr[nq][a][x] = 0;
+                }
 
         float O[NQT][8][4];
         float ZS[NQT][NZ][4];
