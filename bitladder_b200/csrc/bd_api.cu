@@ -320,7 +320,7 @@ int bd_decode_plan(const bd_decode_args *a, int32_t out[4]) {
     out[0] = plan.rows;
     out[1] = bd::decode_ctas_per_sm(a->bits, a->group, gq, plan.two_ctas);
     out[2] = bd::decode_warps(a->bits, a->group, gq, plan.two_ctas);
-    out[3] = (plan.ragged && a->b > bd::kInlineSeqs ? 1 : 0) + (a->rotary_dim > 0 ? 1 : 0) + 1 + (plan.rows > 4 * a->b ? 1 : 0) + (a->advance ? 2 : 0);
+    out[3] = (plan.ragged && a->b > bd::kInlineSeqs ? 1 : 0) + (a->rotary_dim > 0 ? 1 : 0) + 1 + (plan.rows > 4 * a->b ? 1 : 0) + (a->advance ? 1 : 0);
     return BD_OK;
 }
 
@@ -502,6 +502,7 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
         err = bd::launch_rope(rp, stream);
         if (err != cudaSuccess) return BD_ERR_CUDA;
         p.q = rp.q_out; p.q_stride_b = int64_t(a->h) * 128; p.q_stride_h = 128;
+        p.after_rope = 1;
         p.k_new = rp.k_out; p.v_new = rp.v_out; p.new_stride_b = int64_t(a->h_k) * 128; p.new_stride_h = 128;
     }
     p.defer_merge = (x || plan.rows > 4 * a->b) ? 1 : 0;
@@ -523,7 +524,8 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     }
 
     if (a->advance) {
-        // roll-over: tails that this step's token filled become the next pack block of their sequence ...
+        // roll-over: tails that this step's token filled become the next pack block of their sequence, and every
+        // sequence's lengths move on
         PackParams pk;
         std::memset(&pk, 0, sizeof(pk));
         pk.k = a->k_res; pk.v = a->v_res;
@@ -537,16 +539,11 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
         pk.v_params_stride_b = a->v_params_stride_b; pk.v_params_stride_g = a->v_params_stride_g;
         pk.v_params_stride_h = a->v_params_stride_h;
         pk.b = a->b; pk.s = nb; pk.h_k = a->h_k;
-        pk.roll_res_lens = a->res_lens; pk.roll_cache_seqlens = a->cache_seqlens; pk.roll_s_cap = a->s_cap;
+        pk.roll_res_lens = const_cast<int32_t *>(a->res_lens); pk.roll_cache_seqlens = const_cast<int32_t *>(a->cache_seqlens);
+        pk.roll_arrivals = p.counters;                            // zero again when the decode kernel is done
+        pk.roll_status = reinterpret_cast<int32_t *>(ws);
+        pk.roll_s_cap = a->s_cap; pk.roll_res_cap = std::min(a->res_len, bd::kTailMax);
         err = bd::launch_pack(pk, a->bits, a->group, a->dtype, stream);
-        if (err != cudaSuccess) return BD_ERR_CUDA;
-        // ... and every sequence's lengths move on
-        bd::AdvanceParams ad;
-        ad.cache_seqlens = const_cast<int32_t *>(a->cache_seqlens);
-        ad.res_lens = const_cast<int32_t *>(a->res_lens);
-        ad.b = a->b; ad.block_tokens = nb; ad.s_cap = a->s_cap; ad.res_cap = a->res_len;
-        ad.status = reinterpret_cast<int32_t *>(ws);
-        err = bd::launch_advance(ad, stream);
         if (err != cudaSuccess) return BD_ERR_CUDA;
     }
 

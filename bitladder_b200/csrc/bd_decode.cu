@@ -471,6 +471,9 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
     uint32_t phase = 0;    // parity of both barriers: one completion each per consumed block
     bool aborted = false;
 
+    // Launched behind a rotary kernel, everything so far ran beside it: what it writes is read from here on.
+    if (RAGGED && p.after_rope) asm volatile("griddepcontrol.wait;" ::: "memory");
+
     Segment sg;
     while (walk.next(sg)) {
         const int ib = sg.ib;
@@ -1498,9 +1501,17 @@ static cudaError_t launch_r(const DecodeParams &p, const CUtensorMap &kmap, cons
         if (err != cudaSuccess) return err;
         configured[dev] = true;
     }
-    const unsigned grid = unsigned(p.part.R) * unsigned(p.h_k);
-    kern<<<grid, C::THREADS, C::SMEM, stream>>>(p, kmap, vmap);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(p.part.R) * unsigned(p.h_k));
+    cfg.blockDim = dim3(C::THREADS);
+    cfg.dynamicSmemBytes = C::SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;       // staged behind the rotary kernel
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = p.after_rope ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, p, kmap, vmap);
 }
 
 template <int BITS, int GROUP, int NQT, int TWO>
@@ -1531,45 +1542,6 @@ cudaError_t launch_decode(const DecodeParams &p, const CUtensorMap &kmap, const 
     if (bits == 4 && group == 32) return launch_bg<4, 32>(p, kmap, vmap, stream);
     if (bits == 2 && group == 32) return launch_bg<2, 32>(p, kmap, vmap, stream);
     return cudaErrorInvalidValue;
-}
-
-// ---------------------------------------------------------------------------
-// After a step that appended a token to every tail: the lengths the next step will read.  Mirrors
-// what the decode kernel did (a tail that was already full took no token) and what the roll-over
-// pack did (a tail that reached one pack block was packed, room permitting).
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) bd_advance_kernel(const AdvanceParams p) {
-    // staged early behind the roll-over pack kernel (which itself waits for the decode kernel): the lengths
-    // may only move when both are done
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= p.b) return;
-    const int cap = min(kTailMax, p.res_cap);
-    int r = min(max(p.res_lens[i], 0), cap);
-    if (r < cap) r += 1;                                  // the decode kernel filed this step's token
-    if (r == p.block_tokens) {
-        const int cs = p.cache_seqlens[i];
-        if (cs >= 0 && cs % p.block_tokens == 0 && cs + p.block_tokens <= p.s_cap) {
-            p.cache_seqlens[i] = cs + p.block_tokens;
-            r = 0;
-        } else {
-            atomicExch(p.status, BD_ERR_CAPACITY);
-        }
-    }
-    p.res_lens[i] = r;
-}
-
-cudaError_t launch_advance(const AdvanceParams &p, cudaStream_t stream) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned((p.b + 255) / 256));
-    cfg.blockDim = dim3(256);
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;     // staged behind the kernel before it
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, bd_advance_kernel, p);
 }
 
 cudaError_t launch_prefix(const PrefixParams &p, cudaStream_t stream) {

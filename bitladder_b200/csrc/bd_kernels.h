@@ -31,15 +31,12 @@ struct PackParams {
     // Roll-over of full tails (null: plain pack).  The source rows are a sequence's tail buffer; a
     // sequence is packed only if roll_res_lens[ib] + 1 equals one pack block (this step's token filled
     // the tail), into the block that starts at token roll_cache_seqlens[ib] (room permitting).
-    const int32_t *roll_res_lens;
-    const int32_t *roll_cache_seqlens;
-    int32_t roll_s_cap;
-};
-
-struct AdvanceParams {
-    int32_t *cache_seqlens, *res_lens;
-    int32_t b, block_tokens, s_cap, res_cap;
-    int32_t *status;
+    // The CTA of a sequence that has read its lengths last then moves them on.
+    int32_t *roll_res_lens;
+    int32_t *roll_cache_seqlens;
+    int32_t *roll_arrivals;       // [b * h_k], the first of every sequence counts its CTAs; zero between steps
+    int32_t *roll_status;
+    int32_t roll_s_cap, roll_res_cap;
 };
 
 // ---------------------------------------------------------------------------
@@ -204,6 +201,7 @@ BD_HD void for_each_part(const Partition &pt, int ib, F &&f) {
 struct DecodeParams {
     const void *q;
     int64_t q_stride_b, q_stride_h;
+    int32_t after_rope;           // q, k_new and v_new come from the rotary kernel that this launch overlaps
     const uint16_t *k_params;     // viewed as fp16
     const uint16_t *v_params;
     int64_t k_params_stride_b;    // in fp16 elements
@@ -301,7 +299,6 @@ int fill_exchange_params(const ::bd_exchange_args *a, ExchangeParams &p);
 
 cudaError_t launch_pack(const PackParams &p, int bits, int group, int dtype, cudaStream_t stream);
 cudaError_t launch_prefix(const PrefixParams &p, cudaStream_t stream);
-cudaError_t launch_advance(const AdvanceParams &p, cudaStream_t stream);
 cudaError_t launch_merge_parts(const DecodeParams &p, bool early, cudaStream_t stream);
 cudaError_t launch_decode(const DecodeParams &p, const CUtensorMap &kmap, const CUtensorMap &vmap,
                           int bits, int group, cudaStream_t stream);

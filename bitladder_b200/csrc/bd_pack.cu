@@ -153,14 +153,34 @@ bd_pack_kernel(const PackParams p) {
     const int blk = blockIdx.y, ib = blockIdx.z;
     int dst_off = p.dst_token_offset;
     if (p.roll_res_lens != nullptr) {          // roll-over: only sequences whose tail this step's token filled
-        // The roll-over is staged early behind the decode kernel that files the token, and the kernel that moves
-        // the lengths on is staged behind this one: every CTA waits for the decode kernel before it reads a tail
-        // row or leaves (a CTA that left without waiting would let the lengths move under that kernel).
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        // Staged early behind the decode kernel that files the token: every CTA waits for that kernel before it reads a
+        // length or a tail row.  The lengths move only when all CTAs of the sequence have read them (the kernel in
+        // front is done with them by then); a kernel of its own for that cost 0.4 us more per decoder step, and its launch.
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        if (p.roll_res_lens[ib] + 1 != NB) return;
+        const int tail = p.roll_res_lens[ib];
         dst_off = p.roll_cache_seqlens[ib];
-        if (dst_off < 0 || dst_off % NB != 0 || dst_off + NB > p.roll_s_cap) return;   // no room: reported by the advance kernel
+        __syncthreads();
+        if (tid == 0) {
+            int32_t *arrivals = p.roll_arrivals + static_cast<int64_t>(ib) * p.h_k;
+            if (atomicAdd(arrivals, 1) == int(gridDim.x) - 1) {
+                *arrivals = 0;
+                // Mirrors what the decode kernel did (a tail that was already full took no token) and what the CTAs
+                // of this one do (a tail that reached one pack block is packed, room permitting).
+                int r = min(max(tail, 0), p.roll_res_cap), cs = dst_off;
+                if (r < p.roll_res_cap) r += 1;
+                if (r == NB) {
+                    if (cs >= 0 && cs % NB == 0 && cs + NB <= p.roll_s_cap) {
+                        p.roll_cache_seqlens[ib] = cs + NB;
+                        r = 0;
+                    } else {
+                        atomicExch(p.roll_status, BD_ERR_CAPACITY);
+                    }
+                }
+                p.roll_res_lens[ib] = r;
+            }
+        }
+        if (tail + 1 != NB) return;
+        if (dst_off < 0 || dst_off % NB != 0 || dst_off + NB > p.roll_s_cap) return;   // no room: reported above
     }
     const int dst_blk = blk + dst_off / NB;
     const uint16_t *kin = static_cast<const uint16_t *>(p.k);

@@ -27,6 +27,8 @@ __device__ __forceinline__ void rope_store(void *p, int64_t i, float v, bool bf1
 // grid (q heads + 2 x KV heads, b), 64 threads: thread t is pair t of one head's row: a q head, then a k head
 // (both rotated), then a v head (copied beside them)
 __global__ void __launch_bounds__(64) bd_rope_kernel(const RopeParams p) {
+    // the decode kernel behind this one may set itself up; it waits for this grid before it reads a rotated row
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int ib = blockIdx.y;
     const bool bf16 = p.dtype == BD_BF16;
     const int cached = p.cache_seqlens ? max(p.cache_seqlens[ib], 0) : p.s;

@@ -180,7 +180,7 @@ typedef struct bd_decode_args {
                                  res_lens[ib] = 0.  This is the roll-over of the reference's residual scheme
                                  (its imgs/scheme.png; residual_block_size in kernel_traits.h:76-85, not wired up
                                  in its snapshot).  Needs cache_seqlens and res_lens (both are then WRITTEN), a tail
-                                 buffer of at least NB rows, no block_table.  Runs as two small kernels behind the
+                                 buffer of at least NB rows, no block_table.  Runs as one small kernel behind the
                                  decode kernel on the same stream.  No room left for the block: BD_ERR_CAPACITY in
                                  the status word, the tail stays full. */
     uint32_t spin_limit;      /* polls a device-side wait on a copy may take before it gives up with
