@@ -18,7 +18,7 @@ BD_PACK_APPROX_DIV = 1
 BD_ERR_INVALID, BD_ERR_TIMEOUT, BD_ERR_SCRATCH_LIMIT, BD_ERR_PAGE, BD_ERR_CAPACITY, BD_ERR_POSITION = -1, -7, -8, -9, -10, -11
 
 EXPORTS = (
-    "bd_pack", "bd_decode", "bd_decode_workspace_bytes", "bd_plan_splits", "bd_decode_plan",
+    "bd_pack", "bd_prefill", "bd_decode", "bd_decode_workspace_bytes", "bd_plan_splits", "bd_decode_plan",
     "bd_combine", "bd_read_status", "bd_strerror", "bd_version",
     "bd_partition_segments", "bd_partition_parts",
     "bd_decode_noalloc", "bd_noalloc_scratch_bytes",
@@ -39,6 +39,15 @@ class PackArgs(C.Structure):
         ("dst_token_offset", C.c_int32),
         ("bits", C.c_int32), ("group", C.c_int32), ("dtype", C.c_int32),
         ("flags", C.c_int32),
+    ]
+
+
+class PrefillArgs(C.Structure):
+    _fields_ = [
+        ("pack", PackArgs),
+        ("k_tail", C.c_void_p), ("v_tail", C.c_void_p),
+        ("tail_stride_b", C.c_int64), ("tail_stride_s", C.c_int64), ("tail_stride_h", C.c_int64),
+        ("cache_seqlens", C.c_void_p), ("res_lens", C.c_void_p),
     ]
 
 
@@ -114,6 +123,8 @@ def load():
             raise RuntimeError(f"{LIB_PATH} does not export {name}; rebuild it")
     lib.bd_pack.argtypes = [C.POINTER(PackArgs), C.c_void_p]
     lib.bd_pack.restype = C.c_int
+    lib.bd_prefill.argtypes = [C.POINTER(PrefillArgs), C.c_void_p]
+    lib.bd_prefill.restype = C.c_int
     lib.bd_decode.argtypes = [C.POINTER(DecodeArgs), C.c_void_p]
     lib.bd_decode.restype = C.c_int
     lib.bd_decode_noalloc.argtypes = [C.POINTER(DecodeArgs), C.c_void_p]

@@ -156,6 +156,24 @@ def _check_packed(k_pack, k_params, v_pack, v_params, num_bits, group_size):
     return b, s_cap, h_k, d
 
 
+def _pack_args(k_cache, k_pack, k_params, v_cache, v_pack, v_params, group_size, num_bits, dst_token_offset=0,
+               reference_fast_math=False) -> "_lib.PackArgs":
+    b, s, h_k, d = k_cache.shape
+    return _lib.PackArgs(
+        k=k_cache.data_ptr(), v=v_cache.data_ptr(),
+        k_stride_b=k_cache.stride(0), k_stride_s=k_cache.stride(1), k_stride_h=k_cache.stride(2),
+        v_stride_b=v_cache.stride(0), v_stride_s=v_cache.stride(1), v_stride_h=v_cache.stride(2),
+        k_pack=k_pack.data_ptr(), k_params=k_params.data_ptr(),
+        v_pack=v_pack.data_ptr(), v_params=v_params.data_ptr(),
+        k_pack_stride_b=k_pack.stride(0), k_params_stride_b=k_params.stride(0),
+        v_pack_stride_b=v_pack.stride(0),
+        v_params_stride_b=v_params.stride(0), v_params_stride_g=v_params.stride(1),
+        v_params_stride_h=v_params.stride(2),
+        b=b, s=s, h_k=h_k, d=d, dst_token_offset=dst_token_offset,
+        bits=num_bits, group=group_size, dtype=_dtype_code(k_cache.dtype),
+        flags=_lib.BD_PACK_APPROX_DIV if reference_fast_math else 0)
+
+
 def kvcache_pack_int(k_cache: torch.Tensor, k_pack: torch.Tensor, k_params: torch.Tensor,
                      v_cache: torch.Tensor, v_pack: torch.Tensor, v_params: torch.Tensor,
                      opt_block_table: Optional[torch.Tensor] = None,
@@ -201,19 +219,7 @@ def kvcache_pack_int(k_cache: torch.Tensor, k_pack: torch.Tensor, k_params: torc
     _require(dst_token_offset + s <= s_cap, "packed buffers are too small for this many tokens")
     if s == 0:
         return
-    a = _lib.PackArgs(
-        k=k_cache.data_ptr(), v=v_cache.data_ptr(),
-        k_stride_b=k_cache.stride(0), k_stride_s=k_cache.stride(1), k_stride_h=k_cache.stride(2),
-        v_stride_b=v_cache.stride(0), v_stride_s=v_cache.stride(1), v_stride_h=v_cache.stride(2),
-        k_pack=k_pack.data_ptr(), k_params=k_params.data_ptr(),
-        v_pack=v_pack.data_ptr(), v_params=v_params.data_ptr(),
-        k_pack_stride_b=k_pack.stride(0), k_params_stride_b=k_params.stride(0),
-        v_pack_stride_b=v_pack.stride(0),
-        v_params_stride_b=v_params.stride(0), v_params_stride_g=v_params.stride(1),
-        v_params_stride_h=v_params.stride(2),
-        b=b, s=s, h_k=h_k, d=d, dst_token_offset=dst_token_offset,
-        bits=num_bits, group=group_size, dtype=_dtype_code(k_cache.dtype),
-        flags=_lib.BD_PACK_APPROX_DIV if reference_fast_math else 0)
+    a = _pack_args(k_cache, k_pack, k_params, v_cache, v_pack, v_params, group_size, num_bits, dst_token_offset, reference_fast_math)
     with torch.cuda.device(k_cache.device):
         _lib.check(_lib.load().bd_pack(C.byref(a), _stream(k_cache.device)), "bd_pack")
 

@@ -329,14 +329,16 @@ int bd_plan_splits(int b, int h_k, int64_t max_s, int bits, int sm_count, int ct
     return plan_rows(b, h_k, max_s, bits, sm_count, ctas_per_sm);
 }
 
-int bd_pack(const bd_pack_args *a, bd_stream_t stream) {
+// bd_pack; with `f` the prompts of a batch (f->pack is a).
+static int pack_rows(const bd_pack_args *a, const bd_prefill_args *f, bd_stream_t stream) {
     if (!a || !a->k || !a->v || !a->k_pack || !a->k_params || !a->v_pack || !a->v_params) return BD_ERR_INVALID;
     if (a->b <= 0 || a->h_k <= 0 || a->s < 0 || a->dst_token_offset < 0) return BD_ERR_INVALID;
     if (!config_supported(a->bits, a->group, a->d)) return BD_ERR_UNSUPPORTED;
     if (a->dtype != BD_FP16 && a->dtype != BD_BF16) return BD_ERR_UNSUPPORTED;
     const int nb = pack_block_tokens(a->bits);
-    if (a->s % nb || a->dst_token_offset % nb) return BD_ERR_INVALID;
-    if (a->s / nb > 65535 || a->b > 65535) return BD_ERR_INVALID;      // grid.y, grid.z
+    if ((!f && a->s % nb) || a->dst_token_offset % nb) return BD_ERR_INVALID;
+    if (f && (!f->k_tail || !f->v_tail || !f->cache_seqlens || !f->res_lens || a->dst_token_offset != 0)) return BD_ERR_INVALID;
+    if ((int64_t(a->s) + nb - 1) / nb > 65535 || a->b > 65535) return BD_ERR_INVALID;      // grid.y, grid.z
     // 16-byte vector loads of the inputs and 16-byte stores of the V codes
     if ((reinterpret_cast<uintptr_t>(a->k) | reinterpret_cast<uintptr_t>(a->v) |
          reinterpret_cast<uintptr_t>(a->k_pack) | reinterpret_cast<uintptr_t>(a->v_pack) |
@@ -344,6 +346,8 @@ int bd_pack(const bd_pack_args *a, bd_stream_t stream) {
         return BD_ERR_ALIGNMENT;
     if ((a->k_stride_b | a->k_stride_s | a->k_stride_h | a->v_stride_b | a->v_stride_s | a->v_stride_h |
          a->k_pack_stride_b | a->v_pack_stride_b) & 7)
+        return BD_ERR_ALIGNMENT;
+    if (f && (!aligned16(f->k_tail) || !aligned16(f->v_tail) || ((f->tail_stride_b | f->tail_stride_s | f->tail_stride_h) & 7)))
         return BD_ERR_ALIGNMENT;
     if (a->s == 0) return BD_OK;
     DeviceInfo info;
@@ -362,8 +366,20 @@ int bd_pack(const bd_pack_args *a, bd_stream_t stream) {
     p.v_params_stride_h = a->v_params_stride_h;
     p.b = a->b; p.s = a->s; p.h_k = a->h_k; p.dst_token_offset = a->dst_token_offset;
     p.approx_div = (a->flags & BD_PACK_APPROX_DIV) ? 1 : 0;
+    if (f) {
+        p.fill_cache_seqlens = f->cache_seqlens; p.fill_res_lens = f->res_lens;
+        p.k_tail = f->k_tail; p.v_tail = f->v_tail;
+        p.tail_stride_b = f->tail_stride_b; p.tail_stride_s = f->tail_stride_s; p.tail_stride_h = f->tail_stride_h;
+    }
     cudaError_t err = bd::launch_pack(p, a->bits, a->group, a->dtype, static_cast<cudaStream_t>(stream));
     return err == cudaSuccess ? BD_OK : BD_ERR_CUDA;
+}
+
+int bd_pack(const bd_pack_args *a, bd_stream_t stream) { return pack_rows(a, nullptr, stream); }
+
+int bd_prefill(const bd_prefill_args *f, bd_stream_t stream) {
+    if (!f) return BD_ERR_INVALID;
+    return pack_rows(&f->pack, f, stream);
 }
 
 size_t bd_decode_workspace_bytes(const bd_decode_args *a) {

@@ -111,6 +111,9 @@ __device__ __forceinline__ void param_slot(int g, int c, int &row, int &col) {
     }
 }
 
+__device__ __forceinline__ const uint16_t *kin_of(const PackParams &p) { return static_cast<const uint16_t *>(p.k); }
+__device__ __forceinline__ const uint16_t *vin_of(const PackParams &p) { return static_cast<const uint16_t *>(p.v); }
+
 // A block of a head is the work of 2 * kPackSplit CTAs of 128 threads: kPackSplit share its K by channels, as many its
 // V by tokens.  A CTA is three phases (load, reduce, quantize and store) that cannot overlap inside it, so what keeps
 // HBM busy is eight small CTAs per SM in different phases (1024 threads of 64 registers), each thread with 32 words
@@ -182,9 +185,26 @@ bd_pack_kernel(const PackParams p) {
         if (tail + 1 != NB) return;
         if (dst_off < 0 || dst_off % NB != 0 || dst_off + NB > p.roll_s_cap) return;   // no room: reported above
     }
+    if (p.fill_cache_seqlens != nullptr) {
+        const int full = min(max(p.fill_cache_seqlens[ib], 0), p.s) / NB;
+        if (blk >= full) {
+            // behind the whole blocks: one block's worth of rows to the tail, 16 bytes a thread, the K CTAs and the V CTAs
+            // of a head a share of the rows each
+            const int rest = blk > full ? 0 : min(min(p.fill_res_lens[ib], NB), p.s - blk * NB);
+            const bool is_k = blockIdx.x < SPLIT * p.h_k;
+            const int x = is_k ? blockIdx.x : blockIdx.x - SPLIT * p.h_k;
+            const int ih = x / SPLIT, part = x % SPLIT, c = 8 * (tid & 15);
+            const uint16_t *src = is_k ? kin_of(p) + ib * p.k_stride_b + ih * p.k_stride_h : vin_of(p) + ib * p.v_stride_b + ih * p.v_stride_h;
+            const int64_t step = is_k ? p.k_stride_s : p.v_stride_s;
+            uint16_t *dst = static_cast<uint16_t *>(is_k ? p.k_tail : p.v_tail) + ib * p.tail_stride_b + ih * p.tail_stride_h;
+            for (int t = part * (NB / SPLIT) + (tid >> 4); t < min(rest, (part + 1) * (NB / SPLIT)); t += NTHREADS / 16)
+                *reinterpret_cast<uint4 *>(dst + t * p.tail_stride_s + c) =
+                    __ldg(reinterpret_cast<const uint4 *>(src + (int64_t(blk) * NB + t) * step + c));
+            return;
+        }
+    }
     const int dst_blk = blk + dst_off / NB;
-    const uint16_t *kin = static_cast<const uint16_t *>(p.k);
-    const uint16_t *vin = static_cast<const uint16_t *>(p.v);
+    const uint16_t *kin = kin_of(p), *vin = vin_of(p);
 
     // ------------------------------------------------------------------ K
     if (blockIdx.x < SPLIT * p.h_k) {
@@ -381,7 +401,7 @@ template <int BITS, int GROUP, bool BF16>
 static cudaError_t launch_pack_t(const PackParams &p, cudaStream_t stream) {
     constexpr int NB = 32 * (16 / BITS);
     constexpr int NTHREADS = kPackThreads<BITS>;
-    dim3 grid(2 * kPackSplit<BITS> * p.h_k, p.s / NB, p.b);
+    dim3 grid(2 * kPackSplit<BITS> * p.h_k, (p.s + NB - 1) / NB, p.b);       // (whole blocks, except for prompts)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(NTHREADS);

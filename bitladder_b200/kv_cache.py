@@ -18,12 +18,14 @@ device keeps them itself, roll-over included, and the mirror is plain arithmetic
 """
 from __future__ import annotations
 
+import ctypes as C
 from operator import add
 from typing import List, Optional, Sequence
 
 import torch
 
-from .bit_decode_interface import (alloc_packed_cache, fwd_kvcache_int, kvcache_pack_int, pack_block_tokens)
+from . import _lib
+from .bit_decode_interface import (_pack_args, _stream, alloc_packed_cache, fwd_kvcache_int, kvcache_pack_int, pack_block_tokens)
 
 __all__ = ["PackedKVCache"]
 
@@ -48,8 +50,8 @@ class PackedKVCache:
         # lengths: host mirror (exact) and device copies the decode kernel reads
         self._packed: List[int] = [0] * batch
         self._tail: List[int] = [0] * batch
-        self.cache_seqlens = torch.zeros(batch, dtype=torch.int32, device=self.device)
-        self.res_lens = torch.zeros(batch, dtype=torch.int32, device=self.device)
+        self._lengths = torch.zeros(2, batch, dtype=torch.int32, device=self.device)
+        self.cache_seqlens, self.res_lens = self._lengths.unbind()
 
     # ------------------------------------------------------------------ lengths
     def seqlens(self) -> List[int]:
@@ -57,8 +59,20 @@ class PackedKVCache:
         return [p + t for p, t in zip(self._packed, self._tail)]
 
     def _push_lengths(self) -> None:
-        self.cache_seqlens.copy_(torch.tensor(self._packed, dtype=torch.int32), non_blocking=True)
-        self.res_lens.copy_(torch.tensor(self._tail, dtype=torch.int32), non_blocking=True)
+        self._lengths.copy_(torch.tensor([self._packed, self._tail], dtype=torch.int32), non_blocking=True)
+
+    def _fill(self, k: torch.Tensor, v: torch.Tensor) -> bool:
+        """The prompts into blocks and tails in one launch, by the lengths on the device; False for rows the kernel does
+        not take (strides, alignment)."""
+        if not (k.is_cuda and k.device == v.device == self.k_pack.device and k.stride(-1) == v.stride(-1) == 1):
+            return False
+        t = self.k_tail
+        a = _lib.PrefillArgs(
+            _pack_args(k, self.k_pack, self.k_params, v, self.v_pack, self.v_params, self.group_size, self.num_bits),
+            t.data_ptr(), self.v_tail.data_ptr(), t.stride(0), t.stride(1), t.stride(2),
+            self.cache_seqlens.data_ptr(), self.res_lens.data_ptr())
+        with torch.cuda.device(k.device):
+            return _lib.load().bd_prefill(C.byref(a), _stream(k.device)) == _lib.BD_OK
 
     # ------------------------------------------------------------------ filling
     def prefill(self, k: torch.Tensor, v: torch.Tensor, seqlens: Optional[Sequence[int]] = None) -> None:
@@ -76,6 +90,11 @@ class PackedKVCache:
         if any(n > self.capacity for n in lens):
             raise RuntimeError("prompt longer than the cache capacity")
         nb = self.block
+        self._packed = [n // nb * nb for n in lens]
+        self._tail = [n % nb for n in lens]
+        self._push_lengths()
+        if self._fill(k, v):
+            return
         if len(set(lens)) == 1:                       # one launch for the whole batch
             full = lens[0] // nb * nb
             if full:
@@ -94,8 +113,6 @@ class PackedKVCache:
             if rest:
                 self.k_tail[ib, :rest].copy_(k[ib, full:n])
                 self.v_tail[ib, :rest].copy_(v[ib, full:n])
-            self._packed[ib], self._tail[ib] = full, rest
-        self._push_lengths()
 
     def _roll_full_tails(self) -> None:
         """Pack every tail that is full as its sequence's next block (one ``kvcache_pack_int`` call per

@@ -108,6 +108,22 @@ typedef struct bd_pack_args {
 int bd_pack(const bd_pack_args *args, bd_stream_t stream);
 
 /*
+ * The prompts of a batch into a growing cache, in one launch: of sequence ib the first cache_seqlens[ib] tokens of
+ * pack.k / pack.v (a multiple of NB, at most pack.s) are quantize-packed as bd_pack does it, and the res_lens[ib]
+ * rows behind them (fewer than NB) copied to rows 0.. of its tail buffers.  pack.s: token rows of k and v, any
+ * number; pack.dst_token_offset must be 0.  The lengths are read on the device and bounded by pack.s there.  No
+ * counterpart in the reference, whose residual scheme (imgs/scheme.png) is not wired up in its snapshot.
+ */
+typedef struct bd_prefill_args {
+    bd_pack_args pack;
+    void *k_tail, *v_tail;    /* (b, at least NB rows, h_k, d), the type of k and v */
+    int64_t tail_stride_b, tail_stride_s, tail_stride_h;
+    const int32_t *cache_seqlens, *res_lens;    /* (b), device */
+} bd_prefill_args;
+
+int bd_prefill(const bd_prefill_args *args, bd_stream_t stream);
+
+/*
  * One decode-attention step over the packed cache.  Replaces fwd_kvcache_i2 /
  * fwd_kvcache_i4 (reference: csrc/bit_decode/decode_api.cpp:301-441; split-KV
  * launch csrc/bit_decode/src/flash_fwd_launch_template.h:103-146, kernel body

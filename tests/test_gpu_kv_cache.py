@@ -192,3 +192,36 @@ def test_a_full_cache_is_reported_not_overrun():
     assert _lib.load().bd_read_status(ws.data_ptr(), torch.cuda.current_stream().cuda_stream) == _lib.BD_ERR_CAPACITY
     assert int(cs[0]) == nb and int(rl[0]) == nb                                # lengths: the tail stays full
     assert all(torch.equal(a, b_) for a, b_ in zip(before, bufs))
+
+
+@pytest.mark.parametrize("bits,group,dtype", [(4, 128, "fp16"), (4, 32, "bf16"), (2, 64, "fp16"), (2, 128, "bf16")])
+@pytest.mark.parametrize("strided", [False, True])
+def test_prompts_of_unequal_lengths_in_one_launch(bits, group, dtype, strided, monkeypatch):
+    """The one-launch prefill leaves the same bytes (blocks, tails, untouched rows, lengths) as a pack call and a copy per
+    sequence; rows the kernel does not take (misaligned) go that way by themselves."""
+    from bitladder_b200 import PackedKVCache
+    nb = 32 * (16 // bits)
+    s = 3 * nb + 41
+    lens = [s, 0, 7, nb, 2 * nb - 1, 3 * nb, nb + 64]
+    x = H.gen_qkv(len(lens), s, 12, 6, seed=23, dtype=dtype)
+    k, v = x["k"].cuda(), x["v"].cuda()
+    if strided:
+        k, v = (torch.stack([t, -t], 3).flatten(2, 3)[:, :, ::2] for t in (k, v))
+        assert not k.is_contiguous()
+
+    def filled(k, v):
+        c = PackedKVCache(len(lens), s + 1, 6, 128, bits, group, k.dtype)
+        for t in (c.k_tail, c.v_tail):
+            t.fill_(3)
+        c.prefill(k, v, lens)
+        torch.cuda.synchronize()
+        assert c.seqlens() == lens
+        return [t.view(torch.uint8) for t in (c.k_pack, c.k_params, c.v_pack, c.v_params, c.k_tail, c.v_tail)] + [
+            c.cache_seqlens, c.res_lens]
+
+    assert PackedKVCache(len(lens), s, 6, 128, bits, group, k.dtype)._fill(k, v)
+    one = filled(k, v)
+    monkeypatch.setattr(PackedKVCache, "_fill", lambda *_: False)
+    for a, b in zip(one, filled(k, v)):
+        assert torch.equal(a, b)
+    assert one[-2].tolist() == [n // nb * nb for n in lens] and one[-1].tolist() == [n % nb for n in lens]

@@ -27,7 +27,7 @@ def _forms():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("form,bits,group,dtype", _forms())
+@pytest.mark.parametrize("form,bits,group,dtype", list(_forms()))
 def test_same_bits_as_the_python_path(form, bits, group, dtype, monkeypatch):
     import bitladder_b200 as B
     from bitladder_b200 import bit_decode_interface as I
