@@ -441,6 +441,19 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     part.R = plan.rows;
 
     cudaError_t err;
+    // Whether the first kernel of the step is staged early behind whatever runs in front of it (it waits for that before
+    // it touches global memory).  In a stream a kernel otherwise starts on the next 2 us tick after the one in front is
+    // done (b1, 4096 tokens: 12.3 us a step instead of 10.0; 32 x up to 16384 tokens, 32 heads: 219 instead of 216);
+    // between the kernels of a graph there is no such tick and only small steps gain (b1, 2048 tokens, 32 heads 10.8 ->
+    // 9.7 us, b8, 32768 tokens 56.6 -> 57.5).  CTAs that are placed as SMs fall free lose the order in which the heads of a
+    // row stream the same tokens together, which costs long steps of one CTA per SM more than the tick (blocks per
+    // warp in a stream: 10: 57.9 -> 57.1 us, 19: 102.0 -> 104.2, 76: 361 -> 382).
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) return BD_ERR_CUDA;
+    const bool in_graph = capture != cudaStreamCaptureStatusNone;
+    const int64_t warps = int64_t(plan.rows) * bd::decode_warps(a->bits, a->group, a->h / a->h_k, plan.two_ctas);
+    const bool early = (!in_graph && plan.two_ctas) ||
+                       int64_t(a->b) * bd::seq_blocks(a->s, a->s, nb) <= (in_graph ? 2 : 12) * warps;
     const bool inline_table = plan.ragged && a->b <= bd::kInlineSeqs && !x;      // (the exchange kernel reads the table)
     if (plan.ragged && !inline_table) {
         bd::PrefixParams pp;
@@ -515,12 +528,14 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
         rp.rotary_dim = a->rotary_dim; rp.interleaved = a->rotary_interleaved ? 1 : 0;
         rp.positions = a->rotary_positions; rp.dtype = a->dtype;
         rp.status = reinterpret_cast<int32_t *>(ws);
+        rp.early = early ? 1 : 0;
         err = bd::launch_rope(rp, stream);
         if (err != cudaSuccess) return BD_ERR_CUDA;
         p.q = rp.q_out; p.q_stride_b = int64_t(a->h) * 128; p.q_stride_h = 128;
         p.after_rope = 1;
         p.k_new = rp.k_out; p.v_new = rp.v_out; p.new_stride_b = int64_t(a->h_k) * 128; p.new_stride_h = 128;
     }
+    p.early = (early || p.after_rope) ? 1 : 0;
     p.defer_merge = (x || plan.rows > 4 * a->b) ? 1 : 0;
     p.leave_parts = x ? 1 : 0;
     p.two_ctas = plan.two_ctas;

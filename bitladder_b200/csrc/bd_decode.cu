@@ -361,6 +361,9 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
     }
     BD_TRACE_MARK(25);
     // The warps are the rows of the partition with kWarps times the CTA rows.
+    // Staged early (see launch_r), the set-up up to here ran beside the end of the kernel in front.  Behind a rotary kernel
+    // the wait comes later: that kernel lets this one start only when everything in front of it is done.
+    if (RAGGED && !p.after_rope) asm volatile("griddepcontrol.wait;" ::: "memory");
     Partition part = p.part;
     if constexpr (!RAGGED) part.table = nullptr;
     const int32_t *cache_seqlens = RAGGED ? p.cache_seqlens : nullptr, *res_lens = RAGGED ? p.res_lens : nullptr;
@@ -440,6 +443,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
     BlockCursor ld;                 // next block to copy into this warp's tiles
     ld.init(walk, cache_seqlens, p.s, NB);
     BD_TRACE_MARK(27);
+    if constexpr (!RAGGED) asm volatile("griddepcontrol.wait;" ::: "memory");     // (nothing in global memory was read so far)
     if (ld.valid && lane == 0) {
         issue_k(ld.sg.ib, ld.u);
         issue_v(ld.sg.ib, ld.u);
@@ -1507,10 +1511,10 @@ static cudaError_t launch_r(const DecodeParams &p, const CUtensorMap &kmap, cons
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = stream;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;       // staged behind the rotary kernel
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = p.after_rope ? 1 : 0;
+    cfg.numAttrs = p.early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, p, kmap, vmap);
 }
 

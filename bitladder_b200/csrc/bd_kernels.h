@@ -206,6 +206,7 @@ BD_HD void for_each_part(const Partition &pt, int ib, F &&f) {
 struct DecodeParams {
     const void *q;
     int64_t q_stride_b, q_stride_h;
+    int32_t early;                // staged behind the kernel in front of it (programmatic dependent launch)
     int32_t after_rope;           // q, k_new and v_new come from the rotary kernel that this launch overlaps
     const uint16_t *k_params;     // viewed as fp16
     const uint16_t *v_params;
@@ -278,6 +279,7 @@ struct RopeParams {
     int32_t s, res_len;               // lengths of every sequence when the arrays are null
     int32_t b, h, h_k;
     int32_t rotary_dim, interleaved, positions, dtype;
+    int32_t early;                    // staged behind the kernel in front of it
     int32_t *status;
 };
 cudaError_t launch_rope(const RopeParams &p, cudaStream_t stream);

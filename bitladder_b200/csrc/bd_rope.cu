@@ -27,7 +27,9 @@ __device__ __forceinline__ void rope_store(void *p, int64_t i, float v, bool bf1
 // grid (q heads + 2 x KV heads, b), 64 threads: thread t is pair t of one head's row: a q head, then a k head
 // (both rotated), then a v head (copied beside them)
 __global__ void __launch_bounds__(64) bd_rope_kernel(const RopeParams p) {
-    // the decode kernel behind this one may set itself up; it waits for this grid before it reads a rotated row
+    // Everything in front is done from here on; the decode kernel behind this one may start then, and waits for this grid
+    // before it reads a rotated row.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int ib = blockIdx.y;
     const bool bf16 = p.dtype == BD_BF16;
@@ -77,8 +79,16 @@ __global__ void __launch_bounds__(64) bd_rope_kernel(const RopeParams p) {
 
 cudaError_t launch_rope(const RopeParams &p, cudaStream_t stream) {
     static_assert(kHeadDim / 2 == 64, "one thread per pair of a 128-dim head");
-    bd_rope_kernel<<<dim3(unsigned(p.h + 2 * p.h_k), unsigned(p.b)), 64, 0, stream>>>(p);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(p.h + 2 * p.h_k), unsigned(p.b));
+    cfg.blockDim = dim3(64);
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = p.early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, bd_rope_kernel, p);
 }
 
 }  // namespace bd
