@@ -449,8 +449,9 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     // row stream the same tokens together, which costs long steps of one CTA per SM more than the tick (blocks per
     // warp in a stream: 10: 57.9 -> 57.1 us, 19: 102.0 -> 104.2, 76: 361 -> 382).
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) return BD_ERR_CUDA;
-    const bool in_graph = capture != cudaStreamCaptureStatusNone;
+    const bool asked = cudaStreamIsCapturing(stream, &capture) == cudaSuccess;
+    if (!asked) (void)cudaGetLastError();            // (the legacy stream beside a capture: the launches say what is wrong)
+    const bool in_graph = !asked || capture != cudaStreamCaptureStatusNone;
     const int64_t warps = int64_t(plan.rows) * bd::decode_warps(a->bits, a->group, a->h / a->h_k, plan.two_ctas);
     const bool early = (!in_graph && plan.two_ctas) ||
                        int64_t(a->b) * bd::seq_blocks(a->s, a->s, nb) <= (in_graph ? 2 : 12) * warps;
