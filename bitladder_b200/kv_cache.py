@@ -61,16 +61,16 @@ class PackedKVCache:
     def _push_lengths(self) -> None:
         self._lengths.copy_(torch.tensor([self._packed, self._tail], dtype=torch.int32), non_blocking=True)
 
-    def _fill(self, k: torch.Tensor, v: torch.Tensor) -> bool:
-        """The prompts into blocks and tails in one launch, by the lengths on the device; False for rows the kernel does
-        not take (strides, alignment)."""
+    def _fill(self, k: torch.Tensor, v: torch.Tensor, packed: List[int], tail: List[int]) -> bool:
+        """The prompts into blocks and tails in one launch, by lengths on the device; False for rows the kernel does
+        not take (strides, alignment).  The lengths are this launch's own: the cache's move only when rows were taken."""
         if not (k.is_cuda and k.device == v.device == self.k_pack.device and k.stride(-1) == v.stride(-1) == 1):
             return False
-        t = self.k_tail
+        t, lengths = self.k_tail, torch.tensor([packed, tail], dtype=torch.int32).to(k.device, non_blocking=True)
         a = _lib.PrefillArgs(
             _pack_args(k, self.k_pack, self.k_params, v, self.v_pack, self.v_params, self.group_size, self.num_bits),
             t.data_ptr(), self.v_tail.data_ptr(), t.stride(0), t.stride(1), t.stride(2),
-            self.cache_seqlens.data_ptr(), self.res_lens.data_ptr())
+            lengths[0].data_ptr(), lengths[1].data_ptr())
         with torch.cuda.device(k.device):
             return _lib.load().bd_prefill(C.byref(a), _stream(k.device)) == _lib.BD_OK
 
@@ -90,11 +90,15 @@ class PackedKVCache:
         if any(n > self.capacity for n in lens):
             raise RuntimeError("prompt longer than the cache capacity")
         nb = self.block
-        self._packed = [n // nb * nb for n in lens]
-        self._tail = [n % nb for n in lens]
+        packed, tail = [n // nb * nb for n in lens], [n % nb for n in lens]
+        if not self._fill(k, v, packed, tail):
+            self._fill_in_parts(k, v, lens)
+        self._packed, self._tail = packed, tail
         self._push_lengths()
-        if self._fill(k, v):
-            return
+
+    def _fill_in_parts(self, k: torch.Tensor, v: torch.Tensor, lens: List[int]) -> None:
+        """The prompts by a pack call and a copy per sequence, or one call where all are equally long."""
+        nb = self.block
         if len(set(lens)) == 1:                       # one launch for the whole batch
             full = lens[0] // nb * nb
             if full:

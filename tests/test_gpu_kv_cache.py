@@ -219,9 +219,32 @@ def test_prompts_of_unequal_lengths_in_one_launch(bits, group, dtype, strided, m
         return [t.view(torch.uint8) for t in (c.k_pack, c.k_params, c.v_pack, c.v_params, c.k_tail, c.v_tail)] + [
             c.cache_seqlens, c.res_lens]
 
-    assert PackedKVCache(len(lens), s, 6, 128, bits, group, k.dtype)._fill(k, v)
+    assert PackedKVCache(len(lens), s, 6, 128, bits, group, k.dtype)._fill(k, v, [n // nb * nb for n in lens], [n % nb for n in lens])
     one = filled(k, v)
     monkeypatch.setattr(PackedKVCache, "_fill", lambda *_: False)
     for a, b in zip(one, filled(k, v)):
         assert torch.equal(a, b)
     assert one[-2].tolist() == [n // nb * nb for n in lens] and one[-1].tolist() == [n % nb for n in lens]
+
+
+@pytest.mark.parametrize("refused", ["cpu", "stride", "misaligned"])
+def test_a_refused_prefill_leaves_the_cache(refused):
+    """Rows that are refused on the host change nothing: lengths (host and device), blocks and tails stay an earlier
+    prompt's."""
+    from bitladder_b200 import PackedKVCache
+    x = H.gen_qkv(2, 300, 8, 2, seed=29)
+    c = PackedKVCache(2, 512, 2)
+    c.prefill(x["k"].cuda(), x["v"].cuda(), [300, 130])
+    state = lambda: [t.clone().view(torch.uint8) for t in (c.k_pack, c.k_params, c.v_pack, c.v_params, c.k_tail, c.v_tail,
+                                                           c.cache_seqlens, c.res_lens)]
+    before, lens = state(), c.seqlens()
+    k = x["k"] if refused == "cpu" else x["k"].cuda().flip(1)
+    if refused == "stride":
+        k = torch.stack([k, k], -1)[..., 0]
+    if refused == "misaligned":
+        k = torch.cat([k.flatten(), k.flatten()[:8]])[1:1 + k.numel()].view(k.shape)
+    with pytest.raises(RuntimeError):
+        c.prefill(k, k, [290, 300])
+    assert c.seqlens() == lens
+    for a, b in zip(before, state()):
+        assert torch.equal(a, b)

@@ -82,3 +82,17 @@ def test_missing_library_is_an_error_not_a_fallback(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))
     with pytest.raises(RuntimeError, match="no CPU fallback"):
         _lib.load()
+
+
+@pytest.mark.parametrize("earlier", [None, [100, 7]])
+def test_a_refused_prefill_leaves_the_lengths(earlier):
+    """Rows that the pack call refuses (here: not on a GPU) change neither the host's nor the device's lengths."""
+    c = B.PackedKVCache(2, 512, 2, device="cpu")
+    rows = torch.ones(2, 300, 2, 128, dtype=torch.float16)
+    if earlier:
+        c.prefill(rows, rows, earlier)                # fits the tails: no kernel is needed
+    before = c.seqlens(), c.cache_seqlens.tolist(), c.res_lens.tolist()
+    for lens in (None, [300, 5]):
+        with pytest.raises(RuntimeError, match="CUDA"):
+            c.prefill(rows, rows, lens)
+        assert (c.seqlens(), c.cache_seqlens.tolist(), c.res_lens.tolist()) == before
