@@ -159,13 +159,21 @@ bd_pack_kernel(const PackParams p) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (p.roll_res_lens != nullptr) {          // roll-over: only sequences whose tail this step's token filled
         // The lengths move only when all CTAs of the sequence have read them (the decode kernel in front is done with
-        // them); a kernel of its own for that cost 0.4 us more per decoder step, and its launch.
-        const int tail = p.roll_res_lens[ib];
-        dst_off = p.roll_cache_seqlens[ib];
+        // them); a kernel of its own for that cost 0.4 us more per decoder step, and its launch.  One thread reads them
+        // for its CTA, so that the fence in front of its count orders the CTA's only reads before the last one's writes.
+        __shared__ int32_t roll[2];
+        if (tid == 0) {
+            roll[0] = p.roll_res_lens[ib];
+            roll[1] = p.roll_cache_seqlens[ib];
+        }
         __syncthreads();
+        const int tail = roll[0];
+        dst_off = roll[1];
         if (tid == 0) {
             int32_t *arrivals = p.roll_arrivals + static_cast<int64_t>(ib) * p.h_k;
+            __threadfence();
             if (atomicAdd(arrivals, 1) == int(gridDim.x) - 1) {
+                __threadfence();
                 *arrivals = 0;
                 // Mirrors what the decode kernel did (a tail that was already full took no token) and what the CTAs
                 // of this one do (a tail that reached one pack block is packed, room permitting).

@@ -248,3 +248,37 @@ def test_a_refused_prefill_leaves_the_cache(refused):
     assert c.seqlens() == lens
     for a, b in zip(before, state()):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("b,h_k,bits", [(48, 8, 4), (40, 8, 2), (1, 1, 4)])
+def test_every_tail_of_a_large_batch_rolls_over_at_once(b, h_k, bits):
+    """More CTAs than the GPU holds, so that the last of a sequence start when the first have long counted in: every CTA
+    packs its share, at the place the step's lengths say, and the lengths move once."""
+    import bitladder_b200 as B
+    nb = B.pack_block_tokens(bits)
+    x = {k: v.cuda() for k, v in H.gen_qkv(b, nb, h_k, h_k, seed=31).items() if isinstance(v, torch.Tensor)}
+    rolls = torch.arange(b, device="cuda") % 5 != 4          # the others have room left in their tails
+    start = torch.full((b,), nb, dtype=torch.int32, device="cuda"), torch.where(rolls, nb - 1, 3).to(torch.int32)
+    cs, rl = (t.clone() for t in start)
+    bufs = B.alloc_packed_cache(b, 3 * nb, h_k, 128, bits, 128)
+    want = B.alloc_packed_cache(b, 3 * nb, h_k, 128, bits, 128)
+    tails = x["k"].clone(), x["v"].clone()
+    new = x["k"][:, -1:].contiguous(), x["v"][:, -1:].contiguous()
+    step = B.DecodeStep(x["q"], *bufs, None, 0.1, "k-channel", 128, bits, k_res=tails[0], v_res=tails[1], res_lens=rl,
+                        cache_seqlens=cs, k_new=new[0], v_new=new[1], advance=True)
+    B.kvcache_pack_int(x["k"], want[0], want[1], x["v"], want[2], want[3], None, None, nb, "k-channel", 128, bits,
+                       dst_token_offset=nb)
+    for t in want:
+        t.view(torch.int32)[~rolls] = 0
+    for _ in range(5):
+        for t in bufs:
+            t.zero_()
+        for t, full in zip(tails, (x["k"], x["v"])):
+            t.copy_(full)
+        cs.copy_(start[0])
+        rl.copy_(start[1])
+        step.step(check=True)
+        assert cs.tolist() == torch.where(rolls, 2 * nb, nb).tolist()
+        assert rl.tolist() == torch.where(rolls, 0, 4).tolist()
+        for t, w in zip(bufs, want):
+            assert torch.equal(t.view(torch.uint8), w.view(torch.uint8))

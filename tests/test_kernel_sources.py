@@ -1,0 +1,34 @@
+"""Rules that the kernels' memory ordering rests on, read off their sources: what breaks them is a race that no run on a
+GPU shows reliably."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "bitladder_b200", "csrc")
+SOURCES = sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")))
+
+
+def _code(path):
+    """The file's lines without their comments."""
+    return [re.sub(r"//.*", "", line) for line in open(path)]
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_an_arrival_is_counted_in_behind_a_fence(path):
+    """What a CTA or warp has read or written has to be ordered before the count that lets the last one go on."""
+    lines = _code(path)
+    for i, line in enumerate(lines):
+        if "atomicAdd(" in line:
+            assert "__threadfence" in "".join(lines[max(0, i - 4):i]), f"line {i + 1}"
+
+
+def test_a_rolling_cta_reads_its_lengths_once():
+    """The last CTA of a sequence overwrites the lengths: one thread of each CTA reads them, in front of its fence."""
+    code = "".join(_code(os.path.join(CSRC, "bd_pack.cu")))
+    for name in ("roll_res_lens", "roll_cache_seqlens"):
+        reads = [m.start() for m in re.finditer(rf"(?<!\w)p\.{name}\[ib\](?! = )", code)]
+        assert len(reads) == 1
+        opened = code.rindex("if (tid == 0) {", 0, reads[0])
+        assert "}" not in code[opened:reads[0]] and reads[0] < code.index("atomicAdd(")
