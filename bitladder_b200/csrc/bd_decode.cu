@@ -519,8 +519,8 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
             // buffers (8 bytes of K and of V per lane), as it came
             const int64_t src = ib * p.new_stride_b + ih * p.new_stride_h + 4 * lane;
             const int64_t dst = ib * p.res_stride_b + ih * p.res_stride_h + int64_t(res_old) * p.res_stride_s + 4 * lane;
-            const uint2 kw = __ldg(reinterpret_cast<const uint2 *>(static_cast<const uint16_t *>(p.k_new) + src));
-            const uint2 vw = __ldg(reinterpret_cast<const uint2 *>(static_cast<const uint16_t *>(p.v_new) + src));
+            const uint2 kw = *reinterpret_cast<const uint2 *>(static_cast<const uint16_t *>(p.k_new) + src);
+            const uint2 vw = *reinterpret_cast<const uint2 *>(static_cast<const uint16_t *>(p.v_new) + src);
             *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(p.k_res_out) + dst) = kw;
             *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(p.v_res_out) + dst) = vw;
         }
@@ -609,6 +609,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
             const bool okA = tA < res_n, okB = tB < res_n;
             // rows past the end are read from the last valid row (in bounds) and zeroed afterwards,
             // so that every load below is unconditional and all of them are in flight together
+            // (plain loads, never __ldg: launched early, this kernel is resident while its predecessor still writes them)
             const int rA = min(tA, res_n - 1), rB = min(tB, res_n - 1);
             const uint16_t *kres = static_cast<const uint16_t *>(p.k_res) + ib * p.res_stride_b + ih * p.res_stride_h;
             const uint16_t *vres = static_cast<const uint16_t *>(p.v_res) + ib * p.res_stride_b + ih * p.res_stride_h;
@@ -623,14 +624,14 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
             uint4 ka[4], kb[4];
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                ka[a] = __ldg(reinterpret_cast<const uint4 *>(kA + 32 * a));
-                kb[a] = __ldg(reinterpret_cast<const uint4 *>(kB + 32 * a));
+                ka[a] = *reinterpret_cast<const uint4 *>(kA + 32 * a);
+                kb[a] = *reinterpret_cast<const uint4 *>(kB + 32 * a);
             }
             uint32_t va[16], vb[16];     // word i: dims 8 i + 2 l, + 1 of the two token rows
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-                va[i] = __ldg(reinterpret_cast<const unsigned int *>(vA + 8 * i));
-                vb[i] = __ldg(reinterpret_cast<const unsigned int *>(vB + 8 * i));
+                va[i] = *reinterpret_cast<const unsigned int *>(vA + 8 * i);
+                vb[i] = *reinterpret_cast<const unsigned int *>(vB + 8 * i);
             }
             if (bf16) {
 #pragma unroll

@@ -155,7 +155,8 @@ bd_pack_kernel(const PackParams p) {
     // heads vary fastest: CTAs that run together read neighbouring 256-byte pieces of the same token rows
     const int blk = blockIdx.y, ib = blockIdx.z;
     int dst_off = p.dst_token_offset;
-    // Staged early behind the kernel in front; nothing in global memory is read or written before that one is done.
+    // Staged early behind the kernel in front; nothing in global memory is read or written before that one is done, and
+    // what it may write is never read through the non-coherent path (__ldg), which promises constant memory.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (p.roll_res_lens != nullptr) {          // roll-over: only sequences whose tail this step's token filled
         // The lengths move only when all CTAs of the sequence have read them (the decode kernel in front is done with
@@ -205,9 +206,15 @@ bd_pack_kernel(const PackParams p) {
             const uint16_t *src = is_k ? kin_of(p) + ib * p.k_stride_b + ih * p.k_stride_h : vin_of(p) + ib * p.v_stride_b + ih * p.v_stride_h;
             const int64_t step = is_k ? p.k_stride_s : p.v_stride_s;
             uint16_t *dst = static_cast<uint16_t *>(is_k ? p.k_tail : p.v_tail) + ib * p.tail_stride_b + ih * p.tail_stride_h;
-            for (int t = part * (NB / SPLIT) + (tid >> 4); t < min(rest, (part + 1) * (NB / SPLIT)); t += NTHREADS / 16)
-                *reinterpret_cast<uint4 *>(dst + t * p.tail_stride_s + c) =
-                    __ldg(reinterpret_cast<const uint4 *>(src + (int64_t(blk) * NB + t) * step + c));
+            constexpr int ROWS = NTHREADS / 16, STEPS = NB / SPLIT / ROWS;      // rows at a time
+            const int t0 = part * (NB / SPLIT) + (tid >> 4);
+            uint4 row[STEPS];
+#pragma unroll
+            for (int i = 0; i < STEPS; ++i)
+                if (t0 + i * ROWS < rest) row[i] = *reinterpret_cast<const uint4 *>(src + (int64_t(blk) * NB + t0 + i * ROWS) * step + c);
+#pragma unroll
+            for (int i = 0; i < STEPS; ++i)
+                if (t0 + i * ROWS < rest) *reinterpret_cast<uint4 *>(dst + (t0 + i * ROWS) * p.tail_stride_s + c) = row[i];
             return;
         }
     }
@@ -226,7 +233,7 @@ bd_pack_kernel(const PackParams p) {
 #pragma unroll
             for (int j = 0; j < P; ++j) {
                 const int t = T * PPT + pi + 32 * j;
-                raw[pi][j] = __ldg(reinterpret_cast<const unsigned int *>(kbase + t * p.k_stride_s));
+                raw[pi][j] = *reinterpret_cast<const unsigned int *>(kbase + t * p.k_stride_s);
             }
         {
             uint32_t pmn[NGK], pmx[NGK];        // both channels at once, in the input format
@@ -316,7 +323,7 @@ bd_pack_kernel(const PackParams p) {
             const int t = tok0 + u * TPI + tsub;
 #pragma unroll
             for (int j = 0; j < P; ++j)
-                raw[u][j] = __ldg(reinterpret_cast<const uint4 *>(vbase + t * p.v_stride_s + DP * j));
+                raw[u][j] = *reinterpret_cast<const uint4 *>(vbase + t * p.v_stride_s + DP * j);
         }
         // Minima and maxima of all the thread's tokens first; then the lanes that share a token divide the (token, dim
         // group) pairs among themselves: one lane works out a pair's scales and hands the inverse to the others.

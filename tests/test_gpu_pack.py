@@ -78,3 +78,20 @@ def test_pack_reference_call_convention():
                        "k-channel", 128, 4)
     torch.cuda.synchronize()
     G.assert_pack_equal((k_pack, k_params, v_pack, v_params), H.oracle_pack(x["k"], x["v"], 4, 128, "fp16"))
+
+
+@pytest.mark.parametrize("s,bits", [(128, 4), (2048, 4), (256, 2)])
+def test_rows_that_the_kernel_in_front_has_just_written(s, bits):
+    """The pack kernel is resident while the kernel in front still writes its rows: it packs what that kernel leaves."""
+    import bitladder_b200 as B
+    x = H.gen_qkv(4, s, 8, 8, seed=37)
+    k, v = x["k"].cuda(), x["v"].cuda()
+    sides = [(k, v), (-2 * k, v - 1)]
+    want = [[t.clone() for t in G.pack_gpu(B, *side, bits, 128)] for side in sides]
+    rows, bufs = (torch.empty_like(k), torch.empty_like(v)), B.alloc_packed_cache(4, s, 8, 128, bits, 128)
+    for i in range(20):
+        for row, side in zip(rows, sides[i % 2]):
+            torch.mul(side, 1, out=row)              # a kernel, not a copy
+        B.kvcache_pack_int(rows[0], bufs[0], bufs[1], rows[1], bufs[2], bufs[3], None, None, s, "k-channel", 128, bits)
+        for got, w in zip([t.clone() for t in bufs], want[i % 2]):
+            assert torch.equal(got.view(torch.uint8), w.view(torch.uint8))

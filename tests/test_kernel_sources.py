@@ -32,3 +32,12 @@ def test_a_rolling_cta_reads_its_lengths_once():
         assert len(reads) == 1
         opened = code.rindex("if (tid == 0) {", 0, reads[0])
         assert "}" not in code[opened:reads[0]] and reads[0] < code.index("atomicAdd(")
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_nothing_is_read_as_constant_memory(path):
+    """A kernel that is staged early is resident while the kernel in front still writes what it will read, so no load may
+    be non-coherent: those promise memory that nobody writes for the kernel's whole life, and may be moved across the
+    wait."""
+    code = "".join(_code(path))
+    assert "__ldg(" not in code and "global.nc" not in code
