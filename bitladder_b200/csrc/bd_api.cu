@@ -533,10 +533,9 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
         err = bd::launch_rope(rp, stream);
         if (err != cudaSuccess) return BD_ERR_CUDA;
         p.q = rp.q_out; p.q_stride_b = int64_t(a->h) * 128; p.q_stride_h = 128;
-        p.after_rope = 1;
         p.k_new = rp.k_out; p.v_new = rp.v_out; p.new_stride_b = int64_t(a->h_k) * 128; p.new_stride_h = 128;
     }
-    p.early = (early || p.after_rope) ? 1 : 0;
+    p.early = (early || a->rotary_dim > 0) ? 1 : 0;
     p.defer_merge = (x || plan.rows > 4 * a->b) ? 1 : 0;
     p.leave_parts = x ? 1 : 0;
     p.two_ctas = plan.two_ctas;

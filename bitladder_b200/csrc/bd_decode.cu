@@ -338,6 +338,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
     }
 #endif
     if ((smem_base & 1023u) != 0) {                      // never seen; refuse rather than read garbage
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         if (tid == 0) atomicExch(p.status, BD_ERR_ALIGNMENT);
         return;
     }
@@ -361,9 +362,10 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
     }
     BD_TRACE_MARK(25);
     // The warps are the rows of the partition with kWarps times the CTA rows.
-    // Staged early (see launch_r), the set-up up to here ran beside the end of the kernel in front.  Behind a rotary kernel
-    // the wait comes later: that kernel lets this one start only when everything in front of it is done.
-    if (RAGGED && !p.after_rope) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // Staged early (see launch_r), the set-up up to here ran beside the end of the kernel in front.  Nothing that an earlier
+    // kernel may have written is read before this wait, not even behind a rotary kernel, which lets this one start only
+    // when everything in front of it is done: that orders the kernels, but makes nothing visible to this one.
+    if constexpr (RAGGED) asm volatile("griddepcontrol.wait;" ::: "memory");
     Partition part = p.part;
     if constexpr (!RAGGED) part.table = nullptr;
     const int32_t *cache_seqlens = RAGGED ? p.cache_seqlens : nullptr, *res_lens = RAGGED ? p.res_lens : nullptr;
@@ -474,9 +476,6 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
     const bool bf16 = p.dtype == BD_BF16;
     uint32_t phase = 0;    // parity of both barriers: one completion each per consumed block
     bool aborted = false;
-
-    // Launched behind a rotary kernel, everything so far ran beside it: what it writes is read from here on.
-    if (RAGGED && p.after_rope) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     Segment sg;
     while (walk.next(sg)) {
@@ -1352,7 +1351,10 @@ __global__ void __launch_bounds__(128, 1) bd_merge_parts_kernel(const DecodePara
     const int ih = hq / p.gq, qrow = hq % p.gq;
     Partition part = p.part;
     __shared__ int2 table[kInlineSeqs + 1];
-    if (p.inline_table) {            // (as in the decode kernel; its lengths were final before that kernel started)
+    // Launched early (see launch_merge_parts), the integer work below runs beside the decode kernel's end, where it needs
+    // nothing from memory; the lengths or the table of a ragged batch are an earlier kernel's, read behind the wait.
+    if (p.part.table != nullptr) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (p.inline_table) {            // (as in the decode kernel)
         table[lane] = ragged_entry(p, p.block_tokens, lane);
         __syncwarp();
         part.table = reinterpret_cast<const int32_t *>(table);
@@ -1370,9 +1372,7 @@ __global__ void __launch_bounds__(128, 1) bd_merge_parts_kernel(const DecodePara
         const bool live = i < nrows && (pr.dense || row_has_part(part, ib, pr.c0 + i));
         return live ? __ldcg(p.part_lse + (slot0 + int64_t(i) * p.h_k) * p.gq + qrow) : -INFINITY;
     };
-    // Launched early (see launch_merge_parts), the integer work above ran beside the decode kernel's end (the
-    // partition and a ragged batch's table were final before that kernel started); everything it wrote is
-    // visible after this.
+    // Everything that the decode kernel wrote is visible after this.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // Up to 32 parts a round: lane i weighs part i, and every lane asks for its 16 bytes of all the parts of
     // the round together with the round's log-sum-exps before any answer is used (the rows do not depend on

@@ -207,7 +207,6 @@ struct DecodeParams {
     const void *q;
     int64_t q_stride_b, q_stride_h;
     int32_t early;                // staged behind the kernel in front of it (programmatic dependent launch)
-    int32_t after_rope;           // q, k_new and v_new come from the rotary kernel that this launch overlaps
     const uint16_t *k_params;     // viewed as fp16
     const uint16_t *v_params;
     int64_t k_params_stride_b;    // in fp16 elements

@@ -27,8 +27,8 @@ __device__ __forceinline__ void rope_store(void *p, int64_t i, float v, bool bf1
 // grid (q heads + 2 x KV heads, b), 64 threads: thread t is pair t of one head's row: a q head, then a k head
 // (both rotated), then a v head (copied beside them)
 __global__ void __launch_bounds__(64) bd_rope_kernel(const RopeParams p) {
-    // Everything in front is done from here on; the decode kernel behind this one may start then, and waits for this grid
-    // before it reads a rotated row.
+    // Everything in front is done from here on; the decode kernel behind this one may be placed then, and waits for this
+    // grid before it reads anything.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int ib = blockIdx.y;

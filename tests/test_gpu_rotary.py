@@ -124,3 +124,34 @@ def test_positions_follow_the_device_side_lengths_in_a_captured_decoder_loop():
             want = O.apply_rotary(H.to_np(news[i])[ib:ib + 1, 0], H.to_np(cos), H.to_np(sin), [pos], False)
             got = cache.k_tail[ib, r].cpu().numpy()
             assert np.array_equal(got.view(np.uint16), want[0].view(np.uint16)), (ib, r, pos)
+
+
+@pytest.mark.parametrize("b,bits,h_k", [(1, 4, 8), (3, 2, 2), (40, 4, 2)])
+def test_steps_in_a_row_equal_steps_one_by_one(b, bits, h_k):
+    """Rotary, decode, merge and roll-over kernels overlap across steps in a stream: whatever an earlier step wrote (lengths,
+    a packed block, tail rows) has to be there, so the steps give the bits of steps that are waited for one by one."""
+    import bitladder_b200 as B
+    nb, steps = B.pack_block_tokens(bits), 24
+    s = 4 * nb
+    x = {k: v.cuda() for k, v in H.gen_qkv(b, s, 4 * h_k, h_k, seed=61, res=nb).items() if isinstance(v, torch.Tensor)}
+    cos, sin = (t.cuda() for t in _tables(s + nb, 64, x["q"].dtype, 4))
+    g = torch.Generator().manual_seed(8)
+    rows = [torch.randn(steps, b, 1, n, 128, generator=g).half().cuda() for n in (4 * h_k, h_k, h_k)]
+    lens = torch.arange(b, dtype=torch.int32) % 3 * nb, nb - 2 - torch.arange(b, dtype=torch.int32) % 9
+
+    def outputs(one_by_one):
+        bufs = B.alloc_packed_cache(b, s, h_k, 128, bits, 128)
+        B.kvcache_pack_int(x["k"], bufs[0], bufs[1], x["v"], bufs[2], bufs[3], None, None, s, "k-channel", 128, bits)
+        now = [torch.empty_like(r[0]) for r in rows]
+        tails, (cs, rl), outs = [x["k_res"].clone(), x["v_res"].clone()], [t.cuda() for t in lens], []
+        step = B.DecodeStep(now[0], *bufs, None, H.default_scale(), "k-channel", 128, bits, k_res=tails[0], v_res=tails[1],
+                            res_lens=rl, cache_seqlens=cs, k_new=now[1], v_new=now[2], advance=True, rotary_cos=cos, rotary_sin=sin)
+        torch.cuda.synchronize()
+        for i in range(steps):
+            for t, r in zip(now, rows):
+                torch.mul(r[i], 1, out=t)
+            outs.append(step.step(check=one_by_one).clone())
+        return outs + [t.view(torch.uint8) for t in bufs] + tails + [cs, rl]
+
+    for a, c in zip(outputs(True), outputs(False)):
+        assert torch.equal(a, c)

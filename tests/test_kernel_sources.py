@@ -41,3 +41,19 @@ def test_nothing_is_read_as_constant_memory(path):
     wait."""
     code = "".join(_code(path))
     assert "__ldg(" not in code and "global.nc" not in code
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_a_wait_of_its_own_comes_before_what_earlier_kernels_wrote(path):
+    """Only a kernel's own griddepcontrol.wait makes earlier kernels' writes visible to it (that the kernel in front has
+    waited, and let this one start afterwards, does not), so the lengths and the table of a ragged batch are read behind
+    one.  Whether a kernel waits there may hang on nothing but that there is such a table."""
+    code = "".join(_code(path))
+    for cond in re.findall(r"if (?:constexpr )?\(((?:[^()]|\([^()]*\))*)\)\s*\{?\s*asm volatile\(\"griddepcontrol.wait", code):
+        assert "p." not in re.sub(r"p\.part\.table|\browid\b.*|\bn(rows|parts)\b.*", "", cond), cond
+    for body in code.split("__global__")[1:]:
+        if "griddepcontrol.wait" not in body:
+            continue
+        body = re.sub(r"\{[^{}]*griddepcontrol\.wait[^{}]*return;\s*\}", "", body)          # a warp that leaves
+        read = re.search(r"ragged_entry\(|part_range\(|(cache_seqlens|res_lens)\[", body)
+        assert not read or body.index("griddepcontrol.wait") < read.start()
