@@ -866,6 +866,18 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                         // One k-slice after the other, the fields of a slice one by one: four masks and an MMA each,
                         // no two MMAs in a row with the same accumulator.  The masks and the MMAs share the warp
                         // scheduler's dispatch (2 cycles a mask, 4 an MMA), which is what bounds the 2-bit kernels.
+                        // At 4 bits with two query tiles the fields of a whole slice (group 128: of both) come first:
+                        // one by one, the registers spill.  16 query heads per KV head, groups 128 and 64, one by one /
+                        // a slice / both slices: 8 x 32768 tokens 88.0 / 86.3 / 86.1 and 95.4 / 93.0 / 94.2 us,
+                        // 16 x 131072 tokens 608 / 611 / 604 and 661 / 645 / 657 us.
+                        constexpr int AHEAD = BITS == 4 && NQT == 2 ? (GROUP == 128 ? 2 : 1) : 0;
+                        uint32_t F[2][P][4];
+                        auto mma_kfield = [&](int half, int j) {
+#pragma unroll
+                            for (int nq = 0; nq < NQT; ++nq)
+                                mma_f16(S[uu][j][nq], F[half][j][0], F[half][j][1], F[half][j][2], F[half][j][3],
+                                        qs[j / FPG][nq][2 * half], qs[j / FPG][nq][2 * half + 1]);
+                        };
 #pragma unroll
                         for (int half = 0; half < 2; ++half) {
                             const uint32_t w0 = wl[2 * half], w1 = wh[2 * half], w2 = wl[2 * half + 1], w3 = wh[2 * half + 1];
@@ -873,11 +885,9 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                             auto do_kfield = [&](auto jc) {
                                 constexpr int J = decltype(jc)::value;
                                 constexpr bool PR = kFieldPairs<BITS, GROUP>;
-                                const uint32_t f0 = field<BITS, J, PR>(w0, s0), f1 = field<BITS, J, PR>(w1, s1);
-                                const uint32_t f2 = field<BITS, J, PR>(w2, s2), f3 = field<BITS, J, PR>(w3, s3);
-#pragma unroll
-                                for (int nq = 0; nq < NQT; ++nq)
-                                    mma_f16(S[uu][J][nq], f0, f1, f2, f3, qs[J / FPG][nq][2 * half], qs[J / FPG][nq][2 * half + 1]);
+                                F[half][J][0] = field<BITS, J, PR>(w0, s0); F[half][J][1] = field<BITS, J, PR>(w1, s1);
+                                F[half][J][2] = field<BITS, J, PR>(w2, s2); F[half][J][3] = field<BITS, J, PR>(w3, s3);
+                                if constexpr (AHEAD == 0) mma_kfield(half, J);
                             };
                             do_kfield(std::integral_constant<int, 0>{});
                             do_kfield(std::integral_constant<int, 1>{});
@@ -889,6 +899,16 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                                 do_kfield(std::integral_constant<int, 6>{});
                                 do_kfield(std::integral_constant<int, 7>{});
                             }
+                            if constexpr (AHEAD == 1) {
+#pragma unroll
+                                for (int j = 0; j < P; ++j) mma_kfield(half, j);
+                            }
+                        }
+                        if constexpr (AHEAD == 2) {
+#pragma unroll
+                            for (int half = 0; half < 2; ++half)
+#pragma unroll
+                                for (int j = 0; j < P; ++j) mma_kfield(half, j);
                         }
                     }
                 }

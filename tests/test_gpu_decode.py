@@ -236,6 +236,20 @@ def test_ragged_batches_at_the_table_limit(b, s, bits, splits):
     _check(x, ref, out, lse, bits, 128, "fp16", cs, rl, res=True)
 
 
+@pytest.mark.parametrize("group,dtype", [(128, "fp16"), (64, "bf16"), (32, "fp16")])
+@pytest.mark.parametrize("h", [18, 32])
+@pytest.mark.parametrize("ragged", [False, True])
+def test_two_query_tiles_at_four_bits(group, dtype, h, ragged):
+    """9 and 16 query heads per KV head: the kernels that form all fields of a slice ahead of its MMAs."""
+    import bitladder_b200 as B
+    x = H.gen_qkv(2, 1024, h, 2, seed=17, dtype=dtype)
+    ref = H.oracle_pack(x["k"], x["v"], 4, group, dtype)
+    bufs = G.pack_gpu(B, x["k"], x["v"], 4, group)
+    cs = torch.tensor([1000, 129], dtype=torch.int32) if ragged else None
+    out, lse = _run(B, x, bufs, 4, group, dtype, **(dict(cache_seqlens=cs) if ragged else {}))
+    _check(x, ref, out, lse, 4, group, dtype, cs)
+
+
 def test_plan_reports_what_the_step_launches():
     """DecodeStep.plan(): ranges per KV head, CTAs per SM and launches as the library plans them on this GPU."""
     import bitladder_b200 as B
