@@ -441,20 +441,25 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     part.R = plan.rows;
 
     cudaError_t err;
-    // Whether the first kernel of the step is staged early behind whatever runs in front of it (it waits for that before
-    // it touches global memory).  In a stream a kernel otherwise starts on the next 2 us tick after the one in front is
-    // done (b1, 4096 tokens: 12.3 us a step instead of 10.0; 32 x up to 16384 tokens, 32 heads: 219 instead of 216);
-    // between the kernels of a graph there is no such tick and only small steps gain (b1, 2048 tokens, 32 heads 10.8 ->
-    // 9.7 us, b8, 32768 tokens 56.6 -> 57.5).  CTAs that are placed as SMs fall free lose the order in which the heads of a
-    // row stream the same tokens together, which costs long steps of one CTA per SM more than the tick (blocks per
-    // warp in a stream: 10: 57.9 -> 57.1 us, 19: 102.0 -> 104.2, 76: 361 -> 382).
+    // Whether the kernels of the step are staged early behind what runs in front of them (they wait for that before they
+    // touch global memory).  In a stream a kernel otherwise starts on the next 2 us tick after the one in front is done
+    // (b1, 4096 tokens: 12.3 us a step instead of 10.0); between the kernels of a graph there is no such tick and only
+    // small steps gain (b1, 2048 tokens, 32 heads 10.8 -> 9.7 us, b8, 32768 tokens 56.6 -> 57.5).  CTAs that are placed as
+    // SMs fall free lose the order in which the heads of a row stream the same tokens together, which costs long steps
+    // more than the tick.  By blocks per warp, plain -> early in us:
+    //   stream, one CTA per SM    10: 57.9 -> 57.1, 19: 102.0 -> 104.2, 76: 361 -> 382
+    //   stream, two CTAs per SM   38: 236.6 -> 235.5, 76: 426.3 -> 426.8, 152: 840 -> 836, 228: 1245 -> 1265
+    // and of the decode kernel behind the step's own rotary kernel, which is short and never fills the machine:
+    //   stream                    14: 89.5 -> 88.5, 19: 119.8 -> 119.2, 38: 222.9 -> 223.2, 76: 434.8 -> 437.1
+    //   graph                     10: 61.0 -> 60.5, 14: 86.8 -> 86.9, 19: 115.6 -> 117.2, 76: 428 -> 437
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     const bool asked = cudaStreamIsCapturing(stream, &capture) == cudaSuccess;
     if (!asked) (void)cudaGetLastError();            // (the legacy stream beside a capture: the launches say what is wrong)
     const bool in_graph = !asked || capture != cudaStreamCaptureStatusNone;
     const int64_t warps = int64_t(plan.rows) * bd::decode_warps(a->bits, a->group, a->h / a->h_k, plan.two_ctas);
-    const bool early = (!in_graph && plan.two_ctas) ||
-                       int64_t(a->b) * bd::seq_blocks(a->s, a->s, nb) <= (in_graph ? 2 : 12) * warps;
+    const int64_t blocks = int64_t(a->b) * bd::seq_blocks(a->s, a->s, nb);
+    const bool early = blocks <= (in_graph ? 2 : plan.two_ctas ? 160 : 12) * warps;
+    const bool early_decode = early || (a->rotary_dim > 0 && blocks <= (in_graph ? 12 : 24) * warps);
     const bool inline_table = plan.ragged && a->b <= bd::kInlineSeqs && !x;      // (the exchange kernel reads the table)
     if (plan.ragged && !inline_table) {
         bd::PrefixParams pp;
@@ -535,7 +540,7 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
         p.q = rp.q_out; p.q_stride_b = int64_t(a->h) * 128; p.q_stride_h = 128;
         p.k_new = rp.k_out; p.v_new = rp.v_out; p.new_stride_b = int64_t(a->h_k) * 128; p.new_stride_h = 128;
     }
-    p.early = (early || a->rotary_dim > 0) ? 1 : 0;
+    p.early = early_decode ? 1 : 0;
     p.defer_merge = (x || plan.rows > 4 * a->b) ? 1 : 0;
     p.leave_parts = x ? 1 : 0;
     p.two_ctas = plan.two_ctas;
