@@ -8,7 +8,9 @@
 // (a fwd_kvcache_int call of 1 x 4096 tokens, 32/32 heads: 35.0 us a pass before, 16.4 with this file, 14.3 of them kernels;
 // kvcache_pack_int of one block of 8 sequences 26.5 -> 6.8 us).
 //
-// Nothing is kept between calls; the workspaces live in the dictionary that the Python code owns.
+// Nothing is kept between calls; the workspaces live in the dictionary that the Python code owns.  The interpreter lock is
+// let go around allocations and launches (a launch waits where the stream's queue is full, and what it waits for may be a
+// host function that needs the lock), as ctypes does: what is used there is owned by this call, not borrowed.
 #include <Python.h>
 
 #include <ATen/core/Tensor.h>
@@ -31,6 +33,14 @@ struct NotPlain {};      // the Python code takes the call
 inline void need(bool ok) {
     if (!ok) throw NotPlain();
 }
+
+// Other Python threads run while one of these lives; nothing of the interpreter may be touched.
+struct Unlocked {
+    PyThreadState *state = PyEval_SaveThread();
+    Unlocked() = default;
+    Unlocked(const Unlocked &) = delete;
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
 
 // A plain CUDA tensor on `dev` (an index below 0: any, which it then becomes).
 const at::Tensor &tensor(PyObject *o, c10::DeviceIndex &dev) {
@@ -104,8 +114,9 @@ const int32_t *lengths(const at::Tensor &t, int64_t b) {
     return static_cast<const int32_t *>(t.data_ptr());
 }
 
-// The dictionary's workspace for this device and stream, if it is there, large enough and cleared for this layout.
-void workspace(PyObject *dict, c10::DeviceIndex dev, void *stream, bd_decode_args &a) {
+// The dictionary's workspace for this device and stream, if it is there, large enough and cleared for this layout.  The
+// caller owns it: another thread may put a larger one in its place while this call runs.
+at::Tensor workspace(PyObject *dict, c10::DeviceIndex dev, void *stream, bd_decode_args &a) {
     const size_t bytes = g_workspace_bytes(&a);
     need(bytes > 0 && PyDict_CheckExact(dict));
     PyObject *key = Py_BuildValue("(iK)", int(dev), (unsigned long long)(uintptr_t)stream);
@@ -122,6 +133,7 @@ void workspace(PyObject *dict, c10::DeviceIndex dev, void *stream, bd_decode_arg
     need(size_t(ws.numel()) >= bytes);
     a.workspace = ws.data_ptr();
     a.workspace_bytes = size_t(ws.numel());
+    return ws;
 }
 
 PyObject *decode_call(PyObject *const *o) {
@@ -208,15 +220,20 @@ PyObject *decode_call(PyObject *const *o) {
 
     c10::cuda::CUDAGuard guard(dev);
     void *stream = c10::cuda::getCurrentCUDAStream(dev).stream();
-    workspace(o[0], dev, stream, a);
-    at::Tensor out = at::empty(q.sizes(), q.options().dtype(out_type)), lse;
-    a.out = out.data_ptr();
-    a.out_stride_b = out.stride(0); a.out_stride_h = out.stride(2);
-    if (return_lse) {
-        lse = at::empty({b, h}, q.options().dtype(at::kFloat));
-        a.lse = static_cast<float *>(lse.data_ptr());
+    const at::Tensor ws = workspace(o[0], dev, stream, a);
+    const at::TensorOptions options = q.options();
+    at::Tensor out, lse;
+    {
+        Unlocked unlocked;
+        out = at::empty({b, 1, h, 128}, options.dtype(out_type));
+        a.out = out.data_ptr();
+        a.out_stride_b = out.stride(0); a.out_stride_h = out.stride(2);
+        if (return_lse) {
+            lse = at::empty({b, h}, options.dtype(at::kFloat));
+            a.lse = static_cast<float *>(lse.data_ptr());
+        }
+        need(g_decode(&a, stream) == BD_OK);
     }
-    need(g_decode(&a, stream) == BD_OK);
     if (!return_lse) return THPVariable_Wrap(std::move(out));
     PyObject *po = THPVariable_Wrap(std::move(out)), *pl = THPVariable_Wrap(std::move(lse));
     PyObject *pair = PyTuple_New(2);
@@ -251,7 +268,10 @@ PyObject *pack_call(PyObject *const *o) {
     a.bits = bits; a.group = group; a.dtype = dtype_code(type);
     a.flags = approx ? BD_PACK_APPROX_DIV : 0;
     c10::cuda::CUDAGuard guard(dev);
-    need(g_pack(&a, c10::cuda::getCurrentCUDAStream(dev).stream()) == BD_OK);
+    {
+        Unlocked unlocked;
+        need(g_pack(&a, c10::cuda::getCurrentCUDAStream(dev).stream()) == BD_OK);
+    }
     Py_RETURN_TRUE;
 }
 
@@ -288,6 +308,7 @@ PyObject *step(PyObject *, PyObject *const *args, Py_ssize_t n) {
     if (PyErr_Occurred()) return nullptr;
     int rc = BD_ERR_CUDA;
     try {
+        Unlocked unlocked;
         c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev));
         rc = g_decode(static_cast<const bd_decode_args *>(a), c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(dev)).stream());
     } catch (...) {

@@ -1,5 +1,10 @@
 """The extension that takes plainly valid calls to the library: the same results as the Python path in every form of a
 call, and whatever it does not take comes back to the Python path."""
+import ctypes as C
+import subprocess
+import threading
+import time
+
 import pytest
 import torch
 
@@ -102,3 +107,41 @@ def test_refused_calls_are_still_refused():
                  lambda: B.kvcache_pack_int(k, bufs[0], bufs[1], k, bufs[2], bufs[3], None, None, 256, dst_token_offset=128)):
         with pytest.raises(RuntimeError):
             call()
+
+
+@pytest.mark.gpu
+def test_other_threads_run_during_a_launch(tmp_path):
+    """A launch that waits (here: an entry point that sleeps) holds up its own thread only."""
+    from bitladder_b200 import _lib, _torch_calls as T
+    import bitladder_b200 as B
+    source = tmp_path / "slow.c"
+    source.write_text("#include <stddef.h>\n#include <unistd.h>\n"
+                      "int slow(const void *a, void *s) { usleep(300000); return 0; }\nsize_t bytes(const void *a) { return 64; }\n")
+    subprocess.run(["cc", "-shared", "-fPIC", "-o", str(tmp_path / "slow.so"), str(source)], check=True)
+    slow, real = C.CDLL(str(tmp_path / "slow.so")), _lib.load()
+    bind = lambda *f: T.bind(*(C.cast(x, C.c_void_p).value for x in f))
+    x = {k: v.cuda() for k, v in H.gen_qkv(2, 256, 8, 2, seed=5).items() if isinstance(v, torch.Tensor)}
+    bufs = B.alloc_packed_cache(2, 256, 2, 128, 4, 128)
+    stream = torch.cuda.current_stream().cuda_stream
+    spaces = {(0, stream): [torch.zeros(64, dtype=torch.uint8, device="cuda"), (2, 2, False)]}
+    ticks, stop = [0], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            time.sleep(0.002)
+            ticks[0] += 1
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        bind(slow.slow, slow.slow, slow.bytes)
+        for call in (lambda: T.step(0, 0), lambda: T.pack(x["k"], bufs[0], bufs[1], x["v"], bufs[2], bufs[3], "k-channel", 128, 4, 0, False),
+                     lambda: T.decode(spaces, x["q"], *bufs, None, SCALE, "k-channel", 128, 4, None, None, None, None, None, True,
+                                      None, 0, None, None, False, None, None, True)):
+            before = ticks[0]
+            assert call() is not None
+            assert ticks[0] - before >= 20
+    finally:
+        bind(real.bd_decode, real.bd_pack, real.bd_decode_workspace_bytes)
+        stop.set()
+        thread.join()
