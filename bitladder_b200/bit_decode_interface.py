@@ -63,6 +63,10 @@ def _calls():
         lib = _lib.load()
         try:
             from . import _torch_calls as calls
+            from .build import calls_key
+            built_for = getattr(calls, "BUILT_FOR", "another version")
+            if built_for != calls_key():
+                raise ImportError(f"it was built for {built_for}, this is {calls_key()}")
             calls.bind(*(C.cast(f, C.c_void_p).value for f in (lib.bd_decode, lib.bd_pack, lib.bd_decode_workspace_bytes)))
         except ImportError as exc:
             warnings.warn(f"bitladder_b200._torch_calls cannot be loaded ({exc}): calls cost 20 to 30 us more; run "

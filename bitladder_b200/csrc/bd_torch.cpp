@@ -327,4 +327,9 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_torch_calls", nullptr, -1, kMeth
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__torch_calls(void) { return PyModule_Create(&kModule); }
+// BUILT_FOR: the torch and the interpreter whose headers were compiled in; bit_decode_interface.py takes no other.
+PyMODINIT_FUNC PyInit__torch_calls(void) {
+    PyObject *m = PyModule_Create(&kModule);
+    if (m && PyModule_AddStringConstant(m, "BUILT_FOR", BD_BUILT_FOR) < 0) Py_CLEAR(m);
+    return m;
+}
