@@ -50,8 +50,8 @@ class PackedKVCache:
         # lengths: host mirror (exact) and device copies the decode kernel reads
         self._packed: List[int] = [0] * batch
         self._tail: List[int] = [0] * batch
-        self._lengths = torch.zeros(2, batch, dtype=torch.int32, device=self.device)
-        self.cache_seqlens, self.res_lens = self._lengths.unbind()
+        self.cache_seqlens = torch.zeros(batch, dtype=torch.int32, device=self.device)
+        self.res_lens = torch.zeros(batch, dtype=torch.int32, device=self.device)
 
     # ------------------------------------------------------------------ lengths
     def seqlens(self) -> List[int]:
@@ -59,7 +59,8 @@ class PackedKVCache:
         return [p + t for p, t in zip(self._packed, self._tail)]
 
     def _push_lengths(self) -> None:
-        self._lengths.copy_(torch.tensor([self._packed, self._tail], dtype=torch.int32), non_blocking=True)
+        self.cache_seqlens.copy_(torch.tensor(self._packed, dtype=torch.int32), non_blocking=True)
+        self.res_lens.copy_(torch.tensor(self._tail, dtype=torch.int32), non_blocking=True)
 
     def _fill(self, k: torch.Tensor, v: torch.Tensor, packed: List[int], tail: List[int]) -> bool:
         """The prompts into blocks and tails in one launch, by lengths on the device; False for rows the kernel does

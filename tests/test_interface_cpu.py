@@ -1,5 +1,7 @@
 """CPU: the Python entry points keep the reference's signatures and fail loudly (no CPU path)."""
+import copy
 import inspect
+import io
 
 import pytest
 import torch
@@ -96,3 +98,23 @@ def test_a_refused_prefill_leaves_the_lengths(earlier):
         with pytest.raises(RuntimeError, match="CUDA"):
             c.prefill(rows, rows, lens)
         assert (c.seqlens(), c.cache_seqlens.tolist(), c.res_lens.tolist()) == before
+
+
+@pytest.mark.parametrize("form", ["new", "copied", "saved", "replaced"])
+def test_lengths_reach_the_tensors_that_the_cache_names(form):
+    """``cache_seqlens`` and ``res_lens`` are what decode calls read: a cache that was saved, copied or given length tensors
+    of the caller's own writes those."""
+    c = B.PackedKVCache(2, 512, 2, device="cpu")
+    if form == "copied":
+        c = copy.deepcopy(c)
+    if form == "saved":                              # as its attributes alone, every tensor by itself
+        state, c = c.__dict__, B.PackedKVCache.__new__(B.PackedKVCache)
+        c.__dict__.update({k: v.clone() if isinstance(v, torch.Tensor) else v for k, v in state.items()
+                           if k in ("cache_seqlens", "res_lens") or not torch.is_tensor(v) or v.dim() == 4})
+    if form == "replaced":
+        c.cache_seqlens, c.res_lens = torch.zeros(2, dtype=torch.int32), torch.zeros(2, dtype=torch.int32)
+    rows = torch.ones(2, 300, 2, 128, dtype=torch.float16)
+    c.prefill(rows, rows, [100, 7])
+    assert c.cache_seqlens.tolist() == [0, 0] and c.res_lens.tolist() == [100, 7]
+    c.append(rows[:, :1], rows[:, :1])
+    assert c.res_lens.tolist() == [101, 8] == [n for n in c.seqlens()]
