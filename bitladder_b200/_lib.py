@@ -48,6 +48,7 @@ class PrefillArgs(C.Structure):
         ("k_tail", C.c_void_p), ("v_tail", C.c_void_p),
         ("tail_stride_b", C.c_int64), ("tail_stride_s", C.c_int64), ("tail_stride_h", C.c_int64),
         ("cache_seqlens", C.c_void_p), ("res_lens", C.c_void_p),
+        ("s_cap", C.c_int32),
     ]
 
 

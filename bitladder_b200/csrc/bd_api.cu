@@ -338,6 +338,7 @@ static int pack_rows(const bd_pack_args *a, const bd_prefill_args *f, bd_stream_
     const int nb = pack_block_tokens(a->bits);
     if ((!f && a->s % nb) || a->dst_token_offset % nb) return BD_ERR_INVALID;
     if (f && (!f->k_tail || !f->v_tail || !f->cache_seqlens || !f->res_lens || a->dst_token_offset != 0)) return BD_ERR_INVALID;
+    if (f && (f->s_cap <= 0 || f->s_cap % nb)) return BD_ERR_INVALID;
     if ((int64_t(a->s) + nb - 1) / nb > 65535 || a->b > 65535) return BD_ERR_INVALID;      // grid.y, grid.z
     // 16-byte vector loads of the inputs and 16-byte stores of the V codes
     if ((reinterpret_cast<uintptr_t>(a->k) | reinterpret_cast<uintptr_t>(a->v) |
@@ -367,7 +368,7 @@ static int pack_rows(const bd_pack_args *a, const bd_prefill_args *f, bd_stream_
     p.b = a->b; p.s = a->s; p.h_k = a->h_k; p.dst_token_offset = a->dst_token_offset;
     p.approx_div = (a->flags & BD_PACK_APPROX_DIV) ? 1 : 0;
     if (f) {
-        p.fill_cache_seqlens = f->cache_seqlens; p.fill_res_lens = f->res_lens;
+        p.fill_cache_seqlens = f->cache_seqlens; p.fill_res_lens = f->res_lens; p.fill_s_cap = f->s_cap;
         p.k_tail = f->k_tail; p.v_tail = f->v_tail;
         p.tail_stride_b = f->tail_stride_b; p.tail_stride_s = f->tail_stride_s; p.tail_stride_h = f->tail_stride_h;
     }

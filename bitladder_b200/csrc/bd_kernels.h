@@ -37,9 +37,10 @@ struct PackParams {
     int32_t *roll_arrivals;       // [b * h_k], the first of every sequence counts its CTAs; zero between steps
     int32_t *roll_status;
     int32_t roll_s_cap, roll_res_cap;
-    // Prompts of unequal lengths (null: plain pack): a sequence's whole blocks are packed, the rows behind them copied to
-    // its tail buffers.
+    // Prompts of unequal lengths (null: plain pack): a sequence's whole blocks are packed (up to the capacity fill_s_cap of
+    // the packed buffers), the rows behind them copied to its tail buffers.
     const int32_t *fill_cache_seqlens, *fill_res_lens;
+    int32_t fill_s_cap;
     void *k_tail, *v_tail;
     int64_t tail_stride_b, tail_stride_s, tail_stride_h;
 };

@@ -195,7 +195,7 @@ bd_pack_kernel(const PackParams p) {
         if (dst_off < 0 || dst_off % NB != 0 || dst_off + NB > p.roll_s_cap) return;   // no room: reported above
     }
     if (p.fill_cache_seqlens != nullptr) {
-        const int full = min(max(p.fill_cache_seqlens[ib], 0), p.s) / NB;
+        const int full = min(max(p.fill_cache_seqlens[ib], 0), min(p.s, p.fill_s_cap)) / NB;
         if (blk >= full) {
             // behind the whole blocks: one block's worth of rows to the tail, 16 bytes a thread, the K CTAs and the V CTAs
             // of a head a share of the rows each

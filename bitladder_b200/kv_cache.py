@@ -71,7 +71,7 @@ class PackedKVCache:
         a = _lib.PrefillArgs(
             _pack_args(k, self.k_pack, self.k_params, v, self.v_pack, self.v_params, self.group_size, self.num_bits),
             t.data_ptr(), self.v_tail.data_ptr(), t.stride(0), t.stride(1), t.stride(2),
-            lengths[0].data_ptr(), lengths[1].data_ptr())
+            lengths[0].data_ptr(), lengths[1].data_ptr(), self.capacity)
         with torch.cuda.device(k.device):
             return _lib.load().bd_prefill(C.byref(a), _stream(k.device)) == _lib.BD_OK
 

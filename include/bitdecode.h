@@ -40,7 +40,7 @@
 extern "C" {
 #endif
 
-#define BD_VERSION 201
+#define BD_VERSION 202
 
 /* status codes */
 #define BD_OK                0
@@ -111,14 +111,16 @@ int bd_pack(const bd_pack_args *args, bd_stream_t stream);
  * The prompts of a batch into a growing cache, in one launch: of sequence ib the first cache_seqlens[ib] tokens of
  * pack.k / pack.v (a multiple of NB, at most pack.s) are quantize-packed as bd_pack does it, and the res_lens[ib]
  * rows behind them (fewer than NB) copied to rows 0.. of its tail buffers.  pack.s: token rows of k and v, any
- * number; pack.dst_token_offset must be 0.  The lengths are read on the device and bounded by pack.s there.  No
- * counterpart in the reference, whose residual scheme (imgs/scheme.png) is not wired up in its snapshot.
+ * number; pack.dst_token_offset must be 0.  The lengths are read on the device and bounded there by pack.s and by the
+ * packed buffers' capacity s_cap (since version 202; blocks beyond it are left out).  No counterpart in the reference,
+ * whose residual scheme (imgs/scheme.png) is not wired up in its snapshot.
  */
 typedef struct bd_prefill_args {
     bd_pack_args pack;
     void *k_tail, *v_tail;    /* (b, at least NB rows, h_k, d), the type of k and v */
     int64_t tail_stride_b, tail_stride_s, tail_stride_h;
     const int32_t *cache_seqlens, *res_lens;    /* (b), device */
+    int32_t s_cap;            /* token capacity of the packed buffers, a positive multiple of NB */
 } bd_prefill_args;
 
 int bd_prefill(const bd_prefill_args *args, bd_stream_t stream);

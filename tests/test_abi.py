@@ -60,6 +60,11 @@ def test_argument_validation_needs_no_device():
     assert lib.bd_pack(C.byref(a), None) == -2                     # head dim 64
     a.d, a.s = 128, 100
     assert lib.bd_pack(C.byref(a), None) == -1                     # not whole pack blocks
+    a.s = 128
+    f = _lib.PrefillArgs(a, ptr, ptr, 128, 128, 128, ptr, ptr, 128)
+    for f.s_cap in (0, -128, 100):
+        assert lib.bd_prefill(C.byref(f), None) == -1              # capacity: whole pack blocks
+    assert lib.bd_prefill(None, None) == -1
     d = _lib.DecodeArgs(q=ptr, out=ptr, k_pack=ptr, k_params=ptr, v_pack=ptr, v_params=ptr,
                         b=1, h=34, h_k=8, d=128, s=128, s_cap=128, bits=4, group=128)
     assert lib.bd_decode(C.byref(d), None) == -1                   # heads do not divide

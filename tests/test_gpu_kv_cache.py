@@ -282,3 +282,28 @@ def test_every_tail_of_a_large_batch_rolls_over_at_once(b, h_k, bits):
         assert rl.tolist() == torch.where(rolls, 0, 4).tolist()
         for t, w in zip(bufs, want):
             assert torch.equal(t.view(torch.uint8), w.view(torch.uint8))
+
+
+@pytest.mark.parametrize("bits", [4, 2])
+def test_prefill_lengths_beyond_the_capacity_are_bounded(bits):
+    """Lengths on the device that a caller got wrong: blocks beyond the capacity it stated, and rows beyond those it gave,
+    are left out.  (The buffers here are larger than what is stated.)"""
+    import ctypes as C
+    import bitladder_b200 as B
+    from bitladder_b200 import _lib, bit_decode_interface as I
+    nb = B.pack_block_tokens(bits)
+    x = {k: v.cuda() for k, v in H.gen_qkv(3, 4 * nb, 2, 2, seed=43).items() if isinstance(v, torch.Tensor)}
+    bufs, want = B.alloc_packed_cache(3, 4 * nb, 2, 128, bits, 128), B.alloc_packed_cache(3, 4 * nb, 2, 128, bits, 128)
+    B.kvcache_pack_int(x["k"], want[0], want[1], x["v"], want[2], want[3], None, None, 4 * nb, "k-channel", 128, bits)
+    tails = [torch.zeros(3, nb, 2, 128, dtype=torch.float16, device="cuda") for _ in "kv"]
+    lens = torch.tensor([[4 * nb, 1 << 30, -5], [1 << 30, 7, 7]], dtype=torch.int32, device="cuda")
+    a = _lib.PrefillArgs(I._pack_args(x["k"], bufs[0], bufs[1], x["v"], bufs[2], bufs[3], 128, bits), tails[0].data_ptr(),
+                         tails[1].data_ptr(), *tails[0].stride()[:3], lens[0].data_ptr(), lens[1].data_ptr(), 2 * nb)
+    assert _lib.load().bd_prefill(C.byref(a), torch.cuda.current_stream().cuda_stream) == 0
+    rows = [t.shape[3] == 4 * nb for t in bufs]      # v_params: tokens last; the others: dim 1
+    for t, w, last in zip(bufs, want, rows):
+        dim = 3 if last else 1
+        half = t.shape[dim] // 2
+        assert torch.equal(t[:2].narrow(dim, 0, half).view(torch.int16), w[:2].narrow(dim, 0, half).view(torch.int16))
+        assert not t[:2].narrow(dim, half, half).contiguous().view(torch.int16).any()
+        assert not t[2].contiguous().view(torch.int16).any()
