@@ -25,7 +25,8 @@ from typing import List, Optional, Sequence
 import torch
 
 from . import _lib
-from .bit_decode_interface import (_pack_args, _stream, alloc_packed_cache, fwd_kvcache_int, kvcache_pack_int, pack_block_tokens)
+from .bit_decode_interface import (_check_packed, _pack_args, _stream, alloc_packed_cache, fwd_kvcache_int, kvcache_pack_int,
+                                   pack_block_tokens)
 
 __all__ = ["PackedKVCache"]
 
@@ -62,12 +63,28 @@ class PackedKVCache:
         self.cache_seqlens.copy_(torch.tensor(self._packed, dtype=torch.int32), non_blocking=True)
         self.res_lens.copy_(torch.tensor(self._tail, dtype=torch.int32), non_blocking=True)
 
+    def _laid_out(self, k: torch.Tensor) -> bool:
+        """Whether blocks and tails are buffers that the one-launch prefill may write: on k's device, of the shapes and
+        strides that a pack call asks for (they are the caller's to replace), tails of k's type with equal strides."""
+        blocks, tails = (self.k_pack, self.k_params, self.v_pack, self.v_params), (self.k_tail, self.v_tail)
+        if any(t.device != k.device for t in blocks + tails):
+            return False
+        if any(t.dtype != k.dtype or t.shape != (self.batch, self.block, *k.shape[2:]) or t.stride(-1) != 1 or
+               t.stride() != self.k_tail.stride() for t in tails):
+            return False
+        try:
+            return _check_packed(*blocks, self.num_bits, self.group_size) == (self.batch, self.capacity, *k.shape[2:])
+        except RuntimeError:
+            return False
+
     def _fill(self, k: torch.Tensor, v: torch.Tensor, packed: List[int], tail: List[int]) -> bool:
         """The prompts into blocks and tails in one launch, by lengths on the device; False for rows the kernel does
-        not take (strides, alignment).  The lengths are this launch's own: the cache's move only when rows were taken."""
-        if not (k.is_cuda and k.device == v.device == self.k_pack.device and k.stride(-1) == v.stride(-1) == 1):
+        not take (strides, alignment) and buffers of another layout.  The lengths are this launch's own: the cache's move
+        only when rows were taken."""
+        if not (k.is_cuda and k.device == v.device and k.stride(-1) == v.stride(-1) == 1 and self._laid_out(k)):
             return False
-        t, lengths = self.k_tail, torch.tensor([packed, tail], dtype=torch.int32).to(k.device, non_blocking=True)
+        t = self.k_tail
+        lengths = torch.tensor([packed, tail], dtype=torch.int32).to(k.device, non_blocking=True)
         a = _lib.PrefillArgs(
             _pack_args(k, self.k_pack, self.k_params, v, self.v_pack, self.v_params, self.group_size, self.num_bits),
             t.data_ptr(), self.v_tail.data_ptr(), t.stride(0), t.stride(1), t.stride(2),

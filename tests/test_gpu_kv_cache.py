@@ -307,3 +307,30 @@ def test_prefill_lengths_beyond_the_capacity_are_bounded(bits):
         assert torch.equal(t[:2].narrow(dim, 0, half).view(torch.int16), w[:2].narrow(dim, 0, half).view(torch.int16))
         assert not t[:2].narrow(dim, half, half).contiguous().view(torch.int16).any()
         assert not t[2].contiguous().view(torch.int16).any()
+
+
+@pytest.mark.parametrize("what", ["shape", "strides", "tails", "tail_type"])
+def test_prefill_checks_buffers_that_a_caller_put_in_place(what):
+    """A cache whose buffers were replaced: what a pack call refuses is refused, and tails laid out in any way are filled."""
+    from bitladder_b200 import PackedKVCache
+    x = H.gen_qkv(2, 300, 8, 2, seed=47)
+    k, v = x["k"].cuda(), x["v"].cuda()
+    c, want = PackedKVCache(2, 512, 2), PackedKVCache(2, 512, 2)
+    want.prefill(k, v, [300, 5])
+    if what == "shape":
+        c.v_params = c.v_params[..., :256].contiguous()
+    if what == "strides":
+        c.k_pack = torch.zeros(2, 128, 4, 128, dtype=torch.uint16, device="cuda")[:, :, ::2]
+    if what == "tails":
+        c.v_tail = torch.zeros(2, 128, 2, 256, dtype=torch.float16, device="cuda")[..., ::2]
+    if what == "tail_type":
+        c.k_tail, c.v_tail = c.k_tail.float(), c.v_tail.float()
+    if what in ("shape", "strides"):
+        with pytest.raises(RuntimeError):
+            c.prefill(k, v, [300, 5])
+        assert c.seqlens() == [0, 0]
+        return
+    c.prefill(k, v, [300, 5])
+    for a, b in zip((c.k_tail, c.v_tail), (want.k_tail, want.v_tail)):
+        assert torch.equal(a[0, :44].half(), b[0, :44]) and torch.equal(a[1, :5].half(), b[1, :5])
+    assert torch.equal(c.k_pack.view(torch.int16), want.k_pack.view(torch.int16))
