@@ -25,8 +25,7 @@ from typing import List, Optional, Sequence
 import torch
 
 from . import _lib
-from .bit_decode_interface import (_check_packed, _pack_args, _stream, alloc_packed_cache, fwd_kvcache_int, kvcache_pack_int,
-                                   pack_block_tokens)
+from .bit_decode_interface import (_pack_args, _stream, alloc_packed_cache, fwd_kvcache_int, kvcache_pack_int, pack_block_tokens)
 
 __all__ = ["PackedKVCache"]
 
@@ -64,18 +63,17 @@ class PackedKVCache:
         self.res_lens.copy_(torch.tensor(self._tail, dtype=torch.int32), non_blocking=True)
 
     def _laid_out(self, k: torch.Tensor) -> bool:
-        """Whether blocks and tails are buffers that the one-launch prefill may write: on k's device, of the shapes and
-        strides that a pack call asks for (they are the caller's to replace), tails of k's type with equal strides."""
-        blocks, tails = (self.k_pack, self.k_params, self.v_pack, self.v_params), (self.k_tail, self.v_tail)
-        if any(t.device != k.device for t in blocks + tails):
-            return False
-        if any(t.dtype != k.dtype or t.shape != (self.batch, self.block, *k.shape[2:]) or t.stride(-1) != 1 or
-               t.stride() != self.k_tail.stride() for t in tails):
-            return False
-        try:
-            return _check_packed(*blocks, self.num_bits, self.group_size) == (self.batch, self.capacity, *k.shape[2:])
-        except RuntimeError:
-            return False
+        """Whether blocks and tails (a caller may have put others in their place) are laid out as this class allocates them,
+        on k's device, the tails of k's type: what the one-launch prefill writes."""
+        b, cap, bits, (h_k, d) = self.batch, self.capacity, self.num_bits, k.shape[2:]
+        tail, words, pairs = (b, self.block, h_k, d), (torch.uint16, torch.int16), (torch.float32,)
+        for t, shape, types in ((self.k_pack, (b, cap * bits // 16, h_k, d), words), (self.v_pack, (b, cap, h_k, d * bits // 16), words),
+                                (self.k_params, (b, cap // self.group_size, h_k, d), pairs),
+                                (self.v_params, (b, d // self.group_size, h_k, cap), pairs),
+                                (self.k_tail, tail, (k.dtype,)), (self.v_tail, tail, (k.dtype,))):
+            if t.shape != shape or t.dtype not in types or t.device != k.device or not t.is_contiguous():
+                return False
+        return True
 
     def _fill(self, k: torch.Tensor, v: torch.Tensor, packed: List[int], tail: List[int]) -> bool:
         """The prompts into blocks and tails in one launch, by lengths on the device; False for rows the kernel does
