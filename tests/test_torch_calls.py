@@ -145,3 +145,78 @@ def test_other_threads_run_during_a_launch(tmp_path):
         bind(real.bd_decode, real.bd_pack, real.bd_decode_workspace_bytes)
         stop.set()
         thread.join()
+
+
+def _small(B, seed=5):
+    x = {k: v.cuda() for k, v in H.gen_qkv(2, 256, 8, 2, seed=seed).items() if isinstance(v, torch.Tensor)}
+    bufs = B.alloc_packed_cache(2, 256, 2, 128, 4, 128)
+    B.kvcache_pack_int(x["k"], bufs[0], bufs[1], x["v"], bufs[2], bufs[3], None, None, 256, "k-channel", 128, 4)
+    torch.cuda.synchronize()
+    return x, bufs
+
+
+@pytest.mark.gpu
+def test_side_streams_threads_and_captures(monkeypatch):
+    """Calls on streams of their own, from threads of their own and into a graph give the bits of the Python path, each
+    stream with its own workspace."""
+    import bitladder_b200 as B
+    from bitladder_b200 import bit_decode_interface as I
+    sets = [_small(B, seed) for seed in (5, 6, 7)]
+    decode = lambda x, bufs: B.fwd_kvcache_int(x["q"], *bufs, None, SCALE, "k-channel", 128, 4, num_splits=2, return_lse=True)
+    calls = I._calls()
+    monkeypatch.setattr(I, "_CALLS", I._InterpretedCalls)
+    want = [[t.clone() for t in decode(*s)] for s in sets]
+    torch.cuda.synchronize()
+    monkeypatch.setattr(I, "_CALLS", calls)
+    got = [None] * len(sets)
+
+    def work(i):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            for _ in range(50):
+                got[i] = decode(*sets[i])
+            assert (0, stream.cuda_stream) in I._WORKSPACES
+        stream.synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(sets))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for g, w in zip(got, want):
+        assert all(torch.equal(a, b) for a, b in zip(g, w))
+    stream, graph, (x, bufs) = torch.cuda.Stream(), torch.cuda.CUDAGraph(), sets[0]
+    with torch.cuda.stream(stream):
+        decode(x, bufs)                              # the stream's workspace is there before the capture
+        stream.synchronize()
+        taken = []
+        monkeypatch.setattr(I, "_CALLS", type("Watched", (I._InterpretedCalls,), {
+            "decode": staticmethod(lambda *a: taken.append(calls.decode(*a)) or taken[-1])}))
+        with torch.cuda.graph(graph, stream=stream):
+            out, lse = decode(x, bufs)
+        assert taken[0] is not None
+        q = x["q"].clone()
+        for other, w in ((sets[1][0]["q"], None), (q, want[0])):
+            x["q"].copy_(other)
+            graph.replay()
+            stream.synchronize()
+            assert w is None or (torch.equal(out, w[0]) and torch.equal(lse, w[1]))
+
+
+@pytest.mark.gpu
+def test_misaligned_and_empty_tensors():
+    """What the library refuses comes back to the Python path and is an error there; nothing to pack is none."""
+    import bitladder_b200 as B
+    x, bufs = _small(B)
+    before = [t.clone() for t in bufs]
+    shifted = lambda t: torch.cat([t.flatten(), t.flatten()[:8]])[1:1 + t.numel()].view(t.shape)
+    pack = lambda k, v: B.kvcache_pack_int(k, bufs[0], bufs[1], v, bufs[2], bufs[3], None, None, k.shape[1], "k-channel", 128, 4)
+    decode = lambda q, **kw: B.fwd_kvcache_int(q, *bufs, None, SCALE, "k-channel", 128, 4, **kw)
+    for call in (lambda: pack(shifted(x["k"]), x["v"]), lambda: pack(x["k"], shifted(x["v"])), lambda: decode(shifted(x["q"])),
+                 lambda: decode(x["q"], k_res=shifted(x["k"][:, :16].contiguous()), v_res=x["v"][:, :16].contiguous()),
+                 lambda: decode(x["q"][:0]), lambda: pack(x["k"][:0], x["v"][:0])):
+        with pytest.raises(RuntimeError):
+            call()
+    pack(x["k"][:, :0], x["v"][:, :0])
+    assert all(torch.equal(a.view(torch.int16), b.view(torch.int16)) for a, b in zip(before, bufs))
+    assert decode(x["q"], seqlen_k=0).abs().max() == 0
