@@ -309,8 +309,8 @@ struct BlockCursor {
     }
 };
 
-// RAGGED: per-sequence lengths (and with them appends) are compiled in; a uniform batch has no table of units and
-// runs without that code in its start (b1, 4096 tokens: 10.7 us with it, 10.2 without; b8, 32768 tokens and a tail: 56.7, 56.2).
+// RAGGED: per-sequence lengths are compiled in; a uniform batch has no table of units and runs without that code in
+// its start (b1, 4096 tokens: 10.7 us with it, 10.2 without; b8, 32768 tokens and a tail: 56.7, 56.2).
 template <int BITS, int GROUP, int NQT, int TWO, bool RAGGED>
 __global__ void __launch_bounds__(Cfg<BITS, GROUP, NQT, TWO>::THREADS, Cfg<BITS, GROUP, NQT, TWO>::CTAS_PER_SM)
 bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,

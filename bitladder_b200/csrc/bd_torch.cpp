@@ -5,8 +5,8 @@
 // have to accept the same calls and fill the same argument blocks.
 //
 // Why: the checks and the argument block cost 20 to 30 us of interpreter per call, more than the kernels of a small step
-// (a fwd_kvcache_int call of 1 x 4096 tokens, 32/32 heads: 35.0 us a pass before, 16.4 with this file, 14.3 of them kernels;
-// kvcache_pack_int of one block of 8 sequences 26.5 -> 6.8 us).
+// (a fwd_kvcache_int call of 1 x 4096 tokens, 32/32 heads: 34.9 us a pass before, 13.0 with this file;
+// kvcache_pack_int of one block of 8 sequences 27.5 -> 6.4 us).
 //
 // Nothing is kept between calls; the workspaces live in the dictionary that the Python code owns.  The interpreter lock is
 // let go around allocations and launches (a launch waits where the stream's queue is full, and what it waits for may be a
