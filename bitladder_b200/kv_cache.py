@@ -75,14 +75,15 @@ class PackedKVCache:
                 return False
         return True
 
-    def _fill(self, k: torch.Tensor, v: torch.Tensor, packed: List[int], tail: List[int]) -> bool:
-        """The prompts into blocks and tails in one launch, by lengths on the device; False for rows the kernel does
-        not take (strides, alignment) and buffers of another layout.  The lengths are this launch's own: the cache's move
-        only when rows were taken."""
+    def _fill(self, k: torch.Tensor, v: torch.Tensor, packed: Optional[List[int]] = None,
+              tail: Optional[List[int]] = None) -> bool:
+        """The prompts into blocks and tails in one launch, by lengths on the device (default: those the cache holds);
+        False for rows the kernel does not take (strides, alignment) and buffers of another layout.  The lengths are this
+        launch's own: the cache's move only when rows were taken."""
         if not (k.is_cuda and k.device == v.device and k.stride(-1) == v.stride(-1) == 1 and self._laid_out(k)):
             return False
-        t = self.k_tail
-        lengths = torch.tensor([packed, tail], dtype=torch.int32).to(k.device, non_blocking=True)
+        t, held = self.k_tail, [self._packed if packed is None else packed, self._tail if tail is None else tail]
+        lengths = torch.tensor(held, dtype=torch.int32).to(k.device, non_blocking=True)
         a = _lib.PrefillArgs(
             _pack_args(k, self.k_pack, self.k_params, v, self.v_pack, self.v_params, self.group_size, self.num_bits),
             t.data_ptr(), self.v_tail.data_ptr(), t.stride(0), t.stride(1), t.stride(2),

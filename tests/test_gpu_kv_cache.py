@@ -219,7 +219,7 @@ def test_prompts_of_unequal_lengths_in_one_launch(bits, group, dtype, strided, m
         return [t.view(torch.uint8) for t in (c.k_pack, c.k_params, c.v_pack, c.v_params, c.k_tail, c.v_tail)] + [
             c.cache_seqlens, c.res_lens]
 
-    assert PackedKVCache(len(lens), s, 6, 128, bits, group, k.dtype)._fill(k, v, [n // nb * nb for n in lens], [n % nb for n in lens])
+    assert PackedKVCache(len(lens), s, 6, 128, bits, group, k.dtype)._fill(k, v)
     one = filled(k, v)
     monkeypatch.setattr(PackedKVCache, "_fill", lambda *_: False)
     for a, b in zip(one, filled(k, v)):
