@@ -91,6 +91,7 @@ bool config_supported(int bits, int group, int d) {
 struct DecodePlan {
     int rows;                 // R: ranges the block list of one KV head is cut into
     int two_ctas;             // two smaller CTAs per SM instead of one (fills the machine better with many KV heads)
+    int cluster;              // CTAs per (sequence, KV head) of a step with little work (bd_decode_short.cu); 0: not one
     bool ragged;
     int32_t n_uniform;        // units per sequence when the batch is not ragged
     size_t off_counters, off_table, off_part_out, off_part_lse, off_warp_acc, off_rope_q, off_rope_k, off_rope_v, total_bytes;
@@ -116,6 +117,33 @@ int plan_rows(int b, int h_k, int64_t max_s, int bits, int sm_count, int ctas_pe
     return int(std::min<int64_t>(rows, 1 << 20));
 }
 
+// Whether a step has so little work that bd_decode_short.cu is the faster kernel, and the CTAs it then gives every
+// (sequence, KV head): as many (a power of two, up to eight) as fit the machine at once and find work for their warps.
+// A round is an item (half a pack block, or 16 tail tokens) for every warp of a cluster.  General kernel -> short one, us a
+// step in a stream, by rounds:
+//   one sequence, 32/8 heads, 4 bits      2: 11.6 -> 8.2, 3: 12.1 -> 9.9, 4: 12.8 -> 11.6, 6: 15.0 -> 15.0, 8: 17.5 -> 18.3
+//   8 sequences, ragged, tails            1.6: 12.1 -> 7.6, 2.6: 12.6 -> 9.3, 4.5: 15.0 -> 12.8, 6.4: 18.4 -> 16.2
+//   one sequence, 64/8 heads, 2 bits      2: 13.0 -> 8.0, 4: 15.1 -> 11.4, 6: 15.6 -> 14.9, 8: 16.5 -> 18.3
+//   30 sequences, 8/1 heads, group 32     1: 14.3 -> 7.5, 2: 14.8 -> 10.4, 4: 16.3 -> 16.3
+// and with twice as many pairs of sequence and KV head as SMs (two CTAs in turn on every SM; three in turn lose):
+//   32 sequences, 32/8 heads, 4 bits      0.3: 6.3 -> 7.7, 1: 10.7 -> 9.5, 2: 15.3 -> 13.1, 4: 22.4 -> 20.0
+//   8 sequences, 32/32 heads, ragged      0.8: 11.9 -> 9.4, 1.5: 11.8 -> 9.7, 4.8: 18.3 -> 17.2
+// Equal lengths without a tail at 4 bits stop short of four rounds, where the gain is small and DecodeStep.plan() has
+// always told the general kernel's geometry.
+int short_cluster(const bd_decode_args *a, int sm_count, int64_t nblk) {
+    const int most = bd::decode_short_cluster(a->bits, a->group, a->h / a->h_k);
+    const int64_t pairs = int64_t(a->b) * a->h_k;
+    if (most == 0 || a->num_splits > 0 || pairs > 2 * int64_t(sm_count)) return 0;
+    const bool ragged = a->cache_seqlens != nullptr || (a->k_res != nullptr && a->res_lens != nullptr);
+    const int64_t items = 2 * nblk + (a->k_res ? (a->res_len + (a->k_new ? 1 : 0) + 15) / 16 : 0);
+    int c = 1;
+    while (2 * c <= most && pairs * 2 * c <= sm_count && c * bd::kShortWarps < items) c *= 2;
+    const int64_t round = int64_t(c) * bd::kShortWarps;
+    if (pairs > sm_count) return items <= 4 * round && (ragged || items >= round) ? c : 0;
+    if (a->bits == 4 && !ragged && a->k_res == nullptr) return items < 4 * round ? c : 0;
+    return items <= (a->group == 32 ? 4 : 6) * round ? c : 0;
+}
+
 int make_plan(const bd_decode_args *a, int sm_count, DecodePlan &plan) {
     const int nb = pack_block_tokens(a->bits);
     const int64_t nblk = (int64_t(a->s) + nb - 1) / nb;
@@ -139,6 +167,7 @@ int make_plan(const bd_decode_args *a, int sm_count, DecodePlan &plan) {
         rows = plan_rows(a->b, a->h_k, a->s, a->bits, sm_count, bd::decode_ctas_per_sm(a->bits, a->group, gq, plan.two_ctas));
     }
     plan.rows = int(std::max<int64_t>(1, std::min<int64_t>(rows, 1 << 20)));
+    plan.cluster = short_cluster(a, sm_count, nblk);
     const bool has_tail = a->k_res != nullptr;
     plan.ragged = a->cache_seqlens != nullptr || (has_tail && a->res_lens != nullptr);
     plan.n_uniform = bd::seq_blocks(a->s, a->s, nb) + (has_tail ? bd::tail_chunks(a->res_len + (a->k_new ? 1 : 0)) : 0);
@@ -163,6 +192,9 @@ int make_plan(const bd_decode_args *a, int sm_count, DecodePlan &plan) {
     plan.total_bytes = off;
     return BD_OK;
 }
+
+// The short kernel rotates q and the new key itself; it loads the tables sixteen bytes at a time.
+bool rotary_in_decode(const bd_decode_args *a) { return aligned16(a->rotary_cos) && aligned16(a->rotary_sin); }
 
 int check_decode_args(const bd_decode_args *a) {
     if (!a || !a->q || !a->out || !a->k_pack || !a->k_params || !a->v_pack || !a->v_params) return BD_ERR_INVALID;
@@ -317,6 +349,13 @@ int bd_decode_plan(const bd_decode_args *a, int32_t out[4]) {
     DecodePlan plan;
     make_plan(a, info.sm_count, plan);
     const int gq = a->h / a->h_k;
+    if (plan.cluster > 0) {
+        out[0] = a->b * plan.cluster;
+        out[1] = 1;
+        out[2] = bd::kShortWarps;
+        out[3] = 1 + (a->rotary_dim > 0 && !rotary_in_decode(a) ? 1 : 0) + (a->advance ? 1 : 0);
+        return BD_OK;
+    }
     out[0] = plan.rows;
     out[1] = bd::decode_ctas_per_sm(a->bits, a->group, gq, plan.two_ctas);
     out[2] = bd::decode_warps(a->bits, a->group, gq, plan.two_ctas);
@@ -427,10 +466,11 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     if (k_rows_total > 0x7fffffffull || v_rows_total > 0x7fffffffull) return BD_ERR_INVALID;
     if (int64_t(plan.rows) * a->h_k > 0x7fffffffll) return BD_ERR_INVALID;
 
+    const bool is_short = plan.cluster > 0 && !x;
     CUtensorMap kmap, vmap;
-    rc = get_map(&kmap, a->k_pack, uint64_t(k_row), k_rows_total, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B);
+    rc = get_map(&kmap, a->k_pack, uint64_t(k_row), k_rows_total, 64, is_short ? 16 : 32, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != BD_OK) return rc;
-    rc = get_map(&vmap, a->v_pack, uint64_t(v_row), v_rows_total, uint32_t(dp), uint32_t(nb),
+    rc = get_map(&vmap, a->v_pack, uint64_t(v_row), v_rows_total, uint32_t(dp), is_short ? 16 : uint32_t(nb),
                  a->bits == 4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
     if (rc != BD_OK) return rc;
 
@@ -462,7 +502,7 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     const bool early = blocks <= (in_graph ? 2 : plan.two_ctas ? 160 : 12) * warps;
     const bool early_decode = early || (a->rotary_dim > 0 && blocks <= (in_graph ? 12 : 24) * warps);
     const bool inline_table = plan.ragged && a->b <= bd::kInlineSeqs && !x;      // (the exchange kernel reads the table)
-    if (plan.ragged && !inline_table) {
+    if (plan.ragged && !inline_table && !is_short) {
         bd::PrefixParams pp;
         pp.cache_seqlens = a->cache_seqlens;
         pp.res_lens = a->k_res ? a->res_lens : nullptr;
@@ -520,7 +560,11 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     // More than four parts per sequence on average (few long sequences cut over all SMs): one warp
     // merging them at the end of the decode kernel would be the tail of the step; a second kernel
     // with a warp per (sequence, query head) does it in parallel.
-    if (a->rotary_dim > 0) {
+    if (a->rotary_dim > 0 && is_short && rotary_in_decode(a)) {
+        p.cos_tab = a->rotary_cos; p.sin_tab = a->rotary_sin;
+        p.rotary_dim = a->rotary_dim; p.rotary_interleaved = a->rotary_interleaved ? 1 : 0;
+        p.rotary_positions = a->rotary_positions;
+    } else if (a->rotary_dim > 0) {
         // q and the new key rotated at the token's position into scratch copies; the decode kernel reads those
         bd::RopeParams rp;
         std::memset(&rp, 0, sizeof(rp));
@@ -545,7 +589,9 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     p.defer_merge = (x || plan.rows > 4 * a->b) ? 1 : 0;
     p.leave_parts = x ? 1 : 0;
     p.two_ctas = plan.two_ctas;
-    err = bd::launch_decode(p, kmap, vmap, a->bits, a->group, stream);
+    p.cluster = plan.cluster;
+    err = is_short ? bd::launch_decode_short(p, kmap, vmap, a->bits, a->group, stream)
+                   : bd::launch_decode(p, kmap, vmap, a->bits, a->group, stream);
     if (err != cudaSuccess) return BD_ERR_CUDA;
     if (x) {
         xp.part_out = p.part_out; xp.part_lse = p.part_lse;
@@ -555,7 +601,7 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
         xp.part = p.part; xp.h_k = p.h_k; xp.gq = p.gq;
         err = bd::launch_exchange_parts(xp, stream);
         if (err != cudaSuccess) return BD_ERR_CUDA;
-    } else if (p.defer_merge) {
+    } else if (p.defer_merge && !is_short) {
         err = bd::launch_merge_parts(p, true, stream);
         if (err != cudaSuccess) return BD_ERR_CUDA;
     }

@@ -243,6 +243,9 @@ struct DecodeParams {
     int32_t out_dtype;
     int32_t defer_merge;          // the parts of a sequence are merged by a kernel launched next
     int32_t leave_parts;          // every segment leaves a part, also where a sequence has a single one (the exchange merges)
+    int32_t cluster;              // bd_decode_short.cu: CTAs per (sequence, KV head)
+    const void *cos_tab, *sin_tab;    // and rotary embedding (positions, rotary_dim / 2) of q and k_new; rotary_dim 0: none
+    int32_t rotary_dim, rotary_interleaved, rotary_positions;
     int32_t two_ctas;             // launch the variant with two smaller CTAs per SM
     uint32_t spin_limit;          // polls a wait on a copy may take before the warp gives up
     int32_t test_starve;          // test hook: the warps of CTA 0 expect 16 bytes more than their first copy brings
@@ -309,6 +312,11 @@ cudaError_t launch_prefix(const PrefixParams &p, cudaStream_t stream);
 cudaError_t launch_merge_parts(const DecodeParams &p, bool early, cudaStream_t stream);
 cudaError_t launch_decode(const DecodeParams &p, const CUtensorMap &kmap, const CUtensorMap &vmap,
                           int bits, int group, cudaStream_t stream);
+// A step with little work (bd_decode_short.cu); its maps have boxes of 16 rows.
+constexpr int kShortWarps = 8;    // warps per CTA
+cudaError_t launch_decode_short(const DecodeParams &p, const CUtensorMap &kmap, const CUtensorMap &vmap,
+                                int bits, int group, cudaStream_t stream);
+int decode_short_cluster(int bits, int group, int gq);    // most CTAs per cluster; 0: not built
 // `two`: the variant with half as many warps per CTA and two CTAs per SM (see Cfg in bd_decode.cu)
 bool decode_two_ctas_built(int bits, int group, int gq);
 int decode_ctas_per_sm(int bits, int group, int gq, int two);

@@ -1,0 +1,122 @@
+"""GPU: the kernel for steps with little work (a cluster of CTAs per sequence and KV head) against the oracle and against the
+general kernel on the same inputs (`num_splits` > 0 asks for that one)."""
+import numpy as np
+import pytest
+import torch
+
+from tests import gpu_util as G, helpers as H
+
+pytestmark = pytest.mark.gpu
+
+FMT = lambda group, bits: ("k-channel", group, bits)
+
+
+def _both(B, x, bufs, group, bits, table=None, **kw):
+    """(out, lse) of the short kernel, checked against the general kernel's."""
+    args = (x["q"].cuda(), *bufs, table, H.default_scale(), *FMT(group, bits))
+    step = B.DecodeStep(*args, return_lse=True, **kw)
+    assert step.plan()["warps_per_cta"] == 8 and step.plan()["launches"] == 1
+    out, lse = step.step(check=True)
+    o2, l2 = B.fwd_kvcache_int(*args, return_lse=True, num_splits=2, check=True, **kw)
+    # The path's own bounds: q * scale and p * scale are rounded to fp16 in both, in another order of sums; with bf16 the
+    # query, tail and output have 8 bits (the bounds are 8 times the fp16 ones).
+    dtype = "fp16" if x["q"].dtype == torch.float16 else "bf16"
+    assert (out.float() - o2.float()).abs().max() <= G.TOL_O[dtype] * max(1.0, float(o2.float().abs().max()))
+    inf = torch.isinf(l2)
+    assert torch.equal(torch.isinf(lse), inf) and ((lse - l2)[~inf].abs() <= G.TOL_LSE[dtype]).all()
+    return out, lse
+
+
+# (sequences, query heads, KV heads): clusters of 8, 4, 2 and 1 CTAs, and two CTAs in turn on an SM; one and two query tiles
+@pytest.mark.parametrize("b,h,h_k", [(1, 8, 8), (1, 4, 1), (4, 64, 8), (5, 18, 2), (9, 32, 8), (17, 8, 8), (24, 8, 8), (3, 16, 1)])
+@pytest.mark.parametrize("bits,group", [(4, 128), (4, 64), (4, 32), (2, 128), (2, 64), (2, 32)])
+def test_against_oracle_and_general_kernel(b, h, h_k, bits, group):
+    import bitladder_b200 as B
+    if bits == 2 and group == 32 and h > 8 * h_k:
+        pytest.skip("not built")
+    block = B.pack_block_tokens(bits)
+    dtype = "bf16" if (b + group) % 3 == 0 else "fp16"
+    s = 4 * block
+    x = H.gen_qkv(b, s, h, h_k, seed=b + group, dtype=dtype, res=40)
+    bufs = G.pack_gpu(B, x["k"], x["v"], bits, group)
+    # lengths at the edges of half blocks, blocks and tail items, empty ones among them
+    lens = torch.tensor([[0, 1, 16, 31, 32, block - 1, block, block + 1, block + 17, 3 * block, s - 1, s][i * 5 % 12] for i in range(b)],
+                        dtype=torch.int32)
+    tails = torch.tensor([[0, 1, 15, 16, 17, 40][i % 6] for i in range(b)], dtype=torch.int32)
+    kw = dict(cache_seqlens=lens.cuda(), res_lens=tails.cuda(), k_res=x["k_res"].cuda(), v_res=x["v_res"].cuda())
+    out, lse = _both(B, x, bufs, group, bits, **kw)
+    ref = H.oracle_pack(x["k"], x["v"], bits, group, dtype)
+    o_ref, l_ref = H.oracle_decode(x["q"], ref, H.default_scale(), bits, group, dtype, k_res=x["k_res"], v_res=x["v_res"],
+                                   res_lens=tails.numpy(), cache_seqlens=lens.numpy())
+    eo, el = G.errs(out, lse, o_ref, l_ref)
+    assert eo <= G.TOL_O[dtype] and el <= G.TOL_LSE[dtype]
+
+
+@pytest.mark.parametrize("bits", [4, 2])
+@pytest.mark.parametrize("s", [1, 128, 1000, 4096])
+def test_equal_lengths_strided_query_and_32_bit_output(bits, s):
+    import bitladder_b200 as B
+    cap = (s + 255) // 256 * 256
+    x = H.gen_qkv(3, cap, 12, 4, seed=s)
+    bufs = G.pack_gpu(B, x["k"], x["v"], bits, 128)
+    wide = torch.zeros(3, 1, 24, 128, dtype=torch.float16, device="cuda")
+    wide[:, :, ::2] = x["q"].cuda()
+    args = (*bufs, None, H.default_scale(), *FMT(128, bits))
+    got = B.fwd_kvcache_int(wide[:, :, ::2], *args, seqlen_k=s, out_dtype=torch.float32)
+    want = B.fwd_kvcache_int(x["q"].cuda(), *args, seqlen_k=s, out_dtype=torch.float32, num_splits=1)
+    assert got.dtype == torch.float32 and (got - want).abs().max() <= 2e-3
+
+
+@pytest.mark.parametrize("bits", [4, 2])
+def test_pages_in_any_order_and_one_outside_the_pool(bits):
+    import bitladder_b200 as B
+    from bitladder_b200 import _lib
+    b, h, h_k, page, per = 3, 8, 2, 256, 4
+    x = H.gen_qkv(b, page * per, h, h_k, seed=5)
+    table = torch.randperm(b * per, generator=torch.Generator().manual_seed(3)).to(torch.int32).view(b, per)
+    pool = [torch.empty(b * per, page, h_k, 128, dtype=torch.float16) for _ in range(2)]
+    for p, t in zip(pool, (x["k"], x["v"])):
+        p[table.flatten().long()] = t.reshape(b * per, page, h_k, 128)
+    bufs = G.pack_gpu(B, *pool, bits, 128)
+    lens = torch.tensor([page * per, 300, 700], dtype=torch.int32)
+    out, lse = _both(B, x, bufs, 128, bits, table=table.cuda(), cache_seqlens=lens.cuda())
+    ref = H.oracle_pack(x["k"], x["v"], bits, 128, "fp16")
+    o_ref, l_ref = H.oracle_decode(x["q"], ref, H.default_scale(), bits, 128, "fp16", cache_seqlens=lens.numpy())
+    eo, el = G.errs(out, lse, o_ref, l_ref)
+    assert eo <= 2e-3 and el <= 2e-3
+    table[0, per - 1] = b * per + 7
+    step = B.DecodeStep(x["q"].cuda(), *bufs, table.cuda(), H.default_scale(), *FMT(128, bits), cache_seqlens=lens.cuda())
+    out = step.step()
+    assert step.status() == _lib.BD_ERR_PAGE
+    lens[0] = page * (per - 1)
+    o_ref, _ = H.oracle_decode(x["q"], ref, H.default_scale(), bits, 128, "fp16", cache_seqlens=lens.numpy())
+    assert np.abs(out[:, 0].float().cpu().numpy() - o_ref).max() <= 2e-3
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("rotary_dim,interleaved", [(128, True), (128, False), (64, False), (48, True), (32, False), (16, False)])
+def test_rotation_while_loading_files_the_same_key(dtype, rotary_dim, interleaved):
+    """Tables that do not start on 16 bytes take the rotary kernel in front: the same bits in the tail, and the same output up
+    to nothing at all, as the rotated query is the same too."""
+    import bitladder_b200 as B
+    x = H.gen_qkv(3, 512, 8, 2, seed=rotary_dim, dtype=dtype, res=64)
+    bufs = G.pack_gpu(B, x["k"], x["v"], 4, 128)
+    g = torch.Generator().manual_seed(1)
+    tdt = torch.float16 if dtype == "fp16" else torch.bfloat16
+    flat = [torch.randn(700 * rotary_dim // 2 + 8, generator=g).to(tdt).cuda() for _ in range(2)]
+    new = [torch.randn(3, 1, 2, 128, generator=g).to(tdt).cuda() for _ in range(2)]
+    got = []
+    for off in (0, 1):
+        tabs = [torch.empty(700 * rotary_dim // 2 + 8, dtype=tdt, device="cuda")[off:off + 700 * rotary_dim // 2] for _ in range(2)]
+        for t, f in zip(tabs, flat):
+            t.copy_(f[:t.numel()])
+        tail = [x["k_res"].cuda().clone(), x["v_res"].cuda().clone()]
+        step = B.DecodeStep(x["q"].cuda(), *bufs, None, H.default_scale(), *FMT(128, 4), return_lse=True, k_res=tail[0], v_res=tail[1],
+                            cache_seqlens=torch.tensor([512, 100, 0], dtype=torch.int32, device="cuda"),
+                            res_lens=torch.tensor([0, 17, 63], dtype=torch.int32, device="cuda"), k_new=new[0], v_new=new[1],
+                            rotary_cos=tabs[0].view(700, -1), rotary_sin=tabs[1].view(700, -1), rotary_interleaved=interleaved)
+        assert step.plan()["launches"] == 1 + off
+        out, lse = step.step(check=True)
+        got.append([out.clone(), lse.clone(), *tail])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
