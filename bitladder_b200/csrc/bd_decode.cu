@@ -111,7 +111,8 @@ struct Cfg {
     static constexpr size_t OFF_FLAGS = OFF_BAR + 2 * WARPS * 8;            // abort flag, arrivals[WARPS], segment notes[WARPS][4]
     static constexpr size_t OFF_NOTES = OFF_FLAGS + 16 + ((WARPS * 4 + 15) / 16) * 16;
     static constexpr size_t OFF_TABLE = OFF_NOTES + WARPS * 16;             // a small ragged batch's units (kInlineSeqs + 1 entries)
-    static constexpr size_t SMEM = OFF_TABLE + (kInlineSeqs + 1) * 8;
+    static constexpr size_t OFF_LAST = OFF_TABLE + (kInlineSeqs + 1) * 8;   // the CTA's last segment: its note, then the sequence (or -1)
+    static constexpr size_t SMEM = OFF_LAST + 32;
     static constexpr int DEPOSIT_FLOATS = NACC * 32;                        // one warp's share of a segment
     static_assert(DEPOSIT_FLOATS * 4 <= 2 * CODE_BYTES, "a deposit fits the warp's own tile slots");
     static constexpr int CTAS_PER_SM = (SMEM + 1024) * 3 <= 233472 ? 3 : ((SMEM + 1024) * 2 <= 233472 ? 2 : 1);
@@ -169,9 +170,24 @@ struct BlockCursor {
     }
 };
 
+// Element e of m-tile mt of an accumulator: the head dim of fragment row 0.
+template <int BITS> __device__ __forceinline__ constexpr int dim_of(int mt, int e) {
+    const int jv = (BITS == 4) ? (mt & 3) : mt;
+    return ((BITS == 4) ? 16 * (mt >> 2) : 0) + 8 * (e >> 1) + (kHeadDim * BITS / 16) * jv;
+}
+__device__ __forceinline__ void store_out(const DecodeParams &p, int64_t i, float v) {
+    if (p.out_dtype == BD_FP16) static_cast<__half *>(p.out)[i] = __float2half_rn(v);
+    else if (p.out_dtype == BD_BF16) static_cast<__nv_bfloat16 *>(p.out)[i] = __float2bfloat16_rn(v);
+    else static_cast<float *>(p.out)[i] = v;
+}
+
 // RAGGED: per-sequence lengths are compiled in; a uniform batch has no table of units and runs without that code in
 // its start (b1, 4096 tokens: 10.7 us with it, 10.2 without; b8, 32768 tokens and a tail: 56.7, 56.2).
-template <int BITS, int GROUP, int NQT, int TWO, bool RAGGED>
+// FEW: a step of few long sequences (DecodeParams::defer_merge is set): the warps of a CTA put its last sequence together
+// behind the loop, all of them, instead of the one that arrives last (b1, 32768 tokens 17.5 -> 16.2 us, 2 x 16384, 64/8
+// heads, group 64 18.2 -> 16.9).  Steps of many sequences would run that code and a single warp's, each once and so at
+// the speed of instruction fetch (b16 ragged and paged 25.6 -> 28.4 us), and both in one kernel cost the others registers.
+template <int BITS, int GROUP, int NQT, int TWO, bool RAGGED, bool FEW>
 __global__ void __launch_bounds__(Cfg<BITS, GROUP, NQT, TWO>::THREADS, Cfg<BITS, GROUP, NQT, TWO>::CTAS_PER_SM)
 bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                  const __grid_constant__ CUtensorMap vmap) {
@@ -191,6 +207,8 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
     const int ih = blockIdx.x % p.h_k, row = blockIdx.x / p.h_k;
     const int g = lane >> 2, l = lane & 3;
     int4 *note = reinterpret_cast<int4 *>(smem + C::OFF_NOTES) + warp;       // this warp's notes on its current segment
+    int4 *last_note = reinterpret_cast<int4 *>(smem + C::OFF_LAST);
+    volatile int *last_seq = reinterpret_cast<volatile int *>(smem + C::OFF_LAST + 16);
 #ifdef BD_TRACE
     if (tid == 0 && blockIdx.x < 4096) {
         g_trace[blockIdx.x * 32 + 0] = trace_smid();
@@ -215,6 +233,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
         mbar_init(kbar, 1);
         mbar_init(vbar, 1);
         if (warp == 0) *abort_flag = 0;
+        if (FEW && warp == 0) *last_seq = -1;
         arrivals[warp] = 0;
         fence_mbar_init();
         tma_prefetch_desc(&kmap);
@@ -415,6 +434,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
             const uint32_t share_mask = __ballot_sync(0xffffffffu, shares);
             const uint32_t on_mask = __ballot_sync(0xffffffffu, shares && hi > seq_end);
             const int goes_on = on_mask ? 31 - __clz(on_mask) : -1;
+            const bool ends_cta = FEW && __shfl_sync(0xffffffffu, quo, kWarps) <= seq_end;      // the last sequence of the CTA's range
             PartRange pr{0, -1, true};
             if (seq_n > 0 && Tw > 0) {
                 pr.c0 = int(__shfl_sync(0xffffffffu, quo, 16));
@@ -427,7 +447,8 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                 for (int c = pr.c0; c <= pr.c1; ++c) nparts += row_has_part(part, ib, c) ? 1 : 0;
             }
             if (lane == 0)
-                *note = make_int4(int(share_mask), (goes_on + 1) | ((pr.c1 - pr.c0 + 1) << 8), pr.c0, (nparts << 1) | (pr.dense ? 1 : 0));
+                *note = make_int4(int(share_mask), (goes_on + 1) | (ends_cta ? 128 : 0) | ((pr.c1 - pr.c0 + 1) << 8), pr.c0,
+                                  (nparts << 1) | (pr.dense ? 1 : 0));
             __syncwarp();
         }
 #pragma unroll
@@ -908,16 +929,23 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                 acc[32 * NQT + nq * 4 + 2 + c] = sum;
             }
         }
-        // The warps that share the sequence each deposit their partial and count in; the one that counts
-        // in last folds the deposits in warp order (so the result does not depend on who was last).  A
+        // The warps that share a sequence which ends inside the CTA's range each deposit their partial and count in; the one
+        // that counts in last folds the deposits in warp order (so the result does not depend on who was last).  A
         // warp whose range ends inside the sequence deposits into its own tile slots; the one warp in
         // whose range the sequence ends goes on streaming and deposits through global memory.
         const int4 nt = *note;
         const uint32_t share_mask = uint32_t(nt.x);
-        const int goes_on = (nt.y & 0xff) - 1;
+        const int goes_on = (nt.y & 127) - 1;
         const int nshare = __popc(share_mask);
+        // The last sequence of the CTA's range: nobody goes on, all of the CTA's warps put it together behind the loop.
+        const bool together = FEW && (nt.y & 128) && (nshare > 1 || (nt.w >> 1) > 1);
+        if (together && warp == __ffs(share_mask) - 1 && lane == 0) {
+            *last_note = nt;
+            *last_seq = ib;
+        }
+        int old = 0;
         bool finisher = true;
-        if (nshare > 1) {
+        if (nshare > 1 || together) {
             float *gdep = p.warp_acc + (int64_t(ib) * p.h_k + ih) * C::DEPOSIT_FLOATS;
             if (goes_on == warp) {
 #pragma unroll
@@ -930,7 +958,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                 __threadfence_block();
             }
             __syncwarp();
-            int old = 0;
+            if (together) continue;
             if (lane == 0) old = atomicAdd(arrivals + (__ffs(share_mask) - 1), 1);
             old = __shfl_sync(0xffffffffu, old, 0);
             finisher = old == nshare - 1;
@@ -1041,7 +1069,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
             }
             // With many parts per sequence (few long sequences) the merge is left to a second,
             // fully parallel kernel: one warp doing it here would be the tail of the whole step.
-            if (!final_here && !p.defer_merge) {
+            if (!FEW && !final_here && !p.defer_merge) {
                 // publish the partial, count arrivals; the last one merges (same arithmetic as
                 // the reference's combine kernel, flash_fwd_kernel.h:1217-1231, 1280-1298)
                 __threadfence();
@@ -1197,10 +1225,69 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
     }
 
     // ======================================================================
-    // after the stream: error exit
+    // after the stream: the CTA's last sequence, put together by all of its warps
     // ======================================================================
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // a merge kernel staged behind this one may be placed
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // a kernel staged behind this one may be placed
     __syncthreads();
+    BD_TRACE_MARK(16);
+    if (FEW && *last_seq >= 0) {
+        const int4 nt = *last_note;
+        const int ib = *last_seq;
+        const bool final_here = (nt.w >> 1) <= 1 && !p.leave_parts;      // (a sequence split over GPUs always leaves parts)
+        const int64_t slot = (int64_t(row) + ib) * p.h_k + ih;
+        // four values per thread of all deposits a warp and round, in the deposits' order (the result does not depend on
+        // who was when)
+#pragma unroll 1
+        for (int mt = warp; mt < 8 * NQT; mt += kWarps) {
+            const int nq = mt >> 3;
+            float mm[kWarps][2], ll[kWarps][2], M[2] = {-INFINITY, -INFINITY}, L[2] = {0.f, 0.f}, o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int d = 0; d < kWarps; ++d) {
+                if (!((nt.x >> d) & 1)) continue;
+                const float *dep = reinterpret_cast<const float *>(smem + size_t(d) * 2 * C::CODE_BYTES) + lane;
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    mm[d][c] = dep[(32 * NQT + nq * 4 + c) * 32];
+                    ll[d][c] = dep[(32 * NQT + nq * 4 + 2 + c) * 32];
+                    M[c] = fmaxf(M[c], mm[d][c]);
+                }
+            }
+#pragma unroll
+            for (int d = 0; d < kWarps; ++d) {
+                if (!((nt.x >> d) & 1)) continue;
+                const float *dep = reinterpret_cast<const float *>(smem + size_t(d) * 2 * C::CODE_BYTES) + lane;
+                float f[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    f[c] = (mm[d][c] == -INFINITY) ? 0.f : ex2f(mm[d][c] - M[c]);
+                    L[c] = fmaf(f[c], ll[d][c], L[c]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[e] = fmaf(f[e & 1], dep[(mt * 4 + e) * 32], o[e]);
+            }
+            // one part: the final result; more: a normalised partial
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float inv = (L[c] > 0.f) ? 1.0f / L[c] : 0.f;
+                const int qrow = nq * 8 + 2 * l + c;
+                if (qrow >= p.gq) continue;
+                const int64_t hq = int64_t(ih) * p.gq + qrow;
+                if ((mt & 7) == 0 && g == 0) {
+                    const float lse = (L[c] > 0.f) ? fmaf(M[c], 0.6931471805599453f, logf(L[c])) : -INFINITY;
+                    if (!final_here) p.part_lse[slot * p.gq + qrow] = lse;
+                    else if (p.lse) p.lse[int64_t(ib) * p.h + hq] = lse;
+                }
+#pragma unroll
+                for (int eh = 0; eh < 2; ++eh) {
+                    const int dim = dim_of<BITS>(mt & 7, 2 * eh + c) + g;
+                    const float v = o[2 * eh + c] * inv;
+                    if (final_here) store_out(p, ib * p.out_stride_b + hq * p.out_stride_h + dim, v);
+                    else p.part_out[(slot * p.gq + qrow) * kHeadDim + dim] = v;
+                }
+            }
+        }
+        BD_TRACE_MARK(17);
+    }
 #ifdef BD_TRACE
     if (tid == 0 && blockIdx.x < 4096) g_trace[blockIdx.x * 32 + 15] = trace_now();
 #endif
@@ -1374,11 +1461,11 @@ __global__ void __launch_bounds__(256) bd_prefix_kernel(const PrefixParams p) {
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-template <int BITS, int GROUP, int NQT, int TWO, bool RAGGED>
+template <int BITS, int GROUP, int NQT, int TWO, bool RAGGED, bool FEW>
 static cudaError_t launch_r(const DecodeParams &p, const CUtensorMap &kmap, const CUtensorMap &vmap,
                             cudaStream_t stream) {
     using C = Cfg<BITS, GROUP, NQT, TWO>;
-    auto kern = bd_decode_kernel<BITS, GROUP, NQT, TWO, RAGGED>;
+    auto kern = bd_decode_kernel<BITS, GROUP, NQT, TWO, RAGGED, FEW>;
     static bool configured[64] = {};
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
@@ -1404,8 +1491,14 @@ static cudaError_t launch_r(const DecodeParams &p, const CUtensorMap &kmap, cons
 template <int BITS, int GROUP, int NQT, int TWO>
 static cudaError_t launch_t(const DecodeParams &p, const CUtensorMap &kmap, const CUtensorMap &vmap,
                             cudaStream_t stream) {
-    if (p.part.table != nullptr) return launch_r<BITS, GROUP, NQT, TWO, true>(p, kmap, vmap, stream);
-    return launch_r<BITS, GROUP, NQT, TWO, false>(p, kmap, vmap, stream);
+    if constexpr (NQT == 1 && TWO == 0) {
+        if (p.defer_merge) {
+            if (p.part.table != nullptr) return launch_r<BITS, GROUP, NQT, TWO, true, true>(p, kmap, vmap, stream);
+            return launch_r<BITS, GROUP, NQT, TWO, false, true>(p, kmap, vmap, stream);
+        }
+    }
+    if (p.part.table != nullptr) return launch_r<BITS, GROUP, NQT, TWO, true, false>(p, kmap, vmap, stream);
+    return launch_r<BITS, GROUP, NQT, TWO, false, false>(p, kmap, vmap, stream);
 }
 
 template <int BITS, int GROUP>
