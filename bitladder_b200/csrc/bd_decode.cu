@@ -275,6 +275,12 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
         return ok;
     };
     bool starve = p.test_starve != 0 && blockIdx.x == 0;     // test hook: the first K copy of every warp of CTA 0
+    // The lane that issues copies.  Elected, their operands stay in uniform registers (see elect_one): 2 bits, 1 x 131072
+    // tokens 34.4 -> 33.2 us (group 64) and 33.1 -> 31.7, 8 x 32768 64.0 -> 62.3; 4 bits, group 64, ragged 24.0 -> 23.0.  Two
+    // kinds of kernel are short of a register then: equal lengths at 4 bits and group 128 (8 x 32768 tokens 57.3 -> 58.1)
+    // and two query tiles (2 x 200000 28.4 -> 28.7) keep lane 0.
+    constexpr bool kElect = NQT == 1 && (BITS == 2 || GROUP != 128 || RAGGED || FEW);
+    auto issuing_lane = [&]() { return kElect ? elect_one() : lane == 0; };
     auto issue_k = [&](int ib, int blk) {
         resolve(ib, blk);
         mbar_arrive_expect_tx(kbar, C::CODE_BYTES + PRM + (starve ? 16 : 0));
@@ -325,7 +331,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
     ld.init(walk, cache_seqlens, p.s, NB);
     BD_TRACE_MARK(27);
     if constexpr (!RAGGED) asm volatile("griddepcontrol.wait;" ::: "memory");     // (nothing in global memory was read so far)
-    if (ld.valid && lane == 0) {
+    if (ld.valid && issuing_lane()) {
         issue_k(ld.sg.ib, ld.u);
         issue_v(ld.sg.ib, ld.u);
     }
@@ -841,7 +847,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                     if (ug == 1) {
                         // K tile consumed: refill it with the next block's K
                         __syncwarp();
-                        if (lane == 0 && ld.valid) {
+                        if (ld.valid && issuing_lane()) {
                             fence_proxy_async();
                             issue_k(ld.sg.ib, ld.u);
                         }
@@ -857,7 +863,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
             } else {
             // K tile consumed: refill it with the next block's K while V is processed
             __syncwarp();
-            if (lane == 0 && ld.valid) {
+            if (ld.valid && issuing_lane()) {
                 fence_proxy_async();
                 issue_k(ld.sg.ib, ld.u);
             }
@@ -884,7 +890,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
             // V tile consumed: refill it, then move the load cursor on
             __syncwarp();
             if (ld.valid) {
-                if (lane == 0) {
+                if (issuing_lane()) {
                     fence_proxy_async();
                     issue_v(ld.sg.ib, ld.u);
                 }
