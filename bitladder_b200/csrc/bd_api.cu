@@ -124,6 +124,7 @@ int plan_rows(int b, int h_k, int64_t max_s, int bits, int sm_count, int ctas_pe
 //   one sequence, 32/8 heads, 4 bits      2: 11.6 -> 8.2, 3: 12.1 -> 9.9, 4: 12.8 -> 11.6, 6: 15.0 -> 15.0, 8: 17.5 -> 18.3
 //   8 sequences, ragged, tails            1.6: 12.1 -> 7.6, 2.6: 12.6 -> 9.3, 4.5: 15.0 -> 12.8, 6.4: 18.4 -> 16.2
 //   one sequence, 64/8 heads, 2 bits      2: 13.0 -> 8.0, 4: 15.1 -> 11.4, 6: 15.6 -> 14.9, 8: 16.5 -> 18.3
+//   3 sequences, 16/4 heads, 2 bits       4.9: 25.0 -> 21.8, ragged 19.8 -> 21.4
 //   30 sequences, 8/1 heads, group 32     1: 14.3 -> 7.5, 2: 14.8 -> 10.4, 4: 16.3 -> 16.3
 // and with twice as many pairs of sequence and KV head as SMs (two CTAs in turn on every SM; three in turn lose):
 //   32 sequences, 32/8 heads, 4 bits      0.3: 6.3 -> 7.7, 1: 10.7 -> 9.5, 2: 15.3 -> 13.1, 4: 22.4 -> 20.0
@@ -141,7 +142,7 @@ int short_cluster(const bd_decode_args *a, int sm_count, int64_t nblk) {
     const int64_t round = int64_t(c) * bd::kShortWarps;
     if (pairs > sm_count) return items <= 4 * round && (ragged || items >= round) ? c : 0;
     if (a->bits == 4 && !ragged && a->k_res == nullptr) return items < 4 * round ? c : 0;
-    return items <= (a->group == 32 ? 4 : 6) * round ? c : 0;
+    return items <= (a->group == 32 || (a->bits == 2 && ragged) ? 4 : 6) * round ? c : 0;
 }
 
 int make_plan(const bd_decode_args *a, int sm_count, DecodePlan &plan) {
