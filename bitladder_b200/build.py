@@ -24,7 +24,7 @@ LIB_PATH = os.path.join(_HERE, "libbitdecode.so")
 CALLS_PATH = os.path.join(_HERE, "_torch_calls.so")
 CALLS_SOURCE = os.path.join(CSRC, "bd_torch.cpp")
 SOURCES = ["bd_pack.cu", "bd_decode.cu", "bd_decode_short.cu", "bd_combine.cu", "bd_exchange.cu", "bd_rope.cu", "bd_api.cu"]
-HEADERS = ["bd_common.cuh", "bd_decode.cuh", "bd_kernels.h", os.path.join("..", "..", "include", "bitdecode.h")]
+HEADERS = ["bd_common.cuh", "bd_decode.cuh", "bd_pack.cuh", "bd_kernels.h", os.path.join("..", "..", "include", "bitdecode.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -34,11 +34,11 @@ NVCC_FLAGS = [
 ]
 
 
-# Per-file additions.  The decode kernels may use the approximate exp/log/division and
+# Per-file additions.  The decode kernel may use the approximate exp/log/division and
 # flush-to-zero fp32 (its parity bound is 2e-3 and these act on softmax weights and the final
 # normalisation; measured 0.8 us on a 63 us step).  The pack kernel must NOT: its quantizer is
 # bit-exact IEEE arithmetic with explicit rounding intrinsics.
-PER_FILE_FLAGS = {"bd_decode.cu": ["--use_fast_math"], "bd_decode_short.cu": ["--use_fast_math"]}
+PER_FILE_FLAGS = {"bd_decode.cu": ["--use_fast_math"]}
 
 
 def _nvcc() -> str:

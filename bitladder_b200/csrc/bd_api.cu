@@ -354,7 +354,7 @@ int bd_decode_plan(const bd_decode_args *a, int32_t out[4]) {
         out[0] = a->b * plan.cluster;
         out[1] = 1;
         out[2] = bd::kShortWarps;
-        out[3] = 1 + (a->rotary_dim > 0 && !rotary_in_decode(a) ? 1 : 0) + (a->advance ? 1 : 0);
+        out[3] = 1 + (a->rotary_dim > 0 && !rotary_in_decode(a) ? 1 : 0);
         return BD_OK;
     }
     out[0] = plan.rows;
@@ -590,28 +590,11 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     p.defer_merge = (x || plan.rows > 4 * a->b) ? 1 : 0;
     p.leave_parts = x ? 1 : 0;
     p.two_ctas = plan.two_ctas;
-    p.cluster = plan.cluster;
-    err = is_short ? bd::launch_decode_short(p, kmap, vmap, a->bits, a->group, stream)
-                   : bd::launch_decode(p, kmap, vmap, a->bits, a->group, stream);
-    if (err != cudaSuccess) return BD_ERR_CUDA;
-    if (x) {
-        xp.part_out = p.part_out; xp.part_lse = p.part_lse;
-        xp.out = p.out; xp.lse = p.lse;
-        xp.out_stride_b = p.out_stride_b; xp.out_stride_h = p.out_stride_h;
-        xp.h = p.h; xp.out_dtype = p.out_dtype;
-        xp.part = p.part; xp.h_k = p.h_k; xp.gq = p.gq;
-        err = bd::launch_exchange_parts(xp, stream);
-        if (err != cudaSuccess) return BD_ERR_CUDA;
-    } else if (p.defer_merge && !is_short) {
-        err = bd::launch_merge_parts(p, true, stream);
-        if (err != cudaSuccess) return BD_ERR_CUDA;
-    }
-
+    PackParams pk;
+    std::memset(&pk, 0, sizeof(pk));
     if (a->advance) {
         // roll-over: tails that this step's token filled become the next pack block of their sequence, and every
         // sequence's lengths move on
-        PackParams pk;
-        std::memset(&pk, 0, sizeof(pk));
         pk.k = a->k_res; pk.v = a->v_res;
         pk.k_stride_b = pk.v_stride_b = a->res_stride_b;
         pk.k_stride_s = pk.v_stride_s = a->res_stride_s;
@@ -627,6 +610,25 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
         pk.roll_arrivals = p.counters;                            // zero again when the decode kernel is done
         pk.roll_status = reinterpret_cast<int32_t *>(ws);
         pk.roll_s_cap = a->s_cap; pk.roll_res_cap = std::min(a->res_len, bd::kTailMax);
+    }
+    p.cluster = plan.cluster;
+    err = is_short ? bd::launch_decode_short(p, pk, kmap, vmap, a->bits, a->group, stream)
+                   : bd::launch_decode(p, kmap, vmap, a->bits, a->group, stream);
+    if (err != cudaSuccess) return BD_ERR_CUDA;
+    if (x) {
+        xp.part_out = p.part_out; xp.part_lse = p.part_lse;
+        xp.out = p.out; xp.lse = p.lse;
+        xp.out_stride_b = p.out_stride_b; xp.out_stride_h = p.out_stride_h;
+        xp.h = p.h; xp.out_dtype = p.out_dtype;
+        xp.part = p.part; xp.h_k = p.h_k; xp.gq = p.gq;
+        err = bd::launch_exchange_parts(xp, stream);
+        if (err != cudaSuccess) return BD_ERR_CUDA;
+    } else if (p.defer_merge && !is_short) {
+        err = bd::launch_merge_parts(p, true, stream);
+        if (err != cudaSuccess) return BD_ERR_CUDA;
+    }
+
+    if (a->advance && !is_short) {
         err = bd::launch_pack(pk, a->bits, a->group, a->dtype, stream);
         if (err != cudaSuccess) return BD_ERR_CUDA;
     }

@@ -12,11 +12,14 @@
 //    the output; then the CTAs' results the same way in the shared memory of the cluster's first CTA.  No second
 //    kernel, no counters, no trip to L2.
 //  * With rotary embedding, q and the new key are rotated where they are loaded (bd_rope.cu's arithmetic).
+//  * A decoder step's bookkeeping is done here too: the lengths move on, and a tail that the step has filled is packed
+//    by the cluster that has just read it (bd_pack.cuh): one kernel a token.
 //
 // Measured against bd_decode.cu: see launch_decode_short's rule in bd_api.cu.
 #include <type_traits>
 
 #include "bd_decode.cuh"
+#include "bd_pack.cuh"
 
 namespace bd {
 
@@ -114,7 +117,8 @@ __device__ __forceinline__ void rotate8(const DecodeParams &p, const uint16_t *x
 
 template <int BITS, int GROUP, int NQT>
 __global__ void __launch_bounds__(ShortCfg<BITS, GROUP, NQT>::THREADS, 1)
-bd_decode_short_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap) {
+bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid_constant__ CUtensorMap kmap,
+                       const __grid_constant__ CUtensorMap vmap) {
     using C = ShortCfg<BITS, GROUP, NQT>;
     constexpr int P = C::P, NB = C::NB, NGK = C::NGK, FPG = C::FPG, NGD = C::NGD, FPGV = C::FPGV, NZ = C::NZ;
     constexpr int DP = C::DP, RUNS = C::RUNS, PRM = C::PRM, STAGES = C::STAGES, WARPS = C::WARPS;
@@ -211,6 +215,13 @@ bd_decode_short_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap
         if (unit0 + st * stride < items) issue(unit0 + st * stride, st);
     __syncwarp();
 
+    // The lengths move on when every warp that works on the sequence has read them: each counts in behind its reads, and the
+    // last one writes at its end (the answer has that long to arrive).
+    int arrived = -1;
+    if (roll.roll_res_lens != nullptr && lane == 0) {
+        __threadfence();
+        arrived = atomicAdd(roll.roll_arrivals + int64_t(ib) * p.h_k, 1);
+    }
     int pos = max(cached, 0) + max(in_tail, 0);          // of this step's token
     if (p.rotary_dim > 0 && pos >= p.rotary_positions) {
         if (tid == 0 && rank == 0) atomicExch(p.status, BD_ERR_POSITION);
@@ -630,10 +641,10 @@ bd_decode_short_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap
         float inv[2];
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-            inv[c] = L[c] > 0.f ? 1.0f / L[c] : 0.f;
+            inv[c] = L[c] > 0.f ? __fdividef(1.0f, L[c]) : 0.f;
             const int r = mq * 8 + 2 * l + c;
             if (p.lse && e0 % 32 == 0 && g == 0 && r < p.gq)
-                p.lse[int64_t(ib) * p.h + hq0 + r] = L[c] > 0.f ? fmaf(M[c], 0.6931471805599453f, logf(L[c])) : -INFINITY;
+                p.lse[int64_t(ib) * p.h + hq0 + r] = L[c] > 0.f ? fmaf(M[c], 0.6931471805599453f, __logf(L[c])) : -INFINITY;
         }
 #pragma unroll
         for (int i = 0; i < EPW; ++i) {
@@ -649,6 +660,46 @@ bd_decode_short_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap
             else static_cast<float *>(p.out)[oi] = v;
         }
     }
+    if (roll.roll_res_lens != nullptr) {
+        // as bd_pack.cu does it behind the general kernel
+        const bool room = cached >= 0 && cached % NB == 0 && cached + NB <= roll.roll_s_cap;
+        if (arrived == p.h_k * ncta * WARPS - 1) {
+            __threadfence();
+            roll.roll_arrivals[int64_t(ib) * p.h_k] = 0;
+            int r = min(max(in_tail, 0), roll.roll_res_cap);
+            if (r < roll.roll_res_cap) r += 1;
+            if (r == NB) {
+                if (room) {
+                    roll.roll_cache_seqlens[ib] = cached + NB;
+                    r = 0;
+                } else {
+                    atomicExch(roll.roll_status, BD_ERR_CAPACITY);
+                }
+            }
+            roll.roll_res_lens[ib] = r;
+        }
+        if (in_tail + 1 == NB && room) {
+            // (the token's own row, stored by one of the cluster's warps, is visible behind the barriers above)
+            static_assert(PackCfg<BITS, GROUP>::NTHREADS == 128 && WARPS == 8, "two groups of threads pack");
+            static_assert(sizeof(typename PackCfg<BITS, GROUP>::Shared) <= 16384 && C::OFF_PRM >= 32768, "in the warps' tiles");
+            constexpr int SPLIT = PackCfg<BITS, GROUP>::SPLIT;
+            const int group = warp >> 2, t = tid & 127;
+            auto &sh = *reinterpret_cast<typename PackCfg<BITS, GROUP>::Shared *>(smem + group * 16384);
+            auto sync = [&] { asm volatile("barrier.cta.sync %0, 128;" ::"r"(1 + group) : "memory"); };
+            __syncthreads();
+#pragma unroll 1
+            for (int part = 2 * rank + group; part < 2 * SPLIT; part += 2 * ncta) {
+                if (part < SPLIT) {
+                    if (bf16) pack_k_part<BITS, GROUP, true>(roll, sh, t, ib, ih, part, 0, cached / NB, sync);
+                    else pack_k_part<BITS, GROUP, false>(roll, sh, t, ib, ih, part, 0, cached / NB, sync);
+                } else {
+                    if (bf16) pack_v_part<BITS, GROUP, true>(roll, sh, t, ib, ih, part - SPLIT, 0, cached / NB, sync);
+                    else pack_v_part<BITS, GROUP, false>(roll, sh, t, ib, ih, part - SPLIT, 0, cached / NB, sync);
+                }
+                sync();
+            }
+        }
+    }
     if (*abort_flag != 0) {
         if (tid == 0) atomicExch(p.status, BD_ERR_TIMEOUT);
         // give copies that are still in flight time to land before the block's shared memory is released
@@ -661,7 +712,7 @@ bd_decode_short_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap
 // host side
 // ---------------------------------------------------------------------------
 template <int BITS, int GROUP, int NQT>
-static cudaError_t launch_short(const DecodeParams &p, const CUtensorMap &kmap, const CUtensorMap &vmap, cudaStream_t stream) {
+static cudaError_t launch_short(const DecodeParams &p, const PackParams &roll, const CUtensorMap &kmap, const CUtensorMap &vmap, cudaStream_t stream) {
     using C = ShortCfg<BITS, GROUP, NQT>;
     auto kern = bd_decode_short_kernel<BITS, GROUP, NQT>;
     static bool configured[64] = {};
@@ -687,7 +738,7 @@ static cudaError_t launch_short(const DecodeParams &p, const CUtensorMap &kmap, 
     at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = p.cluster > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kern, p, kmap, vmap);
+    return cudaLaunchKernelEx(&cfg, kern, p, roll, kmap, vmap);
 }
 
 #define BD_SHORT_PICK(RESULT)                                                                           \
@@ -699,10 +750,10 @@ static cudaError_t launch_short(const DecodeParams &p, const CUtensorMap &kmap, 
     if (bits == 2 && group == 64) { if (one) RESULT(2, 64, 1) else RESULT(2, 64, 2) }                   \
     if (bits == 2 && group == 32 && one) RESULT(2, 32, 1)      /* two query tiles: a result does not fit the one stage there is */
 
-cudaError_t launch_decode_short(const DecodeParams &p, const CUtensorMap &kmap, const CUtensorMap &vmap, int bits, int group,
-                                cudaStream_t stream) {
+cudaError_t launch_decode_short(const DecodeParams &p, const PackParams &roll, const CUtensorMap &kmap, const CUtensorMap &vmap,
+                                int bits, int group, cudaStream_t stream) {
     const int gq = p.gq;
-#define BD_SHORT_LAUNCH(B, G, Q) return launch_short<B, G, Q>(p, kmap, vmap, stream);
+#define BD_SHORT_LAUNCH(B, G, Q) return launch_short<B, G, Q>(p, roll, kmap, vmap, stream);
     BD_SHORT_PICK(BD_SHORT_LAUNCH)
     return cudaErrorInvalidValue;
 }

@@ -312,9 +312,10 @@ cudaError_t launch_prefix(const PrefixParams &p, cudaStream_t stream);
 cudaError_t launch_merge_parts(const DecodeParams &p, bool early, cudaStream_t stream);
 cudaError_t launch_decode(const DecodeParams &p, const CUtensorMap &kmap, const CUtensorMap &vmap,
                           int bits, int group, cudaStream_t stream);
-// A step with little work (bd_decode_short.cu); its maps have boxes of 16 rows.
+// A step with little work (bd_decode_short.cu); its maps have boxes of 16 rows.  With roll.roll_res_lens set the kernel also
+// does what bd_pack.cu's roll-over does.
 constexpr int kShortWarps = 8;    // warps per CTA
-cudaError_t launch_decode_short(const DecodeParams &p, const CUtensorMap &kmap, const CUtensorMap &vmap,
+cudaError_t launch_decode_short(const DecodeParams &p, const PackParams &roll, const CUtensorMap &kmap, const CUtensorMap &vmap,
                                 int bits, int group, cudaStream_t stream);
 int decode_short_cluster(int bits, int group, int gq);    // most CTAs per cluster; 0: not built
 // `two`: the variant with half as many warps per CTA and two CTAs per SM (see Cfg in bd_decode.cu)

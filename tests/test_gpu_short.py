@@ -120,3 +120,34 @@ def test_rotation_while_loading_files_the_same_key(dtype, rotary_dim, interleave
         got.append([out.clone(), lse.clone(), *tail])
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("bits,group,dtype,h,h_k", [(4, 128, "fp16", 8, 2), (4, 64, "bf16", 16, 16), (4, 32, "fp16", 18, 2), (2, 128, "bf16", 8, 8),
+                                                    (2, 64, "fp16", 4, 1), (2, 32, "fp16", 8, 2)])
+def test_roll_over_leaves_the_same_bytes_as_the_general_kernels(bits, group, dtype, h, h_k):
+    """A step with bookkeeping: tails that are not full, that this step fills, that fill with no room behind them, and a full
+    one; lengths, tails, packed bytes and the reported error are those of the general kernel and the roll-over kernel."""
+    import bitladder_b200 as B
+    block = B.pack_block_tokens(bits)
+    cap = 3 * block
+    tdt = torch.float16 if dtype == "fp16" else torch.bfloat16
+    x = H.gen_qkv(5, cap, h, h_k, seed=bits + group, dtype=dtype, res=block)
+    x["k_res"][:, ::7, :, 3] = 1e-39 if dtype == "bf16" else 6e-8       # subnormal rows are not flushed
+    g = torch.Generator().manual_seed(2)
+    new = [torch.randn(5, 1, h_k, 128, generator=g).to(tdt).cuda() for _ in range(2)]
+    got = []
+    for splits in (0, 2):
+        bufs = [t.clone() for t in G.pack_gpu(B, x["k"], x["v"], bits, group)]
+        tail = [x["k_res"].cuda().clone(), x["v_res"].cuda().clone()]
+        cs = torch.tensor([block, 0, 2 * block, cap, block], dtype=torch.int32, device="cuda")
+        rl = torch.tensor([block - 1, block - 1, block - 2, block - 1, block], dtype=torch.int32, device="cuda")
+        step = B.DecodeStep(x["q"].cuda(), *bufs, None, H.default_scale(), *FMT(group, bits), return_lse=True, k_res=tail[0], v_res=tail[1],
+                            cache_seqlens=cs, res_lens=rl, k_new=new[0], v_new=new[1], advance=True, num_splits=splits)
+        if splits == 0:
+            assert step.plan()["launches"] == 1
+        out, lse = step.step()
+        got.append(([t.view(torch.int16) for t in (*bufs, *tail)] + [cs, rl], out.float(), lse, step.status()))
+    (a, oa, la, sa), (b, ob, lb, sb) = got
+    assert all(torch.equal(s, t) for s, t in zip(a, b)) and sa == sb != 0
+    assert a[6].tolist()[:4] == [2 * block, block, 2 * block, cap]
+    assert (oa - ob).abs().max() <= G.TOL_O[dtype] * max(1.0, float(ob.abs().max())) and (la - lb).abs().max() <= G.TOL_LSE[dtype]
