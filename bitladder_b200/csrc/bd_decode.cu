@@ -274,17 +274,13 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
         ib = ok ? page : 0;
         return ok;
     };
-    bool starve = p.test_starve != 0 && blockIdx.x == 0;     // test hook: the first K copy of every warp of CTA 0
-    // The lane that issues copies.  Elected, their operands stay in uniform registers (see elect_one): 2 bits, 1 x 131072
-    // tokens 34.4 -> 33.2 us (group 64) and 33.1 -> 31.7, 8 x 32768 64.0 -> 62.3; 4 bits, group 64, ragged 24.0 -> 23.0.  Two
-    // kinds of kernel are short of a register then: equal lengths at 4 bits and group 128 (8 x 32768 tokens 57.3 -> 58.1)
-    // and two query tiles (2 x 200000 28.4 -> 28.7) keep lane 0.
-    constexpr bool kElect = NQT == 1 && (BITS == 2 || GROUP != 128 || RAGGED || FEW);
-    auto issuing_lane = [&]() { return kElect ? elect_one() : lane == 0; };
-    auto issue_k = [&](int ib, int blk) {
+    // (Issued by an elected lane, see elect_one: 2 bits, 1 x 131072 tokens 34.4 -> 33.2 us at group 64 and 33.1 -> 31.7 at 128,
+    // 8 x 32768 64.0 -> 62.3; 4 bits, group 64, ragged 24.0 -> 23.0.  `more`: bytes waited for that never come, a test hook; an
+    // argument and not a variable, whose register the loop needs: 1 x 131072 tokens 35.4 -> 34.7, 8 x 16000, 32/32 heads,
+    // 63.5 -> 62.1.)
+    auto issue_k = [&](int ib, int blk, uint32_t more = 0) {
         resolve(ib, blk);
-        mbar_arrive_expect_tx(kbar, C::CODE_BYTES + PRM + (starve ? 16 : 0));
-        starve = false;
+        mbar_arrive_expect_tx(kbar, C::CODE_BYTES + PRM + more);
         const int row0 = ib * p.k_batch_rows + blk * 32;
         tma_load_2d(kcode, &kmap, kbar, ih * kHeadDim, row0);
         tma_load_2d(kcode + 4096, &kmap, kbar, ih * kHeadDim + 64, row0);
@@ -331,8 +327,8 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
     ld.init(walk, cache_seqlens, p.s, NB);
     BD_TRACE_MARK(27);
     if constexpr (!RAGGED) asm volatile("griddepcontrol.wait;" ::: "memory");     // (nothing in global memory was read so far)
-    if (ld.valid && issuing_lane()) {
-        issue_k(ld.sg.ib, ld.u);
+    if (ld.valid && elect_one()) {
+        issue_k(ld.sg.ib, ld.u, p.test_starve != 0 && blockIdx.x == 0 ? 16 : 0);      // (test hook: CTA 0 waits for more than comes)
         issue_v(ld.sg.ib, ld.u);
     }
     if (ld.valid) { BD_TRACE_MARK(20); }
@@ -847,7 +843,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                     if (ug == 1) {
                         // K tile consumed: refill it with the next block's K
                         __syncwarp();
-                        if (ld.valid && issuing_lane()) {
+                        if (ld.valid && elect_one()) {
                             fence_proxy_async();
                             issue_k(ld.sg.ib, ld.u);
                         }
@@ -863,7 +859,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
             } else {
             // K tile consumed: refill it with the next block's K while V is processed
             __syncwarp();
-            if (ld.valid && issuing_lane()) {
+            if (ld.valid && elect_one()) {
                 fence_proxy_async();
                 issue_k(ld.sg.ib, ld.u);
             }
@@ -890,7 +886,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
             // V tile consumed: refill it, then move the load cursor on
             __syncwarp();
             if (ld.valid) {
-                if (issuing_lane()) {
+                if (elect_one()) {
                     fence_proxy_async();
                     issue_v(ld.sg.ib, ld.u);
                 }
