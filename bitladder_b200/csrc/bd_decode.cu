@@ -14,11 +14,13 @@
 //    tokens), two shared-memory slots (one K tile, one V tile) and their
 //    mbarriers, and refills a slot itself, with TMA, as soon as it has consumed
 //    it: the next block's K streams in during the V phase and vice versa.  No
-//    warp ever waits for another, anywhere in the kernel; each keeps its own running
+//    warp waits for another while it streams; each keeps its own running
 //    (max, sum, O).  At the end of a sequence's share the warps that hold a part of it
 //    deposit their partials and count in; the last to count in merges them in a fixed
 //    order, and the CTA that finishes a sequence last merges the CTAs' parts the same
-//    way.  The unquantized fp16/bf16 tail goes through the same tensor-core path and
+//    way.  (In steps of few long sequences the warps of a CTA meet behind the loop and
+//    merge together, see FEW, and a second kernel merges the CTAs' parts.)  The
+//    unquantized fp16/bf16 tail goes through the same tensor-core path and
 //    the same running state.
 //  * Packed codes go global -> shared with tiled TMA copies (128-byte swizzle
 //    for K, 64/32-byte swizzle for V, which makes the transposing ldmatrix on V
@@ -36,9 +38,13 @@
 //    tokens).  Products are exact in fp32; only q*scale and p*scale are rounded
 //    to fp16.
 //
-// tcgen05 is not used: its MMA needs M >= 64 rows of real work per instruction
-// and operands staged through shared memory or TMEM, while this kernel has at
-// most 16 query rows and is bound by HBM bandwidth, not tensor throughput.
+// Steps with little work run in bd_decode_short.cu (the rule: short_cluster in bd_api.cu).
+//
+// tcgen05 was built and measured, and is not used.  With tokens (head dims) as its M = 128 rows the masked fragments
+// below go to tensor memory unchanged, and an MMA of 16 query columns takes 9 cycles; but the masks, which are what
+// dispatch is spent on, stay the same, every step of 128 tokens passes four warps through three meetings, and three
+// warpgroups per SM took 3250 cycles a step where HBM allows 2180: 16 x 131072 tokens 586 us against 421 at 4 bits, 511 against
+// 333 at 2.  (Eight-bit operands would halve the masks at 2 bits; they need q * scale and p * scale split into bytes.)
 #include <type_traits>
 
 #include "bd_decode.cuh"

@@ -198,8 +198,8 @@ typedef struct bd_decode_args {
                                  res_lens[ib] = 0.  This is the roll-over of the reference's residual scheme
                                  (its imgs/scheme.png; residual_block_size in kernel_traits.h:76-85, not wired up
                                  in its snapshot).  Needs cache_seqlens and res_lens (both are then WRITTEN), a tail
-                                 buffer of at least NB rows, no block_table.  Runs as one small kernel behind the
-                                 decode kernel on the same stream.  No room left for the block: BD_ERR_CAPACITY in
+                                 buffer of at least NB rows, no block_table.  Done by the decode kernel itself in
+                                 steps with little work, else by one small kernel behind it.  No room left for the block: BD_ERR_CAPACITY in
                                  the status word, the tail stays full. */
     uint32_t spin_limit;      /* polls a device-side wait on a copy may take before it gives up with
                                  BD_ERR_TIMEOUT; 0 = the default (about 2^22, seconds) */
@@ -215,7 +215,8 @@ typedef struct bd_decode_args {
      * (rotary_positions, rotary_dim / 2) in q's dtype, contiguous.  The first rotary_dim dims of every
      * head are rotated, in fp32, pairs (2i, 2i+1) when interleaved, else (i, i + rotary_dim/2):
      * x0' = x0 cos - x1 sin, x1' = x0 sin + x1 cos.  rotary_dim: a multiple of 16, at most d; 0: none.
-     * One small kernel in front of the decode kernel; its rotated copies live in the workspace. */
+     * Done where the decode kernel loads them in steps with little work (and tables aligned to 16 bytes), else by one small
+     * kernel in front of it, whose rotated copies live in the workspace. */
     const void *rotary_cos, *rotary_sin;
     int32_t rotary_dim;
     int32_t rotary_interleaved;
