@@ -136,6 +136,11 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
     const uint32_t prm = smem_base + C::OFF_PRM + warp * STAGES * 2 * PRM;               // and their scales and zeros
     const uint32_t bars = smem_base + C::OFF_BAR + warp * STAGES * 16;
 
+    if ((smem_base & 1023u) != 0) {                      // never seen (the swizzled tiles need it); refuse rather than read garbage
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (tid == 0) atomicExch(p.status, BD_ERR_ALIGNMENT);
+        return;
+    }
     if (lane == 0) {
         for (int i = 0; i < 2 * STAGES; ++i) mbar_init(bars + 8 * i, 1);
         if (warp == 0) *abort_flag = 0;
