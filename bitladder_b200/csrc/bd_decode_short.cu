@@ -68,50 +68,109 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
 __device__ __forceinline__ float ldsf(uint32_t addr) { return __uint_as_float(lds32(addr)); }
 __device__ __forceinline__ void stsf(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
 
-// Dims c0 .. c0 + 7 of a head's row `x` rotated at table row `pos` (bd_rope.cu's arithmetic, rounded to the input type).
+__device__ __forceinline__ float half_value(uint32_t w, int hi, bool bf16) {
+    const uint16_t h = uint16_t(hi ? w >> 16 : w);
+    return bf16 ? __uint_as_float(uint32_t(h) << 16) : __half2float(__ushort_as_half(h));
+}
+__device__ __forceinline__ uint32_t half_pair(float lo, float hi, bool bf16) {
+    if (bf16) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+        return *reinterpret_cast<const uint32_t *>(&v);
+    }
+    return pack_f16x2(lo, hi);
+}
+// Dims c0 .. c0 + 7 of a head's row `x` rotated at table row `pos` (bd_rope.cu's arithmetic, rounded to the input type):
+// pairs half a rotary_dim apart, rotary_dim below 128 (the other kinds: Trig).
 __device__ __forceinline__ void rotate8(const DecodeParams &p, const uint16_t *x, int c0, int pos, bool bf16, uint32_t (&r)[4]) {
     if (c0 >= p.rotary_dim) return;
     const int half = p.rotary_dim / 2;
-    auto value = [&](uint32_t w, int hi) {
-        const uint16_t h = uint16_t(hi ? w >> 16 : w);
-        return bf16 ? __uint_as_float(uint32_t(h) << 16) : __half2float(__ushort_as_half(h));
-    };
-    auto pack = [&](float lo, float hi) {
-        if (bf16) {
-            const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-            return *reinterpret_cast<const uint32_t *>(&v);
-        }
-        return pack_f16x2(lo, hi);
-    };
+    auto value = [&](uint32_t w, int hi) { return half_value(w, hi, bf16); };
+    auto pack = [&](float lo, float hi) { return half_pair(lo, hi, bf16); };
     const uint16_t *cs = static_cast<const uint16_t *>(p.cos_tab) + int64_t(pos) * half;
     const uint16_t *sn = static_cast<const uint16_t *>(p.sin_tab) + int64_t(pos) * half;
-    if (p.rotary_interleaved) {
-        const uint2 c2 = *reinterpret_cast<const uint2 *>(cs + c0 / 2), s2 = *reinterpret_cast<const uint2 *>(sn + c0 / 2);
-        const uint32_t cw[2] = {c2.x, c2.y}, sw[2] = {s2.x, s2.y};
+    const bool low = c0 < half;
+    const int col = low ? c0 : c0 - half;
+    uint32_t o[4], cw[4], sw[4];
+    ldg128_pinned(x + (low ? c0 + half : c0 - half), o);
+    ldg128_pinned(cs + col, cw);
+    ldg128_pinned(sn + col, sw);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float c = value(cw[i >> 1], i & 1), s = value(sw[i >> 1], i & 1), x0 = value(r[i], 0), x1 = value(r[i], 1);
-            r[i] = pack(__fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s)), __fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c)));
+    for (int i = 0; i < 4; ++i) {
+        float y[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float c = value(cw[i], k), s = value(sw[i], k), a = value(r[i], k), b = value(o[i], k);
+            y[k] = low ? __fsub_rn(__fmul_rn(a, c), __fmul_rn(b, s)) : __fadd_rn(__fmul_rn(b, s), __fmul_rn(a, c));
         }
-    } else {
-        const bool low = c0 < half;
-        const int col = low ? c0 : c0 - half;
-        uint32_t o[4], cw[4], sw[4];
-        ldg128_pinned(x + (low ? c0 + half : c0 - half), o);
-        ldg128_pinned(cs + col, cw);
-        ldg128_pinned(sn + col, sw);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float y[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const float c = value(cw[i], k), s = value(sw[i], k), a = value(r[i], k), b = value(o[i], k);
-                y[k] = low ? __fsub_rn(__fmul_rn(a, c), __fmul_rn(b, s)) : __fadd_rn(__fmul_rn(b, s), __fmul_rn(a, c));
-            }
-            r[i] = pack(y[0], y[1]);
-        }
+        r[i] = pack(y[0], y[1]);
     }
 }
+
+// The table's words that this thread (dims 32 a + 8 l .. + 7) needs, all requested together: cosines, then sines.
+// (Each chunk's words behind the chunk before it cost a step of 8 sequences 1.9 us, of 2 2.2; together 1.0 and 0.8.)
+struct Trig {
+    uint32_t w[2][8];
+    bool near, far;               // pairs (2i, 2i + 1); pairs 64 apart; neither: rotate8
+    __device__ __forceinline__ void load(const DecodeParams &p, int pos, int l) {
+        near = p.rotary_interleaved != 0;
+        far = !near && p.rotary_dim == kHeadDim;
+        const int64_t row = int64_t(pos) * (p.rotary_dim / 2);
+        const uint16_t *tab[2] = {static_cast<const uint16_t *>(p.cos_tab) + row, static_cast<const uint16_t *>(p.sin_tab) + row};
+        if (near) {
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    const int c0 = 32 * a + 8 * l;
+                    const uint2 v = *reinterpret_cast<const uint2 *>(tab[t] + (c0 < p.rotary_dim ? c0 / 2 : 0));
+                    w[t][2 * a] = v.x;
+                    w[t][2 * a + 1] = v.y;
+                }
+        } else if (far) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    const uint4 v = *reinterpret_cast<const uint4 *>(tab[t] + 32 * i + 8 * l);
+                    w[t][4 * i] = v.x; w[t][4 * i + 1] = v.y; w[t][4 * i + 2] = v.z; w[t][4 * i + 3] = v.w;
+                }
+        }
+    }
+    // r[a]: the thread's dims of row x
+    __device__ __forceinline__ void rotate(const DecodeParams &p, const uint16_t *x, int pos, int l, bool bf16, uint32_t (&r)[4][4]) const {
+        if (near) {
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                if (32 * a + 8 * l >= p.rotary_dim) continue;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float c = half_value(w[0][2 * a + (i >> 1)], i & 1, bf16), s = half_value(w[1][2 * a + (i >> 1)], i & 1, bf16);
+                    const float x0 = half_value(r[a][i], 0, bf16), x1 = half_value(r[a][i], 1, bf16);
+                    r[a][i] = half_pair(__fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s)), __fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c)), bf16);
+                }
+            }
+        } else if (far) {
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float lo[2], hi[2];
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const float c = half_value(w[0][4 * a + i], k, bf16), s = half_value(w[1][4 * a + i], k, bf16);
+                        const float x0 = half_value(r[a][i], k, bf16), x1 = half_value(r[a + 2][i], k, bf16);
+                        lo[k] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
+                        hi[k] = __fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c));
+                    }
+                    r[a][i] = half_pair(lo[0], lo[1], bf16);
+                    r[a + 2][i] = half_pair(hi[0], hi[1], bf16);
+                }
+        } else {
+#pragma unroll
+            for (int a = 0; a < 4; ++a) rotate8(p, x, 32 * a + 8 * l, pos, bf16, r[a]);
+        }
+    }
+};
 
 }  // namespace
 
@@ -225,11 +284,16 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
         if (tid == 0 && rank == 0) atomicExch(p.status, BD_ERR_POSITION);
         pos = p.rotary_positions - 1;
     }
+    Trig trig;
+    if (p.rotary_dim > 0) {
+        trig.load(p, pos, l);
+#pragma unroll
+        for (int nq = 0; nq < NQT; ++nq) trig.rotate(p, qrow[nq], pos, l, bf16, qr[nq]);
+    }
 #pragma unroll
     for (int nq = 0; nq < NQT; ++nq)
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            if (p.rotary_dim > 0) rotate8(p, qrow[nq], 32 * a + 8 * l, pos, bf16, qr[nq][a]);
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
                 if (bf16) qr[nq][a][x] = bf16x2_to_f16x2(qr[nq][a][x]);
@@ -291,11 +355,8 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
             vb[i] = *reinterpret_cast<const unsigned int *>(vB + 8 * i + 2 * l);
         }
         if (p.rotary_dim > 0 && (newA || newB)) {
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                if (newA) rotate8(p, knew, 32 * a + 8 * l, pos, bf16, ka[a]);
-                if (newB) rotate8(p, knew, 32 * a + 8 * l, pos, bf16, kb[a]);
-            }
+            if (newA) trig.rotate(p, knew, pos, l, bf16, ka);
+            if (newB) trig.rotate(p, knew, pos, l, bf16, kb);
         }
         // fused append: the four threads that hold this step's token also store it into its row of the tail buffers
         if (res_n > res_old && (tA == res_old || tB == res_old)) {
