@@ -650,22 +650,17 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
         __threadfence();
         arrived = atomicAdd(roll.roll_arrivals + int64_t(ib) * p.h_k, 1);
     }
-    const bool room = cached >= 0 && cached % NB == 0 && cached + NB <= roll.roll_s_cap;
-    auto move_on = [&]() {                   // as bd_pack.cu does it behind the general kernel
+    // (the rule of bd_pack.cu's roll-over, for the lengths and for the block)
+    const bool room = cached >= 0 && cached % NB == 0 && cached <= roll.roll_s_cap - NB;
+    int left = min(max(in_tail, 0), roll.roll_res_cap);
+    if (left < roll.roll_res_cap) left += 1;
+    auto move_on = [&]() {
         if (arrived == p.h_k * ncta - 1) {
             __threadfence();
             roll.roll_arrivals[int64_t(ib) * p.h_k] = 0;
-            int r = min(max(in_tail, 0), roll.roll_res_cap);
-            if (r < roll.roll_res_cap) r += 1;
-            if (r == NB) {
-                if (room) {
-                    roll.roll_cache_seqlens[ib] = cached + NB;
-                    r = 0;
-                } else {
-                    atomicExch(roll.roll_status, BD_ERR_CAPACITY);
-                }
-            }
-            roll.roll_res_lens[ib] = r;
+            if (left == NB && room) roll.roll_cache_seqlens[ib] = cached + NB;
+            if (left == NB && !room) atomicExch(roll.roll_status, BD_ERR_CAPACITY);
+            roll.roll_res_lens[ib] = left == NB && room ? 0 : left;
         }
         __syncwarp();
     };
@@ -749,7 +744,7 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
     }
     if (roll.roll_res_lens != nullptr) {
         if (ncta == 1) move_on();
-        if (in_tail + 1 == NB && room) {
+        if (left == NB && room) {
             // (the token's own row, stored by one of the cluster's warps, is visible behind the barriers above)
             static_assert(PackCfg<BITS, GROUP>::NTHREADS == 128 && WARPS == 8, "two groups of threads pack");
             static_assert(sizeof(typename PackCfg<BITS, GROUP>::Shared) <= 16384 && C::OFF_PRM >= 32768, "in the warps' tiles");

@@ -29,8 +29,8 @@ struct PackParams {
     int32_t dst_token_offset;
     int32_t approx_div;           // divide like the reference built with --use_fast_math (see bd_pack.cu)
     // Roll-over of full tails (null: plain pack).  The source rows are a sequence's tail buffer; a
-    // sequence is packed only if roll_res_lens[ib] + 1 equals one pack block (this step's token filled
-    // the tail), into the block that starts at token roll_cache_seqlens[ib] (room permitting).
+    // sequence is packed only if its tail is one pack block behind this step (the step's token filled it, or it was
+    // full from the start), into the block that starts at token roll_cache_seqlens[ib] (room permitting).
     // The CTA of a sequence that has read its lengths last then moves them on.
     int32_t *roll_res_lens;
     int32_t *roll_cache_seqlens;

@@ -44,31 +44,24 @@ bd_pack_kernel(const PackParams p) {
             roll[1] = p.roll_cache_seqlens[ib];
         }
         __syncthreads();
-        const int tail = roll[0];
         dst_off = roll[1];
+        // The tail as this step leaves it: the decode kernel filed a token where there was room.  One rule for the block
+        // and for the lengths: a tail of one pack block, full from the start or filled now, is packed if there is room.
+        int left = min(max(roll[0], 0), p.roll_res_cap);
+        if (left < p.roll_res_cap) left += 1;
+        const bool room = dst_off >= 0 && dst_off % NB == 0 && dst_off <= p.roll_s_cap - NB;
         if (tid == 0) {
             int32_t *arrivals = p.roll_arrivals + static_cast<int64_t>(ib) * p.h_k;
             __threadfence();
             if (atomicAdd(arrivals, 1) == int(gridDim.x) - 1) {
                 __threadfence();
                 *arrivals = 0;
-                // Mirrors what the decode kernel did (a tail that was already full took no token) and what the CTAs
-                // of this one do (a tail that reached one pack block is packed, room permitting).
-                int r = min(max(tail, 0), p.roll_res_cap), cs = dst_off;
-                if (r < p.roll_res_cap) r += 1;
-                if (r == NB) {
-                    if (cs >= 0 && cs % NB == 0 && cs + NB <= p.roll_s_cap) {
-                        p.roll_cache_seqlens[ib] = cs + NB;
-                        r = 0;
-                    } else {
-                        atomicExch(p.roll_status, BD_ERR_CAPACITY);
-                    }
-                }
-                p.roll_res_lens[ib] = r;
+                if (left == NB && room) p.roll_cache_seqlens[ib] = dst_off + NB;
+                if (left == NB && !room) atomicExch(p.roll_status, BD_ERR_CAPACITY);
+                p.roll_res_lens[ib] = left == NB && room ? 0 : left;
             }
         }
-        if (tail + 1 != NB) return;
-        if (dst_off < 0 || dst_off % NB != 0 || dst_off + NB > p.roll_s_cap) return;   // no room: reported above
+        if (left != NB || !room) return;
     }
     if (p.fill_cache_seqlens != nullptr) {
         const int full = min(max(p.fill_cache_seqlens[ib], 0), min(p.s, p.fill_s_cap)) / NB;

@@ -200,7 +200,9 @@ typedef struct bd_decode_args {
                                  in its snapshot).  Needs cache_seqlens and res_lens (both are then WRITTEN), a tail
                                  buffer of at least NB rows, no block_table.  Done by the decode kernel itself in
                                  steps with little work, else by one small kernel behind it.  No room left for the block: BD_ERR_CAPACITY in
-                                 the status word, the tail stays full. */
+                                 the status word, the tail stays full.  A tail that is full before the step (after such an
+                                 error, in larger buffers) is packed all the same where there is room; this step's token,
+                                 which a full buffer has no row for, is then neither attended to nor filed. */
     uint32_t spin_limit;      /* polls a device-side wait on a copy may take before it gives up with
                                  BD_ERR_TIMEOUT; 0 = the default (about 2^22, seconds) */
     int32_t test_starve;      /* test hook, leave 0.  1: the warps of the first CTA expect 16 bytes more

@@ -149,5 +149,11 @@ def test_roll_over_leaves_the_same_bytes_as_the_general_kernels(bits, group, dty
         got.append(([t.view(torch.int16) for t in (*bufs, *tail)] + [cs, rl], out.float(), lse, step.status()))
     (a, oa, la, sa), (b, ob, lb, sb) = got
     assert all(torch.equal(s, t) for s, t in zip(a, b)) and sa == sb != 0
-    assert a[6].tolist()[:4] == [2 * block, block, 2 * block, cap]
+    assert a[6].tolist() == [2 * block, block, 2 * block, cap, 2 * block] and a[7].tolist() == [0, 0, block - 1, block, 0]
+    # a tail that was full from the start is packed as it is
+    want = [t.clone() for t in G.pack_gpu(B, x["k"], x["v"], bits, group)]
+    rows = [x[n][4:].cuda() for n in ("k_res", "v_res")]
+    B.kvcache_pack_int(rows[0], want[0][4:], want[1][4:], rows[1], want[2][4:], want[3][4:], None, None, block, *FMT(group, bits),
+                       dst_token_offset=block)
+    assert all(torch.equal(s[4], t.view(torch.int16)[4]) for s, t in zip(a, want))
     assert (oa - ob).abs().max() <= G.TOL_O[dtype] * max(1.0, float(ob.abs().max())) and (la - lb).abs().max() <= G.TOL_LSE[dtype]
