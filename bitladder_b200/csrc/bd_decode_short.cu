@@ -49,7 +49,7 @@ struct ShortCfg {
     static constexpr int FIT = (LIMIT - OFF_MERGE) / DEPOSIT;
     static constexpr int CLUSTER = FIT >= 8 ? 8 : (FIT >= 4 ? 4 : (FIT >= 2 ? 2 : 1));
     static constexpr int OFF_BAR = OFF_MERGE + CLUSTER * DEPOSIT;
-    static constexpr int SMEM = OFF_BAR + WARPS * STAGES * 16 + 16;               // barriers, abort flag
+    static constexpr int SMEM = OFF_BAR + WARPS * STAGES * 16;
     static_assert(DEPOSIT <= STAGES * 2 * CODE, "a warp's result fits its own tiles");
     static_assert(SMEM <= kSmemLimit, "shared memory");
 };
@@ -185,7 +185,6 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
 
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t smem_base = smem_u32(smem);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + C::OFF_BAR + WARPS * STAGES * 16);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int g = lane >> 2, l = lane & 3;
     // a cluster's CTAs are consecutive, and so are the heads of a sequence
@@ -202,7 +201,6 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
     }
     if (lane == 0) {
         for (int i = 0; i < 2 * STAGES; ++i) mbar_init(bars + 8 * i, 1);
-        if (warp == 0) *abort_flag = 0;
         fence_mbar_init();
         tma_prefetch_desc(&kmap);
         tma_prefetch_desc(&vmap);
@@ -425,6 +423,7 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
 
     // ---- half blocks ----
     int n = 0;
+    bool gave_up = false;                    // a wait of this warp ran out
 #pragma unroll 1
     for (int item = unit0; item < items; item += stride, ++n) {
         const int st = STAGES == 2 ? n & 1 : 0;
@@ -440,7 +439,7 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
             }
         }
         const bool need_mask = (blk + 1) * NB > seqlen_blk;
-        if (!copied(bars + 16 * st, par)) { *abort_flag = 1; break; }
+        if (!copied(bars + 16 * st, par)) { gave_up = true; break; }
 
         // q . zero per token group, two groups at a time: rows 0-7 the one, rows 8-15 the other
         float Zc[NGK][NQT][2];
@@ -548,7 +547,7 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
                 Pb[j][nq][1] = movmatrix_trans(pack_f16x2(t[j][2], t[j][3]));
             }
         }
-        if (!copied(bars + 16 * st + 8, par)) { *abort_flag = 1; break; }
+        if (!copied(bars + 16 * st + 8, par)) { gave_up = true; break; }
 #pragma unroll
         for (int j = 0; j < P; ++j) {
             const int r0 = 16 * u + 32 * j + 2 * l;               // tokens of fragment register 0
@@ -646,7 +645,7 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
             stsf(mine + ((32 * NQT + nq * 4 + 2 + c) * 32 + lane) * 4, sum);
         }
     }
-    __syncthreads();
+    const bool aborted = __syncthreads_or(gave_up);
     // The lengths move on when every CTA that works on the sequence has read them: each counts in, behind the barrier that
     // all of its warps have met at (a count per warp, each behind its own reads: a step of 8 sequences 11.05 -> 10.4 us, of 2
     // 13.1 -> 12.3), and the last one writes them where the others wait anyway.
@@ -771,7 +770,7 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
             }
         }
     }
-    if (*abort_flag != 0) {
+    if (aborted) {
         if (tid == 0) atomicExch(p.status, BD_ERR_TIMEOUT);
         // give copies that are still in flight time to land before the block's shared memory is released
         for (int it = 0; it < 2000; ++it) __nanosleep(1000);

@@ -57,6 +57,25 @@ def test_decode_step_object_reports_the_status_too():
     assert good.status() == 0
 
 
+@pytest.mark.parametrize("splits,limit", [(0, 1), (2, 2000), (6, 2000)])
+def test_every_step_whose_waits_run_out_says_so(splits, limit):
+    """In the short kernel also with a single poll, where warps give up while others of their CTA have just started: none of
+    their reports is lost.  (splits 2: the general kernel merges its parts; 6: a second kernel does.)"""
+    import bitladder_b200 as B
+    from bitladder_b200 import _lib
+    x = H.gen_qkv(2, 1024, 16, 4, seed=75)
+    bufs = G.pack_gpu(B, x["k"], x["v"], 4, 128)
+    args = (x["q"].cuda(), *bufs, None, H.default_scale(), "k-channel", 128, 4)
+    bad = B.DecodeStep(*args, num_splits=splits, spin_limit=limit, _test_starve=1)
+    assert bad.plan()["warps_per_cta"] == (12 if splits else 8)
+    for _ in range(50):
+        bad.step()
+        assert bad.status() == _lib.BD_ERR_TIMEOUT
+    step = B.DecodeStep(*args, num_splits=splits)
+    want = step.step(check=True).clone()
+    assert torch.equal(step.step(check=True), want)
+
+
 def test_a_page_index_outside_the_pool_is_masked_and_reported():
     """The last page of one sequence points outside the pool: its tokens are left out (the result
     equals the oracle over the sequence without that page), the status word says BD_ERR_PAGE, no
