@@ -746,6 +746,13 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
             else static_cast<float *>(p.out)[oi] = v;
         }
     }
+    if (aborted) {
+        if (tid == 0) atomicExch(p.status, BD_ERR_TIMEOUT);
+        // give copies that are still in flight time to land before a full tail is packed through the tiles, and before the
+        // block's shared memory is released
+        for (int it = 0; it < 2000; ++it) __nanosleep(1000);
+        __syncthreads();
+    }
     if (roll.roll_res_lens != nullptr) {
         if (ncta == 1) move_on();
         if (left == NB && room) {
@@ -769,12 +776,6 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
                 sync();
             }
         }
-    }
-    if (aborted) {
-        if (tid == 0) atomicExch(p.status, BD_ERR_TIMEOUT);
-        // give copies that are still in flight time to land before the block's shared memory is released
-        for (int it = 0; it < 2000; ++it) __nanosleep(1000);
-        __syncthreads();
     }
 }
 

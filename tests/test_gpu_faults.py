@@ -76,6 +76,31 @@ def test_every_step_whose_waits_run_out_says_so(splits, limit):
     assert torch.equal(step.step(check=True), want)
 
 
+@pytest.mark.parametrize("bits,group,h_k", [(4, 128, 2), (4, 32, 8), (2, 64, 2), (2, 128, 40)])
+@pytest.mark.parametrize("splits", [0, 2])
+def test_a_step_whose_wait_runs_out_packs_a_full_tail_as_any_other(bits, group, h_k, splits):
+    """The step reports the error; the block that its token completes and the lengths are those of a step without it."""
+    import bitladder_b200 as B
+    from bitladder_b200 import _lib
+    block = B.pack_block_tokens(bits)
+    x = H.gen_qkv(3, 3 * block, 2 * h_k, h_k, seed=76 + bits, res=block)
+    new = [x[n][:, -1:].cuda() for n in "kv"]
+    got = []
+    for starve in (0, 1):
+        bufs = G.pack_gpu(B, x["k"], x["v"], bits, group)
+        tail = [x["k_res"].cuda(), x["v_res"].cuda()]
+        cs, rl = (torch.tensor(t, dtype=torch.int32, device="cuda") for t in ([2 * block, block, 0], [block - 1, block - 1, 3]))
+        step = B.DecodeStep(x["q"].cuda(), *bufs, None, H.default_scale(), "k-channel", group, bits, k_res=tail[0], v_res=tail[1],
+                            cache_seqlens=cs, res_lens=rl, k_new=new[0], v_new=new[1], advance=True, num_splits=splits,
+                            spin_limit=2000 * starve, _test_starve=starve)
+        assert step.plan()["launches"] == (1 if splits == 0 else 2)
+        step.step()
+        assert step.status() == (_lib.BD_ERR_TIMEOUT if starve else 0)
+        got.append([t.view(torch.int16) for t in (*bufs, *tail)] + [cs, rl])
+    assert got[0][6].tolist() == [3 * block, 2 * block, 0] and got[0][7].tolist() == [0, 0, 4]
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 def test_a_page_index_outside_the_pool_is_masked_and_reported():
     """The last page of one sequence points outside the pool: its tokens are left out (the result
     equals the oracle over the sequence without that page), the status word says BD_ERR_PAGE, no
