@@ -534,7 +534,7 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     p.test_starve = a->test_starve;
     p.k_res = a->k_res; p.v_res = a->v_res;
     p.res_stride_b = a->res_stride_b; p.res_stride_s = a->res_stride_s; p.res_stride_h = a->res_stride_h;
-    p.res_lens = a->res_lens; p.res_len = a->k_res ? a->res_len : 0;
+    p.res_lens = a->k_res ? a->res_lens : nullptr; p.res_len = a->k_res ? a->res_len : 0;      // (without a tail neither is looked at)
     p.res_cap = p.res_len;
     p.k_res_out = const_cast<void *>(a->k_res); p.v_res_out = const_cast<void *>(a->v_res);
     p.k_new = a->k_new; p.v_new = a->v_new;
