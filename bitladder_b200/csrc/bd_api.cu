@@ -118,7 +118,9 @@ int plan_rows(int b, int h_k, int64_t max_s, int bits, int sm_count, int ctas_pe
 }
 
 // Whether a step has so little work that bd_decode_short.cu is the faster kernel, and the CTAs it then gives every
-// (sequence, KV head): as many (a power of two, up to eight) as fit the machine at once and find work for their warps.
+// (sequence, KV head): as many (a power of two, up to eight) as the device runs at once and find work for their warps.  (Not
+// as many as SMs would hold: of clusters of 8 a B200 runs 15 at once, of 4 33, of 2 74, and a 16th waits for the others,
+// 2 x 24576 tokens, 32/8 heads, 2 bits 21.0 -> 26.8 us.)
 // A round is an item (half a pack block, or 16 tail tokens) for every warp of a cluster.  General kernel -> short one, us a
 // step in a stream, by rounds:
 //   one sequence, 32/8 heads, 4 bits      2: 11.6 -> 8.2, 3: 12.1 -> 9.9, 4: 12.8 -> 11.6, 6: 15.0 -> 15.0, 8: 17.5 -> 18.3
@@ -138,7 +140,7 @@ int short_cluster(const bd_decode_args *a, int sm_count, int64_t nblk) {
     const bool ragged = a->cache_seqlens != nullptr || (a->k_res != nullptr && a->res_lens != nullptr);
     const int64_t items = 2 * nblk + (a->k_res ? (a->res_len + (a->k_new ? 1 : 0) + 15) / 16 : 0);
     int c = 1;
-    while (2 * c <= most && pairs * 2 * c <= sm_count && c * bd::kShortWarps < items) c *= 2;
+    while (2 * c <= most && c * bd::kShortWarps < items && pairs <= bd::decode_short_resident(a->bits, a->group, a->h / a->h_k, 2 * c)) c *= 2;
     const int64_t round = int64_t(c) * bd::kShortWarps;
     if (pairs > sm_count) return items <= 4 * round && (ragged || items >= round) ? c : 0;
     if (a->bits == 4 && !ragged && a->k_res == nullptr) return items < 4 * round ? c : 0;

@@ -16,6 +16,7 @@
 //    by the cluster that has just read it (bd_pack.cuh): one kernel a token.
 //
 // Measured against bd_decode.cu: see launch_decode_short's rule in bd_api.cu.
+#include <atomic>
 #include <type_traits>
 
 #include "bd_decode.cuh"
@@ -782,34 +783,65 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+// The launch of a step, but for grid and stream; `at` holds the attributes.
 template <int BITS, int GROUP, int NQT>
-static cudaError_t launch_short(const DecodeParams &p, const PackParams &roll, const CUtensorMap &kmap, const CUtensorMap &vmap, cudaStream_t stream) {
+static cudaError_t short_config(int cluster, cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&at)[2]) {
     using C = ShortCfg<BITS, GROUP, NQT>;
-    auto kern = bd_decode_short_kernel<BITS, GROUP, NQT>;
     static bool configured[64] = {};
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess) return err;
-    if (dev < 64 && !configured[dev]) {
-        err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(C::SMEM));
+    if (dev >= 64 || !configured[dev]) {
+        err = cudaFuncSetAttribute(bd_decode_short_kernel<BITS, GROUP, NQT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(C::SMEM));
         if (err != cudaSuccess) return err;
-        configured[dev] = true;
+        if (dev < 64) configured[dev] = true;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(p.b) * unsigned(p.h_k) * unsigned(p.cluster));
+    cfg = {};
     cfg.blockDim = dim3(C::THREADS);
     cfg.dynamicSmemBytes = C::SMEM;
-    cfg.stream = stream;
-    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = unsigned(p.cluster);
+    at[1].val.clusterDim.x = unsigned(cluster);
     at[1].val.clusterDim.y = 1;
     at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = p.cluster > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kern, p, roll, kmap, vmap);
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaSuccess;
+}
+
+template <int BITS, int GROUP, int NQT>
+static cudaError_t launch_short(const DecodeParams &p, const PackParams &roll, const CUtensorMap &kmap, const CUtensorMap &vmap, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[2];
+    cudaError_t err = short_config<BITS, GROUP, NQT>(p.cluster, cfg, at);
+    if (err != cudaSuccess) return err;
+    cfg.gridDim = dim3(unsigned(p.b) * unsigned(p.h_k) * unsigned(p.cluster));
+    cfg.stream = stream;
+    return cudaLaunchKernelEx(&cfg, bd_decode_short_kernel<BITS, GROUP, NQT>, p, roll, kmap, vmap);
+}
+
+// Clusters of a size that run at once: a cluster's CTAs take an SM each, all in one GPC, and the SMs that a GPC has beyond a
+// multiple of the size stay without one.  Asked once per device.
+template <int BITS, int GROUP, int NQT>
+static int resident_short(int cluster) {
+    static std::atomic<int> known[64][4] = {};           // one more than the answer for clusters of 1, 2, 4 and 8
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    std::atomic<int> *slot = dev < 64 ? &known[dev][cluster == 8 ? 3 : cluster / 2] : nullptr;
+    if (slot && *slot > 0) return *slot - 1;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    cudaError_t err = short_config<BITS, GROUP, NQT>(cluster, cfg, at);
+    cfg.gridDim = dim3(unsigned(cluster));
+    if (err == cudaSuccess) err = cudaOccupancyMaxActiveClusters(&n, bd_decode_short_kernel<BITS, GROUP, NQT>, &cfg);
+    if (err != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    if (slot) *slot = n + 1;
+    return n;
 }
 
 #define BD_SHORT_PICK(RESULT)                                                                           \
@@ -832,6 +864,12 @@ cudaError_t launch_decode_short(const DecodeParams &p, const PackParams &roll, c
 int decode_short_cluster(int bits, int group, int gq) {
 #define BD_SHORT_CLUSTER(B, G, Q) return ShortCfg<B, G, Q>::CLUSTER;
     BD_SHORT_PICK(BD_SHORT_CLUSTER)
+    return 0;
+}
+
+int decode_short_resident(int bits, int group, int gq, int cluster) {
+#define BD_SHORT_RESIDENT(B, G, Q) return resident_short<B, G, Q>(cluster);
+    BD_SHORT_PICK(BD_SHORT_RESIDENT)
     return 0;
 }
 

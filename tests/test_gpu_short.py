@@ -157,3 +157,33 @@ def test_roll_over_leaves_the_same_bytes_as_the_general_kernels(bits, group, dty
                        dst_token_offset=block)
     assert all(torch.equal(s[4], t.view(torch.int16)[4]) for s, t in zip(a, want))
     assert (oa - ob).abs().max() <= G.TOL_O[dtype] * max(1.0, float(ob.abs().max())) and (la - lb).abs().max() <= G.TOL_LSE[dtype]
+
+
+def _cluster(B, b, h, h_k, s, bits, group, tail=0, ragged=False, advance=False):
+    """CTAs per (sequence, KV head) of the short kernel that the step would run; 0: the general kernel."""
+    i32 = lambda n: torch.full((b,), n, dtype=torch.int32, device="cuda")
+    rows = lambda n, heads: torch.zeros(b, n, heads, 128, dtype=torch.float16, device="cuda")
+    block = B.pack_block_tokens(bits)
+    kw = dict(k_res=rows(tail, h_k), v_res=rows(tail, h_k)) if tail else {}
+    if ragged:
+        kw["cache_seqlens"] = i32(block)
+        if tail:
+            kw["res_lens"] = i32(1)
+    if advance:
+        kw.update(k_new=rows(1, h_k), v_new=rows(1, h_k), advance=True)
+    bufs = B.alloc_packed_cache(b, (s + block - 1) // block * block, h_k, 128, bits, group)
+    plan = B.DecodeStep(rows(1, h), *bufs, None, 0.1, *FMT(group, bits), seqlen_k=s, **kw).plan()
+    c = plan["rows"] // b
+    return c if plan["warps_per_cta"] == 8 and plan["launches"] == 1 and plan["rows"] == b * c and c in (1, 2, 4, 8) else 0
+
+
+@pytest.mark.parametrize("pairs,most", [(15, 8), (16, 4), (17, 4), (33, 4), (34, 2), (37, 2), (74, 2), (75, 1)])
+def test_clusters_are_no_larger_than_run_at_once(pairs, most):
+    """On a B200 15 clusters of 8 CTAs, 33 of 4 and 74 of 2; the results with those sizes are the general kernel's."""
+    import bitladder_b200 as B
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes of a device with 148 SMs")
+    assert _cluster(B, pairs, 4, 1, most * 1024, 4, 128, ragged=True) == most          # two rounds
+    x = H.gen_qkv(pairs, 512, 4, 1, seed=pairs)
+    lens = (torch.arange(pairs, dtype=torch.int32) * 97 % 513).cuda()
+    _both(B, x, G.pack_gpu(B, x["k"], x["v"], 4, 128), 128, 4, cache_seqlens=lens)
