@@ -121,30 +121,52 @@ int plan_rows(int b, int h_k, int64_t max_s, int bits, int sm_count, int ctas_pe
 // (sequence, KV head): as many (a power of two, up to eight) as the device runs at once and find work for their warps.  (Not
 // as many as SMs would hold: of clusters of 8 a B200 runs 15 at once, of 4 33, of 2 74, and a 16th waits for the others,
 // 2 x 24576 tokens, 32/8 heads, 2 bits 21.0 -> 26.8 us.)
-// A round is an item (half a pack block, or 16 tail tokens) for every warp of a cluster.  General kernel -> short one, us a
-// step in a stream, by rounds:
-//   one sequence, 32/8 heads, 4 bits      2: 11.6 -> 8.2, 3: 12.1 -> 9.9, 4: 12.8 -> 11.6, 6: 15.0 -> 15.0, 8: 17.5 -> 18.3
-//   8 sequences, ragged, tails            1.6: 12.1 -> 7.6, 2.6: 12.6 -> 9.3, 4.5: 15.0 -> 12.8, 6.4: 18.4 -> 16.2
-//   one sequence, 64/8 heads, 2 bits      2: 13.0 -> 8.0, 4: 15.1 -> 11.4, 6: 15.6 -> 14.9, 8: 16.5 -> 18.3
-//   3 sequences, 16/4 heads, 2 bits       4.9: 25.0 -> 21.8, ragged 19.8 -> 21.4
-//   30 sequences, 8/1 heads, group 32     1: 14.3 -> 7.5, 2: 14.8 -> 10.4, 4: 16.3 -> 16.3
-// and with twice as many pairs of sequence and KV head as SMs (two CTAs in turn on every SM; three in turn lose):
-//   32 sequences, 32/8 heads, 4 bits      0.3: 6.3 -> 7.7, 1: 10.7 -> 9.5, 2: 15.3 -> 13.1, 4: 22.4 -> 20.0
-//   8 sequences, 32/32 heads, ragged      0.8: 11.9 -> 9.4, 1.5: 11.8 -> 9.7, 4.8: 18.3 -> 17.2
-// Equal lengths without a tail at 4 bits stop short of four rounds, where the gain is small and DecodeStep.plan() has
-// always told the general kernel's geometry.
+//
+// A round is an item (half a pack block, or 16 tail tokens) for every warp of a cluster: the short kernel's time is 4 to 6 us
+// and 1.7 to 5.3 a round, by the format.  The general kernel spreads the work over all SMs and takes 12 to 20 us however
+// little there is, so the number of rounds up to which the short one wins falls with the share of the SMs that its clusters
+// take and with the time of a round.  General -> short, us a step in a stream (graph replay: the same order), by rounds:
+//   4 bits, group 128, clusters on 64 SMs         3: 12.8 -> 9.9, ragged 15.6 -> 10.7; 6: ragged 19.2 -> 15.9
+//   the same, 128 SMs                             3: 15.9 -> 9.3, 6: ragged 20.3 -> 14.8
+//   4 bits, group 128, one pair on 8 SMs          ragged 4: 1.26 times as fast; 5: 0.93
+//   4 bits, group 64, 80 SMs, ragged              5: 1.15 times as fast, 6: 0.98
+//   4 bits, group 32, ragged                      32 SMs 3: 15.4 -> 14.0, 4: 15.8 -> 16.8; 128 SMs 4: 18.9 -> 17.5
+//   2 bits, group 64                              32 SMs 3: 17.2 -> 15.3, 4: 15.0 -> 18.6; 128 SMs 6: 31.2 -> 26.1
+//   2 bits, group 128, 128 SMs, ragged            4: 19.6 -> 16.5, 6: 0.96 times as fast
+//   2 bits, group 32                              64 SMs ragged 3: 21.2 -> 18.5, equal 4: 19.3 -> 22.5; 128 SMs ragged 4: 0.98
+//   9 to 16 query heads per KV head, 16 SMs       4 bits, group 64 3: 1.12, 4: 0.96; 2 bits, group 128 2: 19.5 -> 15.9, 4: 19.7 -> 25.1
+// With more pairs than SMs (two CTAs in turn on an SM) it wins where lengths differ, 256 pairs, 4 bits 3: 19.9 -> 15.6, and
+// hardly or not where they are equal: 256 pairs of 32/32 heads 3: 16.9 -> 17.4, 160 pairs 4: 0.92.
+// A step that moves the lengths on saves its roll-over kernel as well, worth a round and more (8 x 2048 tokens 19.5 -> 11.8).
+// Equal lengths without a tail at 4 bits stop short of four rounds; they would win up to six (8 pairs on 64 SMs, 5: 1.20 times
+// as fast), which nobody has built on yet.
+constexpr signed char kShortRounds[2][2][3][3][2] = {
+    // by query tiles, 4 or 2 bits, group 128 / 64 / 32, SMs taken (below two fifths, below three quarters, above): {equal, ragged}
+    {{{{4, 4}, {6, 6}, {6, 6}}, {{3, 4}, {5, 5}, {6, 6}}, {{2, 3}, {3, 3}, {4, 4}}},
+     {{{2, 3}, {3, 3}, {6, 4}}, {{2, 3}, {3, 3}, {6, 4}}, {{2, 3}, {2, 3}, {4, 3}}}},
+    {{{{3, 3}, {4, 4}, {6, 6}}, {{3, 3}, {4, 4}, {6, 6}}, {{2, 3}, {3, 3}, {4, 4}}},
+     {{{2, 2}, {3, 3}, {6, 4}}, {{2, 2}, {3, 3}, {6, 4}}, {{0, 0}, {0, 0}, {0, 0}}}},
+};
 int short_cluster(const bd_decode_args *a, int sm_count, int64_t nblk) {
-    const int most = bd::decode_short_cluster(a->bits, a->group, a->h / a->h_k);
+    const int gq = a->h / a->h_k, most = bd::decode_short_cluster(a->bits, a->group, gq);
     const int64_t pairs = int64_t(a->b) * a->h_k;
     if (most == 0 || a->num_splits > 0 || pairs > 2 * int64_t(sm_count)) return 0;
     const bool ragged = a->cache_seqlens != nullptr || (a->k_res != nullptr && a->res_lens != nullptr);
     const int64_t items = 2 * nblk + (a->k_res ? (a->res_len + (a->k_new ? 1 : 0) + 15) / 16 : 0);
     int c = 1;
-    while (2 * c <= most && c * bd::kShortWarps < items && pairs <= bd::decode_short_resident(a->bits, a->group, a->h / a->h_k, 2 * c)) c *= 2;
-    const int64_t round = int64_t(c) * bd::kShortWarps;
-    if (pairs > sm_count) return items <= 4 * round && (ragged || items >= round) ? c : 0;
-    if (a->bits == 4 && !ragged && a->k_res == nullptr) return items < 4 * round ? c : 0;
-    return items <= (a->group == 32 || (a->bits == 2 && ragged) ? 4 : 6) * round ? c : 0;
+    while (2 * c <= most && c * bd::kShortWarps < items && pairs <= bd::decode_short_resident(a->bits, a->group, gq, 2 * c)) c *= 2;
+    const int64_t round = int64_t(c) * bd::kShortWarps, taken = pairs * c;
+    int rounds;
+    if (pairs > sm_count) {
+        if (!ragged) return 0;
+        rounds = (a->group == 32 ? 2 : 3) + (a->advance ? 1 : 0);
+    } else {
+        const int fill = 5 * taken < 2 * int64_t(sm_count) ? 0 : (4 * taken < 3 * int64_t(sm_count) ? 1 : 2);
+        rounds = kShortRounds[gq > 8][a->bits == 2][a->group == 128 ? 0 : (a->group == 64 ? 1 : 2)][fill][ragged];
+        if (a->advance && fill < 2) rounds = std::min(rounds + 1, 6);
+        if (a->bits == 4 && !ragged && a->k_res == nullptr) return items < std::min(4 * round, rounds * round + 1) ? c : 0;
+    }
+    return items <= rounds * round ? c : 0;
 }
 
 int make_plan(const bd_decode_args *a, int sm_count, DecodePlan &plan) {

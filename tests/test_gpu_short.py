@@ -187,3 +187,20 @@ def test_clusters_are_no_larger_than_run_at_once(pairs, most):
     x = H.gen_qkv(pairs, 512, 4, 1, seed=pairs)
     lens = (torch.arange(pairs, dtype=torch.int32) * 97 % 513).cuda()
     _both(B, x, G.pack_gpu(B, x["k"], x["v"], 4, 128), 128, 4, cache_seqlens=lens)
+
+
+# (sequences, query heads, KV heads, tokens, bits, group, tail, lengths per sequence): on either side of the rule's limits, which
+# lie lower where the clusters take few SMs and a round is long
+@pytest.mark.parametrize("little,shape", [
+    (True, (1, 32, 8, 4096, 4, 128, 0, False)), (True, (8, 32, 8, 2048, 4, 128, 128, True)), (True, (8, 32, 32, 2000, 2, 64, 64, True)),
+    (True, (1, 16, 1, 4096, 2, 64, 0, False)), (False, (1, 16, 1, 12288, 2, 64, 0, False)),
+    (False, (4, 64, 4, 24320, 4, 128, 64, False)), (False, (2, 32, 8, 49152, 2, 128, 0, False)),
+    (True, (1, 32, 8, 8192, 2, 64, 0, False)), (False, (1, 32, 8, 16384, 2, 64, 0, False)),
+    (True, (1, 32, 8, 5888, 4, 32, 64, True)), (False, (1, 32, 8, 7936, 4, 32, 64, True)),
+    (True, (8, 32, 32, 1024, 4, 128, 64, True)), (False, (8, 32, 32, 1536, 4, 32, 0, False)), (False, (20, 32, 8, 2048, 4, 128, 64, False))])
+def test_which_steps_are_little_work(little, shape):
+    import bitladder_b200 as B
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("limits of a device with 148 SMs")
+    b, h, h_k, s, bits, group, tail, ragged = shape
+    assert (_cluster(B, b, h, h_k, s, bits, group, tail, ragged) > 0) == little
