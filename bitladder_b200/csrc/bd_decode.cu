@@ -83,6 +83,11 @@ __device__ __forceinline__ unsigned trace_smid() {
 // one CTA and have the same age: with several CTAs per SM the scheduler favoured the
 // warps of the CTA that was launched first and the others finished up to 40 % later.
 constexpr int kMaxWarps = BD_MAX_WARPS;
+// Warps that a sequence's share of a CTA must have before all of them put it together (see FEW below).  Two or three deposits
+// are folded by one warp while the others would still be on their way to the meeting: 2 x 16384 tokens, 8/1 heads, two shares a
+// CTA, 11.3 us by one warp, 11.9 together; from 3, 5 or 8 shares on, 188 steps of few sequences took 0.959, 0.960 and 0.973 of the
+// one warp's time (median), the slowest of them 1.045, 1.022 and 1.039.
+constexpr int kTogether = 5;
 
 // TWO = 1: half as many warps per CTA and two CTAs per SM.  One CTA of twelve same-age warps per SM is
 // the faster arrangement wherever rows * KV heads fills the machine; with many KV heads (rows are tied
@@ -189,10 +194,12 @@ __device__ __forceinline__ void store_out(const DecodeParams &p, int64_t i, floa
 
 // RAGGED: per-sequence lengths are compiled in; a uniform batch has no table of units and runs without that code in
 // its start (b1, 4096 tokens: 10.7 us with it, 10.2 without; b8, 32768 tokens and a tail: 56.7, 56.2).
-// FEW: a step of few long sequences (DecodeParams::defer_merge is set): the warps of a CTA put its last sequence together
-// behind the loop, all of them, instead of the one that arrives last (b1, 32768 tokens 17.5 -> 16.2 us, 2 x 16384, 64/8
-// heads, group 64 18.2 -> 16.9).  Steps of many sequences would run that code and a single warp's, each once and so at
-// the speed of instruction fetch (b16 ragged and paged 25.6 -> 28.4 us), and both in one kernel cost the others registers.
+// FEW: a step of few long sequences (DecodeParams::defer_merge is set): where a CTA's range lies inside one sequence its warps
+// put that together behind the loop, all of them, instead of the one that arrives last (b1, 32768 tokens 17.5 -> 16.2 us,
+// 2 x 16384, 64/8 heads, group 64 18.2 -> 16.9).  A CTA with several sequences leaves them to single warps: with both codes,
+// each run once and so at the speed of instruction fetch, steps of few sequences were slower where ranges cross (9 x 5888
+// tokens, 16/4 heads 18.1 us by single warps, 18.8 with both; 40000 and 2500 tokens 23.9, 24.2, now 23.6), and so were steps of
+// many (b16 ragged and paged 25.6 -> 28.4), whose kernels do without.
 template <int BITS, int GROUP, int NQT, int TWO, bool RAGGED, bool FEW>
 __global__ void __launch_bounds__(Cfg<BITS, GROUP, NQT, TWO>::THREADS, Cfg<BITS, GROUP, NQT, TWO>::CTAS_PER_SM)
 bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
@@ -442,7 +449,9 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
             const uint32_t share_mask = __ballot_sync(0xffffffffu, shares);
             const uint32_t on_mask = __ballot_sync(0xffffffffu, shares && hi > seq_end);
             const int goes_on = on_mask ? 31 - __clz(on_mask) : -1;
-            const bool ends_cta = FEW && __shfl_sync(0xffffffffu, quo, kWarps) <= seq_end;      // the last sequence of the CTA's range
+            // the sequence takes all of the CTA's range, and enough of its warps have a share of it
+            const bool fills_cta = FEW && __popc(share_mask) >= kTogether && __shfl_sync(0xffffffffu, quo, 0) >= seq_first &&
+                                   __shfl_sync(0xffffffffu, quo, kWarps) <= seq_end;
             PartRange pr{0, -1, true};
             if (seq_n > 0 && Tw > 0) {
                 pr.c0 = int(__shfl_sync(0xffffffffu, quo, 16));
@@ -455,7 +464,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
                 for (int c = pr.c0; c <= pr.c1; ++c) nparts += row_has_part(part, ib, c) ? 1 : 0;
             }
             if (lane == 0)
-                *note = make_int4(int(share_mask), (goes_on + 1) | (ends_cta ? 128 : 0) | ((pr.c1 - pr.c0 + 1) << 8), pr.c0,
+                *note = make_int4(int(share_mask), (goes_on + 1) | (fills_cta ? 128 : 0) | ((pr.c1 - pr.c0 + 1) << 8), pr.c0,
                                   (nparts << 1) | (pr.dense ? 1 : 0));
             __syncwarp();
         }
@@ -945,7 +954,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
         const uint32_t share_mask = uint32_t(nt.x);
         const int goes_on = (nt.y & 127) - 1;
         const int nshare = __popc(share_mask);
-        // The last sequence of the CTA's range: nobody goes on, all of the CTA's warps put it together behind the loop.
+        // A sequence that takes all of the CTA's range: nobody goes on, all of the CTA's warps put it together behind the loop.
         const bool together = FEW && (nt.y & 128) && (nshare > 1 || (nt.w >> 1) > 1);
         if (together && warp == __ffs(share_mask) - 1 && lane == 0) {
             *last_note = nt;
@@ -1233,7 +1242,7 @@ bd_decode_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap kmap,
     }
 
     // ======================================================================
-    // after the stream: the CTA's last sequence, put together by all of its warps
+    // after the stream: the sequence that takes all of the CTA's range, put together by all of its warps
     // ======================================================================
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // a kernel staged behind this one may be placed
     __syncthreads();

@@ -236,6 +236,24 @@ def test_ragged_batches_at_the_table_limit(b, s, bits, splits):
     _check(x, ref, out, lse, bits, 128, "fp16", cs, rl, res=True)
 
 
+@pytest.mark.parametrize("bits,group", [(4, 128), (2, 64), (4, 32)])
+@pytest.mark.parametrize("blocks,extra", [((128,), 0), ((119, 7), 0), ((128, 0, 12), 5), ((3, 110, 1, 40), 17)])
+def test_few_sequences_cut_into_many_parts(bits, group, blocks, extra):
+    """More than four ranges per sequence, about seven blocks each: ranges that lie inside a sequence (put together by all of
+    the CTA's warps), ranges that several share, a sequence that is exactly one range, a short and an empty one, with tails."""
+    import bitladder_b200 as B
+    b, nb = len(blocks), B.pack_block_tokens(bits)
+    x = H.gen_qkv(b, max(blocks) * nb, 8, 2, seed=19, res=40)
+    ref = H.oracle_pack(x["k"], x["v"], bits, group, "fp16")
+    bufs = G.pack_gpu(B, x["k"], x["v"], bits, group)
+    cs = torch.tensor([max(0, n * nb - extra) for n in blocks], dtype=torch.int32)
+    rl = torch.tensor([(7 * i + extra) % 41 if extra else 0 for i in range(b)], dtype=torch.int32)
+    kw = dict(cache_seqlens=cs, k_res=x["k_res"], v_res=x["v_res"], res_lens=rl) if b > 1 else {}
+    splits = 18 // b if b > 1 else 18
+    out, lse = _run(B, x, bufs, bits, group, "fp16", num_splits=splits, **kw)
+    _check(x, ref, out, lse, bits, group, "fp16", cs if b > 1 else None, rl if b > 1 else None, res=b > 1)
+
+
 @pytest.mark.parametrize("group,dtype", [(128, "fp16"), (64, "bf16"), (32, "fp16")])
 @pytest.mark.parametrize("h", [18, 32])
 @pytest.mark.parametrize("ragged", [False, True])
