@@ -126,15 +126,17 @@ int plan_rows(int b, int h_k, int64_t max_s, int bits, int sm_count, int ctas_pe
 // and 1.7 to 5.3 a round, by the format.  The general kernel spreads the work over all SMs and takes 12 to 20 us however
 // little there is, so the number of rounds up to which the short one wins falls with the share of the SMs that its clusters
 // take and with the time of a round.  General -> short, us a step in a stream (graph replay: the same order), by rounds:
-//   4 bits, group 128, clusters on 64 SMs         3: 12.8 -> 9.9, ragged 15.6 -> 10.7; 6: ragged 19.2 -> 15.9
-//   the same, 128 SMs                             3: 15.9 -> 9.3, 6: ragged 20.3 -> 14.8
+//   4 bits, group 128, clusters on 64 SMs         3: 12.8 -> 9.9, ragged 15.6 -> 10.7; ragged 5: 18.4 -> 14.0
+//   the same, 128 SMs                             3: 15.9 -> 9.3, ragged 5: 17.1 -> 13.2
 //   4 bits, group 128, one pair on 8 SMs          ragged 4: 1.26 times as fast; 5: 0.93
 //   4 bits, group 64, 80 SMs, ragged              5: 1.15 times as fast, 6: 0.98
 //   4 bits, group 32, ragged                      32 SMs 3: 15.4 -> 14.0, 4: 15.8 -> 16.8; 128 SMs 4: 18.9 -> 17.5
 //   2 bits, group 64                              32 SMs 3: 17.2 -> 15.3, 4: 15.0 -> 18.6; 128 SMs 6: 31.2 -> 26.1
-//   2 bits, group 128, 128 SMs, ragged            4: 19.6 -> 16.5, 6: 0.96 times as fast
 //   2 bits, group 32                              64 SMs ragged 3: 21.2 -> 18.5, equal 4: 19.3 -> 22.5; 128 SMs ragged 4: 0.98
 //   9 to 16 query heads per KV head, 16 SMs       4 bits, group 64 3: 1.12, 4: 0.96; 2 bits, group 128 2: 19.5 -> 15.9, 4: 19.7 -> 25.1
+// Ragged lengths in these lines are spread evenly.  The general kernel shares out what there is, a cluster has its own
+// sequence: with one sequence of s tokens among others of s / 16 the limits lie lower.  4 bits, 4 sequences, 32/32 heads,
+// group 64 5: 13.9 -> 12.6, 6: 14.1 -> 14.5; group 32 4: 13.1 -> 15.5; 2 bits, group 128 4: 14.9 -> 16.6.
 // With more pairs than SMs (two CTAs in turn on an SM) it wins where lengths differ, 256 pairs, 4 bits 3: 19.9 -> 15.6, and
 // hardly or not where they are equal: 256 pairs of 32/32 heads 3: 16.9 -> 17.4, 160 pairs 4: 0.92.
 // A step that moves the lengths on saves its roll-over kernel as well, worth a round and more (8 x 2048 tokens 19.5 -> 11.8).
@@ -142,10 +144,10 @@ int plan_rows(int b, int h_k, int64_t max_s, int bits, int sm_count, int ctas_pe
 // as fast), which nobody has built on yet.
 constexpr signed char kShortRounds[2][2][3][3][2] = {
     // by query tiles, 4 or 2 bits, group 128 / 64 / 32, SMs taken (below two fifths, below three quarters, above): {equal, ragged}
-    {{{{4, 4}, {6, 6}, {6, 6}}, {{3, 4}, {5, 5}, {6, 6}}, {{2, 3}, {3, 3}, {4, 4}}},
-     {{{2, 3}, {3, 3}, {6, 4}}, {{2, 3}, {3, 3}, {6, 4}}, {{2, 3}, {2, 3}, {4, 3}}}},
-    {{{{3, 3}, {4, 4}, {6, 6}}, {{3, 3}, {4, 4}, {6, 6}}, {{2, 3}, {3, 3}, {4, 4}}},
-     {{{2, 2}, {3, 3}, {6, 4}}, {{2, 2}, {3, 3}, {6, 4}}, {{0, 0}, {0, 0}, {0, 0}}}},
+    {{{{4, 4}, {6, 5}, {6, 5}}, {{3, 4}, {5, 5}, {6, 5}}, {{2, 3}, {3, 3}, {4, 3}}},
+     {{{2, 3}, {3, 3}, {6, 3}}, {{2, 3}, {3, 3}, {6, 3}}, {{2, 3}, {2, 3}, {4, 3}}}},
+    {{{{3, 3}, {4, 4}, {6, 5}}, {{3, 3}, {4, 4}, {6, 5}}, {{2, 3}, {3, 3}, {4, 3}}},
+     {{{2, 2}, {3, 3}, {6, 3}}, {{2, 2}, {3, 3}, {6, 3}}, {{0, 0}, {0, 0}, {0, 0}}}},
 };
 int short_cluster(const bd_decode_args *a, int sm_count, int64_t nblk) {
     const int gq = a->h / a->h_k, most = bd::decode_short_cluster(a->bits, a->group, gq);
@@ -163,7 +165,7 @@ int short_cluster(const bd_decode_args *a, int sm_count, int64_t nblk) {
     } else {
         const int fill = 5 * taken < 2 * int64_t(sm_count) ? 0 : (4 * taken < 3 * int64_t(sm_count) ? 1 : 2);
         rounds = kShortRounds[gq > 8][a->bits == 2][a->group == 128 ? 0 : (a->group == 64 ? 1 : 2)][fill][ragged];
-        if (a->advance && fill < 2) rounds = std::min(rounds + 1, 6);
+        if (a->advance) rounds = std::min(rounds + 1, 6);
         if (a->bits == 4 && !ragged && a->k_res == nullptr) return items < std::min(4 * round, rounds * round + 1) ? c : 0;
     }
     return items <= rounds * round ? c : 0;
