@@ -38,8 +38,13 @@ def _check(x, ref, out, lse, bits, group, dtype, cs=None, rl=None, res=False):
     (2, 128, 320, 160, 512, 0),
     (4, 32, 32, 8, 2048, 0), (2, 32, 32, 8, 2048, 0), (4, 32, 64, 8, 1024, 2), (2, 32, 8, 8, 512, 0),   # group 32
 ])
-def test_decode_matches_oracle(bits, group, h, h_k, s, splits):
+@pytest.mark.parametrize("general", [False, True])
+def test_decode_matches_oracle(bits, group, h, h_k, s, splits, general):
+    """As the library chooses, and in the general kernel, which steps as small as these would not take by themselves."""
     import bitladder_b200 as B
+    if general and splits:
+        pytest.skip("the general kernel either way")
+    splits = splits or 2 * general
     x = H.gen_qkv(2, s, h, h_k, seed=5)
     ref = H.oracle_pack(x["k"], x["v"], bits, group, "fp16")
     bufs = G.pack_gpu(B, x["k"], x["v"], bits, group)
@@ -56,9 +61,10 @@ def test_decode_matches_oracle(bits, group, h, h_k, s, splits):
     (4, 64, "fp16", 16, 1, 4096, 256, True),
     (4, 128, "fp16", 8, 8, 256, 1, True),
     (4, 32, "fp16", 32, 8, 1024, 100, True),
-    (2, 32, "bf16", 16, 2, 1024, 33, True),
+    (2, 32, "bf16", 16, 2, 1024, 33, True), (2, 32, "fp16", 18, 2, 1024, 33, True), (2, 64, "bf16", 32, 2, 1024, 33, True),
 ])
-def test_decode_tail_and_ragged(bits, group, dtype, h, h_k, s, res, ragged):
+@pytest.mark.parametrize("splits", [0, 2])
+def test_decode_tail_and_ragged(bits, group, dtype, h, h_k, s, res, ragged, splits):
     import bitladder_b200 as B
     b = 5
     x = H.gen_qkv(b, s, h, h_k, seed=9, dtype=dtype, res=res)
@@ -73,7 +79,7 @@ def test_decode_tail_and_ragged(bits, group, dtype, h, h_k, s, res, ragged):
         rl = torch.randint(0, res + 1, (b,), generator=g, dtype=torch.int32)
         rl[0], rl[2] = res, 0
         kw.update(cache_seqlens=cs, res_lens=rl)
-    out, lse = _run(B, x, bufs, bits, group, dtype, **kw)
+    out, lse = _run(B, x, bufs, bits, group, dtype, num_splits=splits, **kw)
     _check(x, ref, out, lse, bits, group, dtype, cs, rl, res=True)
 
 
@@ -122,7 +128,8 @@ def test_config5_gqa8_long():
         _check(x, ref, out, lse, bits, 128, "fp16")
 
 
-def test_empty_and_degenerate_sequences():
+@pytest.mark.parametrize("splits", [0, 2])
+def test_empty_and_degenerate_sequences(splits):
     """No tokens at all gives out = 0 and lse = -inf; one valid token gives that token's V row."""
     import bitladder_b200 as B
     x = H.gen_qkv(3, 256, 8, 2, seed=21, res=4)
@@ -130,7 +137,7 @@ def test_empty_and_degenerate_sequences():
     bufs = G.pack_gpu(B, x["k"], x["v"], 4, 128)
     cs = torch.tensor([0, 1, 256], dtype=torch.int32)
     rl = torch.tensor([0, 0, 4], dtype=torch.int32)
-    out, lse = _run(B, x, bufs, 4, 128, "fp16", cache_seqlens=cs, res_lens=rl, k_res=x["k_res"], v_res=x["v_res"])
+    out, lse = _run(B, x, bufs, 4, 128, "fp16", cache_seqlens=cs, res_lens=rl, k_res=x["k_res"], v_res=x["v_res"], num_splits=splits)
     assert torch.all(out[0] == 0) and torch.all(torch.isinf(lse[0])) and torch.all(lse[0] < 0)
     _check(x, ref, out, lse, 4, 128, "fp16", cs, rl, res=True)
 
@@ -150,16 +157,17 @@ def test_reference_call_convention_and_defaults():
     assert mae < 4e-3, mae                       # the reference records 0.002773 for this shape
 
 
-def test_outputs_fp32_lse_and_caller_buffers():
+@pytest.mark.parametrize("splits", [0, 2])
+def test_outputs_fp32_lse_and_caller_buffers(splits):
     import bitladder_b200 as B
     x = H.gen_qkv(2, 1024, 32, 8, seed=31)
     ref = H.oracle_pack(x["k"], x["v"], 4, 128, "fp16")
     bufs = G.pack_gpu(B, x["k"], x["v"], 4, 128)
     q = x["q"].cuda()
     out32 = torch.empty(q.shape, dtype=torch.float32, device="cuda")
-    ws = torch.zeros(B.decode_workspace_bytes(q, *bufs), dtype=torch.uint8, device="cuda")
+    ws = torch.zeros(B.decode_workspace_bytes(q, *bufs, num_splits=splits), dtype=torch.uint8, device="cuda")
     o, lse = B.fwd_kvcache_int(q, *bufs, None, H.default_scale(), "k-channel", 128, 4, out=out32, workspace=ws,
-                               return_lse=True)
+                               return_lse=True, num_splits=splits)
     assert o.data_ptr() == out32.data_ptr()
     _check(x, ref, o, lse, 4, 128, "fp16")
     from bitladder_b200 import _lib
@@ -185,13 +193,14 @@ def test_combine_partials_equals_single_pass():
     assert (lse - full_lse).abs().max().item() <= 1e-3
 
 
-def test_two_calls_return_the_same_bits():
+@pytest.mark.parametrize("splits", [0, 2, 6])
+def test_two_calls_return_the_same_bits(splits):
     """Every warp streams a fixed share and every merge runs in a fixed order, so a repeated
     call (same inputs, same workspace state) must reproduce the result bit for bit."""
     import bitladder_b200 as B
     x = H.gen_qkv(3, 8192, 32, 8, seed=13, res=40)
     bufs = G.pack_gpu(B, x["k"], x["v"], 4, 128)
-    kw = dict(k_res=x["k_res"].cuda(), v_res=x["v_res"].cuda(), return_lse=True)
+    kw = dict(k_res=x["k_res"].cuda(), v_res=x["v_res"].cuda(), return_lse=True, num_splits=splits)
     args = (x["q"].cuda(), *bufs, None, H.default_scale(), "k-channel", 128, 4)
     o1, l1 = B.fwd_kvcache_int(*args, **kw)
     for _ in range(3):
@@ -199,12 +208,12 @@ def test_two_calls_return_the_same_bits():
         assert torch.equal(o1, o2) and torch.equal(l1, l2)
 
 
-@pytest.mark.parametrize("bits,dtype", [(4, "fp16"), (2, "fp16")])
-def test_many_short_ragged_sequences(bits, dtype):
-    """More sequences than CTA rows: every warp's range crosses several sequence boundaries, some
-    sequences are empty, some have only a tail, most are finished by a single warp."""
+@pytest.mark.parametrize("bits,s,dtype", [(4, 512, "fp16"), (2, 512, "fp16"), (4, 2048, "fp16"), (2, 4096, "fp16")])
+def test_many_short_ragged_sequences(bits, s, dtype):
+    """More sequences than the general kernel has CTA rows (37; the longer ones run in it): ranges cross several sequence
+    boundaries, some sequences are empty, some have only a tail, most are finished by a single warp."""
     import bitladder_b200 as B
-    b, s, h, h_k, res = 67, 512, 16, 4, 24
+    b, h, h_k, res = 67, 16, 4, 24
     x = H.gen_qkv(b, s, h, h_k, seed=77, dtype=dtype, res=res)
     ref = H.oracle_pack(x["k"], x["v"], bits, 128, dtype)
     bufs = G.pack_gpu(B, x["k"], x["v"], bits, 128)
@@ -219,7 +228,8 @@ def test_many_short_ragged_sequences(bits, dtype):
     _check(x, ref, out, lse, bits, 128, dtype, cs, rl, res=True)
 
 
-@pytest.mark.parametrize("b,s,bits,splits", [(1, 4096, 4, 0), (2, 4096, 2, 0), (31, 512, 4, 0), (32, 512, 4, 0), (31, 512, 2, 3)])
+@pytest.mark.parametrize("b,s,bits,splits", [(1, 4096, 4, 0), (2, 4096, 2, 0), (31, 512, 4, 0), (32, 512, 4, 0), (31, 512, 2, 3),
+                                             (1, 4096, 4, 4), (2, 4096, 2, 6), (31, 512, 4, 1), (32, 512, 4, 1), (32, 512, 2, 6)])
 def test_ragged_batches_at_the_table_limit(b, s, bits, splits):
     """Up to 31 sequences the kernels work the table of units out themselves (a lane per sequence and one for the
     total), with the parts merged in the decode kernel or, for few sequences, by the kernel behind it."""
@@ -257,14 +267,15 @@ def test_few_sequences_cut_into_many_parts(bits, group, blocks, extra):
 @pytest.mark.parametrize("group,dtype", [(128, "fp16"), (64, "bf16"), (32, "fp16")])
 @pytest.mark.parametrize("h", [18, 32])
 @pytest.mark.parametrize("ragged", [False, True])
-def test_two_query_tiles_at_four_bits(group, dtype, h, ragged):
+@pytest.mark.parametrize("splits", [0, 3])
+def test_two_query_tiles_at_four_bits(group, dtype, h, ragged, splits):
     """9 and 16 query heads per KV head: the kernels that form all fields of a slice ahead of its MMAs."""
     import bitladder_b200 as B
     x = H.gen_qkv(2, 1024, h, 2, seed=17, dtype=dtype)
     ref = H.oracle_pack(x["k"], x["v"], 4, group, dtype)
     bufs = G.pack_gpu(B, x["k"], x["v"], 4, group)
     cs = torch.tensor([1000, 129], dtype=torch.int32) if ragged else None
-    out, lse = _run(B, x, bufs, 4, group, dtype, **(dict(cache_seqlens=cs) if ragged else {}))
+    out, lse = _run(B, x, bufs, 4, group, dtype, num_splits=splits, **(dict(cache_seqlens=cs) if ragged else {}))
     _check(x, ref, out, lse, 4, group, dtype, cs)
 
 

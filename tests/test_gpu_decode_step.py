@@ -10,7 +10,8 @@ from tests import gpu_util as G, helpers as H
 pytestmark = pytest.mark.gpu
 
 
-def test_prepared_step_equals_the_plain_call_and_follows_content_changes():
+@pytest.mark.parametrize("splits", [0, 2])
+def test_prepared_step_equals_the_plain_call_and_follows_content_changes(splits):
     import bitladder_b200 as B
     x = H.gen_qkv(3, 2048, 32, 8, seed=17, res=32)
     bufs = G.pack_gpu(B, x["k"], x["v"], 4, 128)
@@ -20,10 +21,10 @@ def test_prepared_step_equals_the_plain_call_and_follows_content_changes():
     lens = torch.tensor([2048, 1000, 128], dtype=torch.int32, device="cuda")
     scale = 1.0 / math.sqrt(128)
     run = B.DecodeStep(q, *bufs, None, scale, "k-channel", 128, 4, k_res=k_res, v_res=v_res, res_lens=res_lens,
-                       cache_seqlens=lens, return_lse=True)
+                       cache_seqlens=lens, return_lse=True, num_splits=splits)
     for it in range(3):
         o_ref, l_ref = B.fwd_kvcache_int(q, *bufs, None, scale, "k-channel", 128, 4, k_res=k_res, v_res=v_res,
-                                         res_lens=res_lens, cache_seqlens=lens, return_lse=True)
+                                         res_lens=res_lens, cache_seqlens=lens, return_lse=True, num_splits=splits)
         o, l = run.step()
         assert torch.equal(o, o_ref) and torch.equal(l, l_ref)
         # new contents in the same buffers: the prepared step must see them
@@ -32,8 +33,9 @@ def test_prepared_step_equals_the_plain_call_and_follows_content_changes():
         lens.copy_(torch.tensor([1024, 2048 - 128 * it, 0], dtype=torch.int32))
 
 
-@pytest.mark.parametrize("b,s,rotary", [(1, 512, False), (2, 256, True), (3, 16384, False)])
-def test_captured_behind_copies_and_joined_streams(b, s, rotary):
+@pytest.mark.parametrize("b,s,rotary,splits", [(1, 512, False, 0), (2, 256, True, 0), (3, 16384, False, 0), (1, 512, False, 8),
+                                               (2, 256, True, 2)])
+def test_captured_behind_copies_and_joined_streams(b, s, rotary, splits):
     """The step's first kernel may be staged early behind what runs in front of it: in a graph that is a copy of the
     query, or the join of a side stream that writes it; in a stream, a kernel that has just written it."""
     import bitladder_b200 as B
@@ -46,7 +48,7 @@ def test_captured_behind_copies_and_joined_streams(b, s, rotary):
         kw = dict(k_res=x["k_res"], v_res=x["v_res"], k_new=x["k"][:, :1], v_new=x["v"][:, :1], rotary_cos=a.cos().half(),
                   rotary_sin=a.sin().half(), cache_seqlens=torch.full((b,), s, dtype=torch.int32, device="cuda"),
                   res_lens=torch.full((b,), 5, dtype=torch.int32, device="cuda"))
-    step = B.DecodeStep(q, *bufs, None, H.default_scale(), "k-channel", 128, 4, **kw)
+    step = B.DecodeStep(q, *bufs, None, H.default_scale(), "k-channel", 128, 4, num_splits=splits, **kw)
     q.copy_(x["q"])
     torch.cuda.synchronize()
     want = step.step().clone()

@@ -15,7 +15,10 @@ from tests import gpu_util as G, helpers as H
 pytestmark = pytest.mark.gpu
 
 
-def test_a_wait_that_runs_out_is_reported_and_the_workspace_is_reusable():
+# Small steps are the short kernel's; num_splits > 0 asks for the general one (2: it merges the parts itself and counts them;
+# 6: a second kernel merges them).
+@pytest.mark.parametrize("splits", [0, 2, 6])
+def test_a_wait_that_runs_out_is_reported_and_the_workspace_is_reusable(splits):
     """One warp of the first CTA expects 16 bytes more than its first copy delivers (test hook of the
     C-ABI), with a poll limit of 2000: the warp gives up after microseconds, keeps counting in so that
     every sequence still finds its last arrival, and the kernel returns with BD_ERR_TIMEOUT in the
@@ -26,8 +29,10 @@ def test_a_wait_that_runs_out_is_reported_and_the_workspace_is_reusable():
     ref = H.oracle_pack(x["k"], x["v"], 4, 128, "fp16")
     bufs = G.pack_gpu(B, x["k"], x["v"], 4, 128)
     q = x["q"].cuda()
-    kw = dict(k_res=x["k_res"].cuda(), v_res=x["v_res"].cuda())
+    kw = dict(k_res=x["k_res"].cuda(), v_res=x["v_res"].cuda(), num_splits=splits)
     need = B.decode_workspace_bytes(q, *bufs, **kw)
+    plan = B.DecodeStep(q, *bufs, None, H.default_scale(), "k-channel", 128, 4, **kw).plan()
+    assert plan["warps_per_cta"] == (12 if splits else 8) and plan["launches"] == (2 if splits == 6 else 1)
     ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
     args = (q, *bufs, None, H.default_scale(), "k-channel", 128, 4)
     B.fwd_kvcache_int(*args, workspace=ws, spin_limit=2000, _test_starve=1, **kw)
@@ -44,15 +49,16 @@ def test_a_wait_that_runs_out_is_reported_and_the_workspace_is_reusable():
     assert eo <= 2e-3 and el <= 2e-3
 
 
-def test_decode_step_object_reports_the_status_too():
+@pytest.mark.parametrize("splits", [0, 2])
+def test_decode_step_object_reports_the_status_too(splits):
     import bitladder_b200 as B
     x = H.gen_qkv(2, 2048, 16, 4, seed=72)
     bufs = G.pack_gpu(B, x["k"], x["v"], 4, 128)
     bad = B.DecodeStep(x["q"].cuda(), *bufs, None, H.default_scale(), "k-channel", 128, 4, spin_limit=2000,
-                       _test_starve=1)
+                       _test_starve=1, num_splits=splits)
     with pytest.raises(RuntimeError, match="wait"):
         bad.step(check=True)
-    good = B.DecodeStep(x["q"].cuda(), *bufs, None, H.default_scale(), "k-channel", 128, 4)
+    good = B.DecodeStep(x["q"].cuda(), *bufs, None, H.default_scale(), "k-channel", 128, 4, num_splits=splits)
     good.step(check=True)
     assert good.status() == 0
 
@@ -101,7 +107,8 @@ def test_a_step_whose_wait_runs_out_packs_a_full_tail_as_any_other(bits, group, 
     assert all(torch.equal(a, b) for a, b in zip(*got))
 
 
-def test_a_page_index_outside_the_pool_is_masked_and_reported():
+@pytest.mark.parametrize("splits", [0, 2, 6])
+def test_a_page_index_outside_the_pool_is_masked_and_reported(splits):
     """The last page of one sequence points outside the pool: its tokens are left out (the result
     equals the oracle over the sequence without that page), the status word says BD_ERR_PAGE, no
     address is formed from the bad index."""
@@ -122,9 +129,10 @@ def test_a_page_index_outside_the_pool_is_masked_and_reported():
         t2 = table.clone()
         t2[1, pages_per_seq - 1] = bad
         q = x["q"].cuda()
-        ws = torch.zeros(B.decode_workspace_bytes(q, *bufs, block_table=t2.cuda()), dtype=torch.uint8, device="cuda")
+        ws = torch.zeros(B.decode_workspace_bytes(q, *bufs, block_table=t2.cuda(), num_splits=splits), dtype=torch.uint8,
+                         device="cuda")
         out, lse = B.fwd_kvcache_int(q, *bufs, t2.cuda(), H.default_scale(), "k-channel", 128, 4, return_lse=True,
-                                     workspace=ws)
+                                     workspace=ws, num_splits=splits)
         rc = _lib.load().bd_read_status(ws.data_ptr(), torch.cuda.current_stream().cuda_stream)
         assert rc == _lib.BD_ERR_PAGE
         lens = np.array([s, s - page], dtype=np.int32)
@@ -133,7 +141,8 @@ def test_a_page_index_outside_the_pool_is_masked_and_reported():
         assert eo <= 2e-3 and el <= 2e-3
 
 
-def test_tail_lengths_beyond_the_buffers_are_clamped():
+@pytest.mark.parametrize("splits", [0, 2])
+def test_tail_lengths_beyond_the_buffers_are_clamped(splits):
     """res_lens[ib] larger than the rows the tail buffers hold: the kernel reads the rows there are."""
     import bitladder_b200 as B
     x = H.gen_qkv(3, 512, 8, 2, seed=74, res=40)
@@ -141,7 +150,8 @@ def test_tail_lengths_beyond_the_buffers_are_clamped():
     bufs = G.pack_gpu(B, x["k"], x["v"], 4, 128)
     rl = torch.tensor([40, 1000, 200], dtype=torch.int32)
     out, lse = B.fwd_kvcache_int(x["q"].cuda(), *bufs, None, H.default_scale(), "k-channel", 128, 4, return_lse=True,
-                                 k_res=x["k_res"].cuda(), v_res=x["v_res"].cuda(), res_lens=rl.cuda(), check=True)
+                                 k_res=x["k_res"].cuda(), v_res=x["v_res"].cuda(), res_lens=rl.cuda(), check=True,
+                                 num_splits=splits)
     o_ref, l_ref = H.oracle_decode(x["q"], ref, H.default_scale(), 4, 128, "fp16", k_res=x["k_res"], v_res=x["v_res"],
                                    res_lens=np.array([40, 40, 40], dtype=np.int32))
     eo, el = G.errs(out, lse, o_ref, l_ref)

@@ -10,8 +10,9 @@ from tests import gpu_util as G, helpers as H
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("splits", [0, 2])
 @pytest.mark.parametrize("name", sorted(H.load_golden()))
-def test_golden_fixture(name):
+def test_golden_fixture(name, splits):
     import bitladder_b200 as B
     case = H.load_golden()[name]
     cfg = case["cfg"]
@@ -27,7 +28,7 @@ def test_golden_fixture(name):
     if "res_lens" in case:
         kw["res_lens"] = torch.from_numpy(case["res_lens"]).cuda()
     out, lse = B.fwd_kvcache_int(q.cuda(), *bufs, None, 1.0 / math.sqrt(128), "k-channel", cfg["group"], cfg["bits"],
-                                 return_lse=True, **kw)
+                                 return_lse=True, num_splits=splits, **kw)
     eo, el = G.errs(out, lse, case["out"].astype(np.float64), case["lse"].astype(np.float64))
     tol = G.tol_o(cfg["dtype"], case["out"])
     assert eo <= tol and el <= 2 * tol, (name, eo, el, tol)

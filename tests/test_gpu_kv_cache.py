@@ -29,10 +29,11 @@ def _oracle_step(hist_k, hist_v, q, packed_lens, tail_lens, bits, group, dtype):
     return out
 
 
-@pytest.mark.parametrize("fused", [False, True])
+# (splits 0: one kernel a step; 2: the general kernel and the roll-over kernel behind it)
+@pytest.mark.parametrize("fused,splits", [(False, 0), (True, 0), (True, 2)])
 @pytest.mark.parametrize("bits,group,dtype,prompt", [(4, 128, "fp16", [200, 130]), (2, 128, "bf16", [300, 512]),
                                                       (4, 64, "fp16", [0, 127])])
-def test_cache_grows_across_block_boundaries(bits, group, dtype, prompt, fused):
+def test_cache_grows_across_block_boundaries(bits, group, dtype, prompt, fused, splits):
     """fused=False: append (copies) then decode; fused=True: one launch per step that attends over the
     new token and stores it in the tail (`append_and_decode`)."""
     from bitladder_b200.kv_cache import PackedKVCache
@@ -60,7 +61,7 @@ def test_cache_grows_across_block_boundaries(bits, group, dtype, prompt, fused):
         v_new = torch.randn(b, 1, h_k, 128, generator=g).to(tdt)
         q = torch.randn(b, 1, h, 128, generator=g).to(tdt)
         if fused:
-            out = cache.append_and_decode(q.cuda(), k_new.cuda(), v_new.cuda(), 1.0 / math.sqrt(128))
+            out = cache.append_and_decode(q.cuda(), k_new.cuda(), v_new.cuda(), 1.0 / math.sqrt(128), num_splits=splits)
         else:
             cache.append(k_new.cuda(), v_new.cuda())
         for ib in range(b):
@@ -99,8 +100,9 @@ def test_cache_rejects_bad_calls():
                       torch.zeros(2, 512, 2, 128, dtype=torch.float16, device="cuda"))
 
 
+@pytest.mark.parametrize("splits", [0, 2])
 @pytest.mark.parametrize("bits,group,dtype", [(4, 128, "fp16"), (2, 64, "bf16"), (4, 32, "fp16")])
-def test_decoder_step_as_a_cuda_graph_rolls_tails_over_on_the_device(bits, group, dtype):
+def test_decoder_step_as_a_cuda_graph_rolls_tails_over_on_the_device(bits, group, dtype, splits):
     """The whole decoder step (attend over the new token, file it, pack a tail that filled up, move the
     lengths on) captured ONCE in a CUDA graph and replayed for 300 tokens with fresh q / k_new / v_new in the
     same buffers: no host logic between steps.  Afterwards the lengths on the device are what the history
@@ -127,7 +129,8 @@ def test_decoder_step_as_a_cuda_graph_rolls_tails_over_on_the_device(bits, group
     q_buf = torch.zeros(b, 1, h, 128, dtype=tdt, device="cuda")
     k_buf = torch.zeros(b, 1, h_k, 128, dtype=tdt, device="cuda")
     v_buf = torch.zeros_like(k_buf)
-    step = cache.decoder_step(q_buf, k_buf, v_buf, 1.0 / math.sqrt(128))
+    step = cache.decoder_step(q_buf, k_buf, v_buf, 1.0 / math.sqrt(128), num_splits=splits)
+    assert step.plan()["launches"] == (2 if splits else 1)
     # warm up outside the capture on a clone of the state?  Not needed: the first launch is the capture's replay.
     graph = torch.cuda.CUDAGraph()
     side = torch.cuda.Stream()
@@ -169,7 +172,8 @@ def test_decoder_step_as_a_cuda_graph_rolls_tails_over_on_the_device(bits, group
         assert np.array_equal(H.f32_as_u16(cache.v_params[ib:ib + 1, :, :, :n]), ref["v_params"].view(np.uint16))
 
 
-def test_a_full_cache_is_reported_not_overrun():
+@pytest.mark.parametrize("splits", [0, 2])
+def test_a_full_cache_is_reported_not_overrun(splits):
     """advance with no room for the tail's block: the status word says so and nothing is written past the end."""
     import bitladder_b200 as B
     from bitladder_b200 import _lib
@@ -183,12 +187,12 @@ def test_a_full_cache_is_reported_not_overrun():
     cs = torch.tensor([nb], dtype=torch.int32, device="cuda")
     rl = torch.tensor([nb - 1], dtype=torch.int32, device="cuda")              # this step's token fills the tail
     q = x["q"].cuda()
-    ws = torch.zeros(B.decode_workspace_bytes(q, *bufs, k_res=k_tail, v_res=v_tail, res_lens=rl, cache_seqlens=cs),
+    ws = torch.zeros(B.decode_workspace_bytes(q, *bufs, k_res=k_tail, v_res=v_tail, res_lens=rl, cache_seqlens=cs, num_splits=splits),
                      dtype=torch.uint8, device="cuda")
     before = [t.clone() for t in bufs]
     B.fwd_kvcache_int(q, *bufs, None, H.default_scale(), "k-channel", 128, 4, k_res=k_tail, v_res=v_tail, res_lens=rl,
                       cache_seqlens=cs, k_new=x["k"][:, -1:].cuda(), v_new=x["v"][:, -1:].cuda(), advance=True,
-                      workspace=ws)
+                      workspace=ws, num_splits=splits)
     assert _lib.load().bd_read_status(ws.data_ptr(), torch.cuda.current_stream().cuda_stream) == _lib.BD_ERR_CAPACITY
     assert int(cs[0]) == nb and int(rl[0]) == nb                                # lengths: the tail stays full
     assert all(torch.equal(a, b_) for a, b_ in zip(before, bufs))

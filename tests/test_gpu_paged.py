@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("bits,group,page,dtype", [(4, 128, 256, "fp16"), (2, 128, 512, "fp16"), (4, 64, 256, "bf16")])
-def test_paged_pack_and_decode(bits, group, page, dtype):
+@pytest.mark.parametrize("splits", [0, 2, 6])
+def test_paged_pack_and_decode(bits, group, page, dtype, splits):
     import bitladder_b200 as B
 
     b, h, h_k, pages_per_seq = 3, 16, 4, 5
@@ -45,7 +46,7 @@ def test_paged_pack_and_decode(bits, group, page, dtype):
     res_lens = torch.tensor([48, 5, 0], dtype=torch.int32)
     out, lse = B.fwd_kvcache_int(x["q"].cuda(), *bufs, tab, H.default_scale(), "k-channel", group, bits,
                                  cache_seqlens=lens.cuda(), k_res=x["k_res"].cuda(), v_res=x["v_res"].cuda(),
-                                 res_lens=res_lens.cuda(), return_lse=True)
+                                 res_lens=res_lens.cuda(), return_lse=True, num_splits=splits)
     o_ref, l_ref = H.oracle_decode(x["q"], ref, H.default_scale(), bits, group, dtype, cache_seqlens=lens.numpy(),
                                    k_res=x["k_res"], v_res=x["v_res"], res_lens=res_lens.numpy())
     tol = 2e-3 if dtype == "fp16" else 1.6e-2

@@ -58,7 +58,8 @@ def _group_errors(o, ref, h_k):
 
 @pytest.mark.parametrize("name", ("mha_g128",) + H.REF_HASHED)
 @pytest.mark.parametrize("variant", ["ieee", "fast"])
-def test_decode_against_the_reference_decode_kernel(name, variant):
+@pytest.mark.parametrize("splits", [0, 2])
+def test_decode_against_the_reference_decode_kernel(name, variant, splits):
     """fwd_kvcache_int over the bytes the reference's pack kernel wrote, against the output of the
     reference's split-KV decode kernel on those bytes (fp16), per (sequence, KV head).
 
@@ -72,7 +73,7 @@ def test_decode_against_the_reference_decode_kernel(name, variant):
     cfg, blob = case["cfg"], case["blob"]
     bufs = _pack(B, case, fast=(variant == "fast"))
     out, lse = B.fwd_kvcache_int(case["q"].cuda(), *bufs, None, 1.0 / math.sqrt(128), "k-channel", cfg["group"], 4,
-                                 return_lse=True, check=True)
+                                 return_lse=True, check=True, num_splits=splits)
     o = out[:, 0].float().cpu().numpy().astype(np.float64)
     ref = blob[f"{name}/{variant}/out"].view(np.float16).astype(np.float64)[:, 0]
     err = _group_errors(o, ref, cfg["h_k"])

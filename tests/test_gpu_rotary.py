@@ -19,9 +19,11 @@ def _tables(positions, half, tdt, seed):
     return torch.cos(ang).to(tdt), torch.sin(ang).to(tdt)
 
 
+# (splits 0: the short kernel rotates; 2: the rotary kernel in front of the general one, the roll-over kernel behind it)
+@pytest.mark.parametrize("splits", [0, 2])
 @pytest.mark.parametrize("dtype,rotary_dim,interleaved,advance", [("fp16", 128, True, False), ("fp16", 64, False, True),
                                                                   ("bf16", 32, True, True), ("bf16", 128, False, False)])
-def test_step_with_rotary_equals_the_oracle_on_rotated_inputs(dtype, rotary_dim, interleaved, advance):
+def test_step_with_rotary_equals_the_oracle_on_rotated_inputs(dtype, rotary_dim, interleaved, advance, splits):
     import bitladder_b200 as B
     b, s, h, h_k, bits, group, res_cap = 3, 512, 8, 2, 4, 128, 128
     x = H.gen_qkv(b, s, h, h_k, seed=77, dtype=dtype, res=res_cap)
@@ -54,7 +56,8 @@ def test_step_with_rotary_equals_the_oracle_on_rotated_inputs(dtype, rotary_dim,
     cs, rl = torch.from_numpy(seqlens).cuda(), torch.from_numpy(res_lens).cuda()
     out = B.fwd_kvcache_int(x["q"].cuda(), *bufs, None, scale, "k-channel", group, bits, k_res=k_tail, v_res=v_tail,
                             res_lens=rl, cache_seqlens=cs, k_new=k_new.cuda(), v_new=v_new.cuda(), advance=advance,
-                            rotary_cos=cos.cuda(), rotary_sin=sin.cuda(), rotary_interleaved=interleaved, check=True)
+                            rotary_cos=cos.cuda(), rotary_sin=sin.cuda(), rotary_interleaved=interleaved, check=True,
+                            num_splits=splits)
     tol = G.TOL_O[dtype]
     assert np.abs(out[:, 0].float().cpu().numpy() - o_ref).max() <= tol
     for ib in range(b):          # the filed key is the oracle's rotated key, bit for bit; the value as it came
@@ -64,7 +67,8 @@ def test_step_with_rotary_equals_the_oracle_on_rotated_inputs(dtype, rotary_dim,
         assert rl.cpu().tolist() == (res_lens + 1).tolist()
 
 
-def test_a_position_beyond_the_tables_is_reported():
+@pytest.mark.parametrize("splits", [0, 2])
+def test_a_position_beyond_the_tables_is_reported(splits):
     import bitladder_b200 as B
     b, s, h, h_k = 1, 256, 4, 1
     x = H.gen_qkv(b, s, h, h_k, seed=78, res=64)
@@ -72,7 +76,7 @@ def test_a_position_beyond_the_tables_is_reported():
     cos, sin = _tables(100, 64, torch.float16, 4)            # tables of 100 positions, the token sits at 256 + 3
     rl = torch.tensor([3], dtype=torch.int32, device="cuda")
     kw = dict(k_res=x["k_res"].cuda(), v_res=x["v_res"].cuda(), res_lens=rl, k_new=x["k"][:, :1].cuda(),
-              v_new=x["v"][:, :1].cuda(), rotary_cos=cos.cuda(), rotary_sin=sin.cuda())
+              v_new=x["v"][:, :1].cuda(), rotary_cos=cos.cuda(), rotary_sin=sin.cuda(), num_splits=splits)
     with pytest.raises(RuntimeError, match="rotary"):
         B.fwd_kvcache_int(x["q"].cuda(), *bufs, None, 0.1, "k-channel", 128, 4, check=True, **kw)
     # and rotary without an appended token is refused on the host
@@ -81,7 +85,8 @@ def test_a_position_beyond_the_tables_is_reported():
         B.fwd_kvcache_int(x["q"].cuda(), *bufs, None, 0.1, "k-channel", 128, 4, **kw)
 
 
-def test_positions_follow_the_device_side_lengths_in_a_captured_decoder_loop():
+@pytest.mark.parametrize("splits", [0, 2])
+def test_positions_follow_the_device_side_lengths_in_a_captured_decoder_loop(splits):
     """A decoder step with rotary captured once as a CUDA graph and replayed: the position of every new token
     comes from the lengths the device itself advances, across a roll-over of the tail."""
     from bitladder_b200.kv_cache import PackedKVCache
@@ -94,7 +99,8 @@ def test_positions_follow_the_device_side_lengths_in_a_captured_decoder_loop():
     q = torch.zeros(b, 1, h, 128, dtype=torch.float16, device="cuda")
     kn = torch.zeros(b, 1, h_k, 128, dtype=torch.float16, device="cuda")
     vn = torch.zeros_like(kn)
-    step = cache.decoder_step(q, kn, vn, 0.1, rotary_cos=cos.cuda(), rotary_sin=sin.cuda(), rotary_interleaved=False)
+    step = cache.decoder_step(q, kn, vn, 0.1, rotary_cos=cos.cuda(), rotary_sin=sin.cuda(), rotary_interleaved=False,
+                              num_splits=splits)
     step.step()                                    # warm-up outside the capture, with zero rows: token 0
     torch.cuda.synchronize()
     gr = torch.cuda.CUDAGraph()
@@ -126,10 +132,12 @@ def test_positions_follow_the_device_side_lengths_in_a_captured_decoder_loop():
             assert np.array_equal(got.view(np.uint16), want[0].view(np.uint16)), (ib, r, pos)
 
 
+@pytest.mark.parametrize("splits", [0, 2, 6])
 @pytest.mark.parametrize("b,bits,h_k", [(1, 4, 8), (3, 2, 2), (40, 4, 2)])
-def test_steps_in_a_row_equal_steps_one_by_one(b, bits, h_k):
-    """Rotary, decode, merge and roll-over kernels overlap across steps in a stream: whatever an earlier step wrote (lengths,
-    a packed block, tail rows) has to be there, so the steps give the bits of steps that are waited for one by one."""
+def test_steps_in_a_row_equal_steps_one_by_one(b, bits, h_k, splits):
+    """The kernel of a step with little work (splits 0), and the rotary, prefix (40 sequences), decode, merge (splits 6) and
+    roll-over kernels of the general path, overlap across steps in a stream: whatever an earlier step wrote (lengths, a packed
+    block, tail rows) has to be there, so the steps give the bits of steps that are waited for one by one."""
     import bitladder_b200 as B
     nb, steps = B.pack_block_tokens(bits), 24
     s = 4 * nb
@@ -145,7 +153,9 @@ def test_steps_in_a_row_equal_steps_one_by_one(b, bits, h_k):
         now = [torch.empty_like(r[0]) for r in rows]
         tails, (cs, rl), outs = [x["k_res"].clone(), x["v_res"].clone()], [t.cuda() for t in lens], []
         step = B.DecodeStep(now[0], *bufs, None, H.default_scale(), "k-channel", 128, bits, k_res=tails[0], v_res=tails[1],
-                            res_lens=rl, cache_seqlens=cs, k_new=now[1], v_new=now[2], advance=True, rotary_cos=cos, rotary_sin=sin)
+                            res_lens=rl, cache_seqlens=cs, k_new=now[1], v_new=now[2], advance=True, rotary_cos=cos, rotary_sin=sin,
+                            num_splits=splits)
+        assert step.plan()["launches"] == (1 if splits == 0 else 3 + (b > 31) + (splits > 4))
         torch.cuda.synchronize()
         for i in range(steps):
             for t, r in zip(now, rows):

@@ -121,7 +121,8 @@ def test_noalloc_with_per_sequence_lengths():
     assert np.abs(o_na[:, 0] - o_ref).max() <= 2e-3
 
 
-def test_noalloc_keeps_an_error_code_until_it_is_read():
+@pytest.mark.parametrize("splits", [0, 2])      # the short kernel, the general one
+def test_noalloc_keeps_an_error_code_until_it_is_read(splits):
     """A step whose bounded wait runs out (test hook, poll limit 2000) leaves BD_ERR_TIMEOUT in the fixed
     area; the next call does not erase it; bd_read_status(NULL, stream) returns and clears it."""
     import bitladder_b200 as B
@@ -134,10 +135,10 @@ def test_noalloc_keeps_an_error_code_until_it_is_read():
     q = x["q"].cuda()
     out = torch.empty_like(q)
     stream = torch.cuda.current_stream().cuda_stream
-    a = I._decode_args(q, *bufs, 1.0 / math.sqrt(128), 128, 4, None, None, None, None, None, out, None, 0,
+    a = I._decode_args(q, *bufs, 1.0 / math.sqrt(128), 128, 4, None, None, None, None, None, out, None, splits,
                        spin_limit=2000, test_starve=1)
     assert lib.bd_decode_noalloc(C.byref(a), stream) == 0
-    a = I._decode_args(q, *bufs, 1.0 / math.sqrt(128), 128, 4, None, None, None, None, None, out, None, 0)
+    a = I._decode_args(q, *bufs, 1.0 / math.sqrt(128), 128, 4, None, None, None, None, None, out, None, splits)
     assert lib.bd_decode_noalloc(C.byref(a), stream) == 0
     assert lib.bd_read_status(None, stream) == _lib.BD_ERR_TIMEOUT
     assert lib.bd_read_status(None, stream) == 0
