@@ -33,8 +33,10 @@ bd_pack_kernel(const PackParams p) {
     // what it may write is never read through the non-coherent path (__ldg), which promises constant memory.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (p.roll_res_lens != nullptr) {          // roll-over: only sequences whose tail this step's token filled
-        // (the next step's kernel may be placed beside this short one; it waits for it before it reads anything)
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        // The next step's kernel may be placed beside this short one; it waits for it before it reads anything.  Few sequences
+        // gain in a graph (1 x 32768 tokens, group 64 25.4 -> 24.8 us a step, 8 x 8192 at 2 bits 26.0 -> 25.5) and lose nothing
+        // in a stream; many short ones lose (16 of up to 2560 tokens, most of 128, stream 18.0 -> 18.9 us, graph 17.3 -> 17.5).
+        if (p.b <= 8) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         // The lengths move only when all CTAs of the sequence have read them (the decode kernel in front is done with
         // them); a kernel of its own for that cost 0.4 us more per decoder step, and its launch.  One thread reads them
         // for its CTA, so that the fence in front of its count orders the CTA's only reads before the last one's writes.
