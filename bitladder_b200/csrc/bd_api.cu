@@ -584,9 +584,6 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     p.part_out = reinterpret_cast<float *>(ws + plan.off_part_out);
     p.part_lse = reinterpret_cast<float *>(ws + plan.off_part_lse);
 
-    // More than four parts per sequence on average (few long sequences cut over all SMs): one warp
-    // merging them at the end of the decode kernel would be the tail of the step; a second kernel
-    // with a warp per (sequence, query head) does it in parallel.
     if (a->rotary_dim > 0 && is_short && rotary_in_decode(a)) {
         p.cos_tab = a->rotary_cos; p.sin_tab = a->rotary_sin;
         p.rotary_dim = a->rotary_dim; p.rotary_interleaved = a->rotary_interleaved ? 1 : 0;
@@ -613,6 +610,9 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
         p.k_new = rp.k_out; p.v_new = rp.v_out; p.new_stride_b = int64_t(a->h_k) * 128; p.new_stride_h = 128;
     }
     p.early = early_decode ? 1 : 0;
+    // More than four parts per sequence on average (few long sequences cut over all SMs): one warp
+    // merging them at the end of the decode kernel would be the tail of the step; a second kernel
+    // with a warp per (sequence, query head) does it in parallel.
     p.defer_merge = (x || plan.rows > 4 * a->b) ? 1 : 0;
     p.leave_parts = x ? 1 : 0;
     p.two_ctas = plan.two_ctas;

@@ -40,11 +40,8 @@
 //
 // Steps with little work run in bd_decode_short.cu (the rule: short_cluster in bd_api.cu).
 //
-// tcgen05 was built and measured, and is not used.  With tokens (head dims) as its M = 128 rows the masked fragments
-// below go to tensor memory unchanged, and an MMA of 16 query columns takes 9 cycles; but the masks, which are what
-// dispatch is spent on, stay the same, every step of 128 tokens passes four warps through three meetings, and three
-// warpgroups per SM took 3250 cycles a step where HBM allows 2180: 16 x 131072 tokens 586 us against 421 at 4 bits, 511 against
-// 333 at 2.  (Eight-bit operands would halve the masks at 2 bits; they need q * scale and p * scale split into bytes.)
+// tcgen05 is not used: an MMA has 16 query columns here and costs little either way, while the masks, which are what dispatch
+// is spent on, stay the same for operands in tensor memory, and warps that work on one tile have to meet at every step.
 #include <type_traits>
 
 #include "bd_decode.cuh"

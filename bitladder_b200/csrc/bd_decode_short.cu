@@ -10,12 +10,12 @@
 //    unquantized tail, dealt out in turn over all warps of the cluster.
 //  * The warps' results are merged by all of them together: deposits in shared memory, a barrier, every warp an eighth of
 //    the output; then the CTAs' results the same way in the shared memory of the cluster's first CTA.  No second
-//    kernel, no counters, no trip to L2.
+//    kernel, no trip to L2.
 //  * With rotary embedding, q and the new key are rotated where they are loaded (bd_rope.cu's arithmetic).
-//  * A decoder step's bookkeeping is done here too: the lengths move on, and a tail that the step has filled is packed
-//    by the cluster that has just read it (bd_pack.cuh): one kernel a token.
+//  * A decoder step's bookkeeping is done here too: the lengths move on, and a tail that is full behind the step is
+//    packed by the cluster that has just read it (bd_pack.cuh): one kernel a token.
 //
-// Measured against bd_decode.cu: see launch_decode_short's rule in bd_api.cu.
+// Measured against bd_decode.cu, and the rule that chooses between them: short_cluster in bd_api.cu.
 #include <atomic>
 #include <type_traits>
 

@@ -283,7 +283,8 @@ int bd_plan_splits(int b, int h_k, int64_t max_s, int bits, int sm_count, int ct
  * out[2] = streaming warps per CTA, out[3] = kernels launched per call (prefix table of a large ragged
  * batch, rotary embedding, decode, parts merge, roll-over). A step with little work runs on clusters of
  * 1, 2, 4 or 8 CTAs of eight warps per (sequence, KV head), which merge, rotate and roll over by themselves: then out[0] = that
- * many ranges times the sequences, and there is one kernel to launch.  No counterpart in the reference (its grid is
+ * many ranges times the sequences, and there is one kernel to launch (two with rotary tables that do not start on 16 bytes).
+ * No counterpart in the reference (its grid is
  * (1, num_splits, b * h_k), csrc/bit_decode/src/flash_fwd_launch_template.h:110).
  */
 int bd_decode_plan(const bd_decode_args *args, int32_t out[4]);
