@@ -57,3 +57,13 @@ def test_a_wait_of_its_own_comes_before_what_earlier_kernels_wrote(path):
         body = re.sub(r"\{[^{}]*griddepcontrol\.wait[^{}]*return;\s*\}", "", body)          # a warp that leaves
         read = re.search(r"ragged_entry\(|part_range\(|(cache_seqlens|res_lens)\[", body)
         assert not read or body.index("griddepcontrol.wait") < read.start()
+
+
+def test_the_short_kernel_gives_up_as_one():
+    """What a wait that runs out leads to (nothing of it can be provoked on a GPU at will): the lanes of a warp agree, the
+    warps report through a barrier and not through a flag that another of them initialises, and copies in flight are given
+    time to land before a full tail is packed through the tiles they arrive in."""
+    code = "".join(_code(os.path.join(CSRC, "bd_decode_short.cu")))
+    assert re.findall(r"(\w+)\([^;]*mbar_wait_bounded\(", code) == ["__all_sync"]
+    assert "__syncthreads_or(gave_up)" in code and "abort_flag" not in code
+    assert code.index("__nanosleep(") < code.index("pack_k_part<")
