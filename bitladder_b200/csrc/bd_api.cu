@@ -134,38 +134,49 @@ int plan_rows(int b, int h_k, int64_t max_s, int bits, int sm_count, int ctas_pe
 //   2 bits, group 64                              32 SMs 3: 17.2 -> 15.3, 4: 15.0 -> 18.6; 128 SMs 6: 31.2 -> 26.1
 //   2 bits, group 32                              64 SMs ragged 3: 21.2 -> 18.5, equal 4: 19.3 -> 22.5; 128 SMs ragged 4: 0.98
 //   9 to 16 query heads per KV head, 16 SMs       4 bits, group 64 3: 1.12, 4: 0.96; 2 bits, group 128 2: 19.5 -> 15.9, 4: 19.7 -> 25.1
+//   2 bits, 80 to 96 SMs                          group 64 5: 1.19 times as fast, ragged 5: 0.90; group 128 5: 1.01 to 1.37
 // Ragged lengths in these lines are spread evenly.  The general kernel shares out what there is, a cluster has its own
-// sequence: with one sequence of s tokens among others of s / 16 the limits lie lower.  4 bits, 4 sequences, 32/32 heads,
-// group 64 5: 13.9 -> 12.6, 6: 14.1 -> 14.5; group 32 4: 13.1 -> 15.5; 2 bits, group 128 4: 14.9 -> 16.6.
-// With more pairs than SMs (two CTAs in turn on an SM) it wins where lengths differ, 256 pairs, 4 bits 3: 19.9 -> 15.6, and
-// hardly or not where they are equal: 256 pairs of 32/32 heads 3: 16.9 -> 17.4, 160 pairs 4: 0.92.
-// A step that moves the lengths on saves its roll-over kernel as well, worth a round and more (8 x 2048 tokens 19.5 -> 11.8).
+// sequence: with one sequence of s tokens among others of s / 16 the general kernel has the less to do the fewer they are, and
+// the limits of two to seven sequences lie a round lower.  4 sequences, 32/32 heads: 4 bits, group 64 5: 13.9 -> 12.6, 6: 14.1
+// -> 14.5; group 32 4: 13.1 -> 15.5; 2 bits, group 128 4: 14.9 -> 16.6; 8 sequences, 32/8 heads, group 64 6: 16.7 -> 16.1.  Of
+// sixteen and more each adds a segment's end to the general kernel, worth a round at 4 bits, where rounds are short (20
+// sequences, 32/8 heads, group 32 4: 1.35); at 2 it is not (one long one of 20, group 32 4: 0.95).
+// With more pairs than SMs (two CTAs in turn on an SM) it wins where lengths differ, 256 pairs, 4 bits 3: 19.9 -> 15.6, 288
+// pairs of nine sequences 4: 0.98, group 32 3: 0.87.  Where they are equal it wins if the second turn is half full at least
+// (160 pairs, 2 bits 2: 0.94, 224 pairs 2: 1.28), unless the general kernel's ranges are whole sequences (8 sequences in 4
+// ranges 1: 0.92, 9 in 4 1.21), and not at group 32 (256 pairs 3: 0.97).
+// A step that moves the lengths on saves its roll-over kernel as well, worth two rounds (8 x 2048 tokens 19.5 -> 11.8).
 // Equal lengths without a tail at 4 bits stop short of four rounds; they would win up to six (8 pairs on 64 SMs, 5: 1.20 times
 // as fast), which nobody has built on yet.
-constexpr signed char kShortRounds[2][2][3][3][2] = {
-    // by query tiles, 4 or 2 bits, group 128 / 64 / 32, SMs taken (below two fifths, below three quarters, above): {equal, ragged}
-    {{{{4, 4}, {6, 5}, {6, 5}}, {{3, 4}, {5, 5}, {6, 5}}, {{2, 3}, {3, 3}, {4, 3}}},
-     {{{2, 3}, {3, 3}, {6, 3}}, {{2, 3}, {3, 3}, {6, 3}}, {{2, 3}, {2, 3}, {4, 3}}}},
-    {{{{3, 3}, {4, 4}, {6, 5}}, {{3, 3}, {4, 4}, {6, 5}}, {{2, 3}, {3, 3}, {4, 3}}},
-     {{{2, 2}, {3, 3}, {6, 3}}, {{2, 2}, {3, 3}, {6, 3}}, {{0, 0}, {0, 0}, {0, 0}}}},
+constexpr signed char kShortRounds[2][2][3][4][2] = {
+    // by query tiles, 4 or 2 bits, group 128 / 64 / 32, SMs taken (below two fifths, a half, three quarters, above): {equal, ragged}
+    {{{{4, 4}, {6, 6}, {6, 6}, {6, 6}}, {{3, 4}, {6, 5}, {6, 5}, {6, 6}}, {{2, 3}, {3, 3}, {4, 3}, {4, 4}}},
+     {{{2, 3}, {3, 3}, {6, 4}, {6, 4}}, {{2, 3}, {3, 3}, {6, 4}, {6, 4}}, {{2, 3}, {2, 3}, {2, 3}, {4, 3}}}},
+    {{{{3, 3}, {4, 4}, {6, 5}, {6, 6}}, {{3, 3}, {4, 4}, {6, 5}, {6, 6}}, {{2, 3}, {3, 3}, {4, 4}, {4, 4}}},
+     {{{2, 2}, {3, 3}, {4, 3}, {6, 4}}, {{2, 2}, {3, 3}, {4, 3}, {6, 4}}, {{0, 0}, {0, 0}, {0, 0}, {0, 0}}}},
 };
-int short_cluster(const bd_decode_args *a, int sm_count, int64_t nblk) {
+// `rows`: ranges per KV head of the general kernel
+int short_cluster(const bd_decode_args *a, int sm_count, int64_t nblk, int rows) {
     const int gq = a->h / a->h_k, most = bd::decode_short_cluster(a->bits, a->group, gq);
-    const int64_t pairs = int64_t(a->b) * a->h_k;
-    if (most == 0 || a->num_splits > 0 || pairs > 2 * int64_t(sm_count)) return 0;
+    const int64_t pairs = int64_t(a->b) * a->h_k, sms = sm_count;
+    if (most == 0 || a->num_splits > 0 || pairs > 2 * sms) return 0;
     const bool ragged = a->cache_seqlens != nullptr || (a->k_res != nullptr && a->res_lens != nullptr);
     const int64_t items = 2 * nblk + (a->k_res ? (a->res_len + (a->k_new ? 1 : 0) + 15) / 16 : 0);
     int c = 1;
     while (2 * c <= most && c * bd::kShortWarps < items && pairs <= bd::decode_short_resident(a->bits, a->group, gq, 2 * c)) c *= 2;
     const int64_t round = int64_t(c) * bd::kShortWarps, taken = pairs * c;
+    const int top = a->bits == 4 && a->group >= 64 ? 6 : 4;          // of ragged lengths
     int rounds;
-    if (pairs > sm_count) {
-        if (!ragged) return 0;
-        rounds = (a->group == 32 ? 2 : 3) + (a->advance ? 1 : 0);
+    if (pairs > sms) {
+        if (!ragged) return a->group >= 64 && 2 * pairs >= 3 * sms && a->b % rows != 0 && items >= round && items <= 4 * round ? c : 0;
+        rounds = a->b >= 16 ? (a->bits == 4 ? 4 : 3) : (a->group >= 64 ? 3 : 2);
+        if (a->advance) rounds += 1;
     } else {
-        const int fill = 5 * taken < 2 * int64_t(sm_count) ? 0 : (4 * taken < 3 * int64_t(sm_count) ? 1 : 2);
+        const int fill = 5 * taken < 2 * sms ? 0 : (2 * taken <= sms ? 1 : (4 * taken < 3 * sms ? 2 : 3));
         rounds = kShortRounds[gq > 8][a->bits == 2][a->group == 128 ? 0 : (a->group == 64 ? 1 : 2)][fill][ragged];
-        if (a->advance) rounds = std::min(rounds + 1, 6);
+        if (ragged && a->b >= 16 && fill >= 2 && gq <= 8 && a->bits == 4) rounds = std::min(rounds + 1, top);
+        if (ragged && a->b > 1 && a->b < 8 && fill > 0 && (rounds == 4 || rounds == 6)) rounds -= 1;
+        if (a->advance) rounds = std::min(rounds + 2, top);
         if (a->bits == 4 && !ragged && a->k_res == nullptr) return items < std::min(4 * round, rounds * round + 1) ? c : 0;
     }
     return items <= rounds * round ? c : 0;
@@ -194,7 +205,7 @@ int make_plan(const bd_decode_args *a, int sm_count, DecodePlan &plan) {
         rows = plan_rows(a->b, a->h_k, a->s, a->bits, sm_count, bd::decode_ctas_per_sm(a->bits, a->group, gq, plan.two_ctas));
     }
     plan.rows = int(std::max<int64_t>(1, std::min<int64_t>(rows, 1 << 20)));
-    plan.cluster = short_cluster(a, sm_count, nblk);
+    plan.cluster = short_cluster(a, sm_count, nblk, plan.rows);
     const bool has_tail = a->k_res != nullptr;
     plan.ragged = a->cache_seqlens != nullptr || (has_tail && a->res_lens != nullptr);
     plan.n_uniform = bd::seq_blocks(a->s, a->s, nb) + (has_tail ? bd::tail_chunks(a->res_len + (a->k_new ? 1 : 0)) : 0);

@@ -197,8 +197,10 @@ def test_clusters_are_no_larger_than_run_at_once(pairs, most):
     (False, (4, 64, 4, 24320, 4, 128, 64, False)), (False, (2, 32, 8, 49152, 2, 128, 0, False)),
     (True, (1, 32, 8, 8192, 2, 64, 0, False)), (False, (1, 32, 8, 16384, 2, 64, 0, False)),
     (True, (1, 32, 8, 5888, 4, 32, 64, True)), (False, (1, 32, 8, 7936, 4, 32, 64, True)),
-    (True, (3, 32, 32, 1536, 4, 32, 0, True)), (False, (3, 32, 32, 2048, 4, 32, 0, True)), (False, (4, 32, 32, 4096, 2, 128, 0, True)),
-    (True, (8, 32, 32, 1024, 4, 128, 64, True)), (False, (8, 32, 32, 1536, 4, 32, 0, False)), (False, (20, 32, 8, 2048, 4, 128, 64, False))])
+    (True, (2, 32, 8, 1024, 4, 128, 0, True)), (True, (3, 32, 32, 1536, 4, 32, 0, True)), (False, (3, 32, 32, 2048, 4, 32, 0, True)), (False, (4, 32, 32, 4096, 2, 128, 0, True)),
+    (True, (8, 32, 32, 1024, 4, 128, 64, True)), (False, (8, 32, 32, 1536, 4, 32, 0, False)), (False, (20, 32, 8, 2048, 4, 128, 64, False)),
+    (True, (15, 32, 8, 2048, 4, 32, 0, True)), (True, (32, 32, 8, 2048, 4, 128, 0, False)), (False, (32, 32, 8, 4096, 4, 128, 0, False)),
+    (False, (36, 32, 8, 2048, 4, 128, 0, False)), (False, (32, 32, 8, 1024, 4, 32, 0, False))])
 def test_which_steps_are_little_work(little, shape):
     import bitladder_b200 as B
     if torch.cuda.get_device_properties(0).multi_processor_count != 148:
