@@ -50,7 +50,8 @@ struct ShortCfg {
     static constexpr int FIT = (LIMIT - OFF_MERGE) / DEPOSIT;
     static constexpr int CLUSTER = FIT >= 8 ? 8 : (FIT >= 4 ? 4 : (FIT >= 2 ? 2 : 1));
     static constexpr int OFF_BAR = OFF_MERGE + CLUSTER * DEPOSIT;
-    static constexpr int SMEM = OFF_BAR + WARPS * STAGES * 16;
+    static constexpr int OFF_FLAGS = OFF_BAR + WARPS * STAGES * 16;
+    static constexpr int SMEM = OFF_FLAGS + WARPS * 4;
     static_assert(DEPOSIT <= STAGES * 2 * CODE, "a warp's result fits its own tiles");
     static_assert(SMEM <= kSmemLimit, "shared memory");
 };
@@ -186,6 +187,8 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
 
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t smem_base = smem_u32(smem);
+    // Whether a wait of a warp ran out; written by that warp, read by the others behind the barrier that follows the loop.
+    volatile int *gave_up = reinterpret_cast<volatile int *>(smem + C::OFF_FLAGS);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int g = lane >> 2, l = lane & 3;
     // a cluster's CTAs are consecutive, and so are the heads of a sequence
@@ -202,6 +205,7 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
     }
     if (lane == 0) {
         for (int i = 0; i < 2 * STAGES; ++i) mbar_init(bars + 8 * i, 1);
+        gave_up[warp] = 0;
         fence_mbar_init();
         tma_prefetch_desc(&kmap);
         tma_prefetch_desc(&vmap);
@@ -424,7 +428,6 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
 
     // ---- half blocks ----
     int n = 0;
-    bool gave_up = false;                    // a wait of this warp ran out
 #pragma unroll 1
     for (int item = unit0; item < items; item += stride, ++n) {
         const int st = STAGES == 2 ? n & 1 : 0;
@@ -440,7 +443,7 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
             }
         }
         const bool need_mask = (blk + 1) * NB > seqlen_blk;
-        if (!copied(bars + 16 * st, par)) { gave_up = true; break; }
+        if (!copied(bars + 16 * st, par)) { gave_up[warp] = 1; break; }
 
         // q . zero per token group, two groups at a time: rows 0-7 the one, rows 8-15 the other
         float Zc[NGK][NQT][2];
@@ -548,7 +551,7 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
                 Pb[j][nq][1] = movmatrix_trans(pack_f16x2(t[j][2], t[j][3]));
             }
         }
-        if (!copied(bars + 16 * st + 8, par)) { gave_up = true; break; }
+        if (!copied(bars + 16 * st + 8, par)) { gave_up[warp] = 1; break; }
 #pragma unroll
         for (int j = 0; j < P; ++j) {
             const int r0 = 16 * u + 32 * j + 2 * l;               // tokens of fragment register 0
@@ -646,7 +649,7 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
             stsf(mine + ((32 * NQT + nq * 4 + 2 + c) * 32 + lane) * 4, sum);
         }
     }
-    const bool aborted = __syncthreads_or(gave_up);
+    __syncthreads();
     // The lengths move on when every CTA that works on the sequence has read them: each counts in, behind the barrier that
     // all of its warps have met at (a count per warp, each behind its own reads: a step of 8 sequences 11.05 -> 10.4 us, of 2
     // 13.1 -> 12.3), and the last one writes them where the others wait anyway.
@@ -656,11 +659,15 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
         arrived = atomicAdd(roll.roll_arrivals + int64_t(ib) * p.h_k, 1);
     }
     // (the rule of bd_pack.cu's roll-over, for the lengths and for the block)
-    const bool room = cached >= 0 && cached % NB == 0 && cached <= roll.roll_s_cap - NB;
-    int left = min(max(in_tail, 0), roll.roll_res_cap);
-    if (left < roll.roll_res_cap) left += 1;
+    auto room_for_block = [&]() { return cached >= 0 && cached % NB == 0 && cached <= roll.roll_s_cap - NB; };
+    auto tail_behind_step = [&]() {
+        const int r = min(max(in_tail, 0), roll.roll_res_cap);
+        return r < roll.roll_res_cap ? r + 1 : r;
+    };
     auto move_on = [&]() {
         if (arrived == p.h_k * ncta - 1) {
+            const bool room = room_for_block();
+            const int left = tail_behind_step();
             __threadfence();
             roll.roll_arrivals[int64_t(ib) * p.h_k] = 0;
             if (left == NB && room) roll.roll_cache_seqlens[ib] = cached + NB;
@@ -747,7 +754,10 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
             else static_cast<float *>(p.out)[oi] = v;
         }
     }
-    if (aborted) {
+    int aborted = 0;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) aborted |= gave_up[w];
+    if (aborted != 0) {
         if (tid == 0) atomicExch(p.status, BD_ERR_TIMEOUT);
         // give copies that are still in flight time to land before a full tail is packed through the tiles, and before the
         // block's shared memory is released
@@ -756,7 +766,7 @@ bd_decode_short_kernel(const DecodeParams p, const PackParams roll, const __grid
     }
     if (roll.roll_res_lens != nullptr) {
         if (ncta == 1) move_on();
-        if (left == NB && room) {
+        if (tail_behind_step() == NB && room_for_block()) {
             // (the token's own row, stored by one of the cluster's warps, is visible behind the barriers above)
             static_assert(PackCfg<BITS, GROUP>::NTHREADS == 128 && WARPS == 8, "two groups of threads pack");
             static_assert(sizeof(typename PackCfg<BITS, GROUP>::Shared) <= 16384 && C::OFF_PRM >= 32768, "in the warps' tiles");
