@@ -25,6 +25,7 @@ struct DeviceInfo {
     bool ok = false;
     int sm_count = 0;
     int cc_major = 0;
+    int dev = -1;
 };
 
 int current_device_info(DeviceInfo &info) {
@@ -40,6 +41,7 @@ int current_device_info(DeviceInfo &info) {
         if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return BD_ERR_CUDA;
         cache[dev].sm_count = sm;
         cache[dev].cc_major = major;
+        cache[dev].dev = dev;
         cache[dev].ok = true;
     }
     info = cache[dev];
@@ -156,14 +158,15 @@ constexpr signed char kShortRounds[2][2][3][4][2] = {
      {{{2, 2}, {3, 3}, {4, 3}, {6, 4}}, {{2, 2}, {3, 3}, {4, 3}, {6, 4}}, {{0, 0}, {0, 0}, {0, 0}, {0, 0}}}},
 };
 // `rows`: ranges per KV head of the general kernel
-int short_cluster(const bd_decode_args *a, int sm_count, int64_t nblk, int rows) {
+int short_cluster(const bd_decode_args *a, const DeviceInfo &info, int64_t nblk, int rows) {
     const int gq = a->h / a->h_k, most = bd::decode_short_cluster(a->bits, a->group, gq);
-    const int64_t pairs = int64_t(a->b) * a->h_k, sms = sm_count;
+    const int64_t pairs = int64_t(a->b) * a->h_k, sms = info.sm_count;
     if (most == 0 || a->num_splits > 0 || pairs > 2 * sms) return 0;
     const bool ragged = a->cache_seqlens != nullptr || (a->k_res != nullptr && a->res_lens != nullptr);
     const int64_t items = 2 * nblk + (a->k_res ? (a->res_len + (a->k_new ? 1 : 0) + 15) / 16 : 0);
     int c = 1;
-    while (2 * c <= most && c * bd::kShortWarps < items && pairs <= bd::decode_short_resident(a->bits, a->group, gq, 2 * c)) c *= 2;
+    while (2 * c <= most && c * bd::kShortWarps < items && pairs * 2 * c <= sms &&
+           pairs <= bd::decode_short_resident(a->bits, a->group, gq, 2 * c, info.dev)) c *= 2;
     const int64_t round = int64_t(c) * bd::kShortWarps, taken = pairs * c;
     const int top = a->bits == 4 && a->group >= 64 ? 6 : 4;          // of ragged lengths
     int rounds;
@@ -182,7 +185,8 @@ int short_cluster(const bd_decode_args *a, int sm_count, int64_t nblk, int rows)
     return items <= rounds * round ? c : 0;
 }
 
-int make_plan(const bd_decode_args *a, int sm_count, DecodePlan &plan) {
+int make_plan(const bd_decode_args *a, const DeviceInfo &info, DecodePlan &plan) {
+    const int sm_count = info.sm_count;
     const int nb = pack_block_tokens(a->bits);
     const int64_t nblk = (int64_t(a->s) + nb - 1) / nb;
     const int gq = a->h / a->h_k;
@@ -205,7 +209,7 @@ int make_plan(const bd_decode_args *a, int sm_count, DecodePlan &plan) {
         rows = plan_rows(a->b, a->h_k, a->s, a->bits, sm_count, bd::decode_ctas_per_sm(a->bits, a->group, gq, plan.two_ctas));
     }
     plan.rows = int(std::max<int64_t>(1, std::min<int64_t>(rows, 1 << 20)));
-    plan.cluster = short_cluster(a, sm_count, nblk, plan.rows);
+    plan.cluster = short_cluster(a, info, nblk, plan.rows);
     const bool has_tail = a->k_res != nullptr;
     plan.ragged = a->cache_seqlens != nullptr || (has_tail && a->res_lens != nullptr);
     plan.n_uniform = bd::seq_blocks(a->s, a->s, nb) + (has_tail ? bd::tail_chunks(a->res_len + (a->k_new ? 1 : 0)) : 0);
@@ -385,7 +389,7 @@ int bd_decode_plan(const bd_decode_args *a, int32_t out[4]) {
     rc = current_device_info(info);
     if (rc != BD_OK) return rc;
     DecodePlan plan;
-    make_plan(a, info.sm_count, plan);
+    make_plan(a, info, plan);
     const int gq = a->h / a->h_k;
     if (plan.cluster > 0) {
         out[0] = a->b * plan.cluster;
@@ -463,13 +467,13 @@ int bd_prefill(const bd_prefill_args *f, bd_stream_t stream) {
 size_t bd_decode_workspace_bytes(const bd_decode_args *a) {
     if (!a || a->b <= 0 || a->h <= 0 || a->h_k <= 0 || (a->bits != 2 && a->bits != 4)) return 0;
     DeviceInfo info;
-    int sm = 148;
     if (a->num_splits <= 0) {
         if (current_device_info(info) != BD_OK) return 0;
-        sm = info.sm_count;
+    } else {
+        info.sm_count = 148;
     }
     DecodePlan plan;
-    make_plan(a, sm, plan);
+    make_plan(a, info, plan);
     return plan.total_bytes;
 }
 
@@ -491,7 +495,7 @@ static int decode_step(const bd_decode_args *a, const bd_exchange_args *x, bd_st
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
 
     DecodePlan plan;
-    make_plan(a, info.sm_count, plan);
+    make_plan(a, info, plan);
     if (!a->workspace || a->workspace_bytes < plan.total_bytes) return BD_ERR_WORKSPACE;
     if (!aligned16(a->workspace)) return BD_ERR_ALIGNMENT;
 
@@ -726,7 +730,7 @@ int bd_decode_noalloc(const bd_decode_args *a, bd_stream_t stream_) {
     if (rc != BD_OK) return rc;
     if (info.cc_major != 10) return BD_ERR_DEVICE;
     DecodePlan plan;
-    make_plan(a, info.sm_count, plan);
+    make_plan(a, info, plan);
     if (plan.total_bytes > BD_NOALLOC_SCRATCH_BYTES) return BD_ERR_SCRATCH_LIMIT;
     void *scratch = noalloc_scratch_address(&rc);
     if (rc != BD_OK) return rc;

@@ -834,12 +834,11 @@ static cudaError_t launch_short(const DecodeParams &p, const PackParams &roll, c
 // Clusters of a size that run at once: a cluster's CTAs take an SM each, all in one GPC, and the SMs that a GPC has beyond a
 // multiple of the size stay without one.  Asked once per device.
 template <int BITS, int GROUP, int NQT>
-static int resident_short(int cluster) {
+static int resident_short(int cluster, int dev) {
     static std::atomic<int> known[64][4] = {};           // one more than the answer for clusters of 1, 2, 4 and 8
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    std::atomic<int> *slot = dev < 64 ? &known[dev][cluster == 8 ? 3 : cluster / 2] : nullptr;
-    if (slot && *slot > 0) return *slot - 1;
+    if (dev < 0 || dev >= 64) return 0;
+    std::atomic<int> &slot = known[dev][cluster == 8 ? 3 : cluster / 2];
+    if (slot > 0) return slot - 1;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[2];
     int n = 0;
@@ -850,7 +849,7 @@ static int resident_short(int cluster) {
         (void)cudaGetLastError();
         return 0;
     }
-    if (slot) *slot = n + 1;
+    slot = n + 1;
     return n;
 }
 
@@ -877,8 +876,8 @@ int decode_short_cluster(int bits, int group, int gq) {
     return 0;
 }
 
-int decode_short_resident(int bits, int group, int gq, int cluster) {
-#define BD_SHORT_RESIDENT(B, G, Q) return resident_short<B, G, Q>(cluster);
+int decode_short_resident(int bits, int group, int gq, int cluster, int dev) {
+#define BD_SHORT_RESIDENT(B, G, Q) return resident_short<B, G, Q>(cluster, dev);
     BD_SHORT_PICK(BD_SHORT_RESIDENT)
     return 0;
 }

@@ -318,7 +318,8 @@ constexpr int kShortWarps = 8;    // warps per CTA
 cudaError_t launch_decode_short(const DecodeParams &p, const PackParams &roll, const CUtensorMap &kmap, const CUtensorMap &vmap,
                                 int bits, int group, cudaStream_t stream);
 int decode_short_cluster(int bits, int group, int gq);    // most CTAs per cluster; 0: not built
-int decode_short_resident(int bits, int group, int gq, int cluster);      // clusters of that many CTAs that the device runs at once
+// Clusters of that many CTAs that the current device, number `dev`, runs at once.
+int decode_short_resident(int bits, int group, int gq, int cluster, int dev);
 // `two`: the variant with half as many warps per CTA and two CTAs per SM (see Cfg in bd_decode.cu)
 bool decode_two_ctas_built(int bits, int group, int gq);
 int decode_ctas_per_sm(int bits, int group, int gq, int two);
